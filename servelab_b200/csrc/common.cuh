@@ -188,6 +188,21 @@ static inline int slb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The same without the attribute: for kernels of at most a wave of blocks that compute for long.  Placed
+// while the preceding kernel still holds part of the SMs, several of their blocks land on the SMs that are
+// free first and the others stay idle (a float32 product of 126 blocks behind SwiGLU: 304 us, and 114
+// when it begins on an empty device).
+template <typename... KArgs, typename... Args>
+static inline int slb_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                   cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // A status word on the device with its host accessor `fn(reset)`: 0, or the code of the first
 // event recorded since the last reset.  Reading synchronises with the device.
 #define SLB_DEFINE_STATUS_WORD(var, fn)                                               \

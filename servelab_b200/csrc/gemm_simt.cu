@@ -198,9 +198,9 @@ static int launch_f32_tile(const F32Args& g, cudaStream_t st) {
     auto kernel = gemm_tn_f32_kernel<BM, BN, TM, TN, BK>;
     const int err = slb_configure(&configured, kernel, smem);
     if (err) return err;
-    return slb_launch(kernel, dim3((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, g.batch), dim3((BM / TM) * (BN / TN)),
-                      smem, st, g.A, g.lda, g.W, g.ldw, g.C, g.ldc, g.bias, g.M, g.N, g.K, g.batch_a, g.batch_w,
-                      g.batch_c);
+    return slb_launch_after(kernel, dim3((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, g.batch),
+                            dim3((BM / TM) * (BN / TN)), smem, st, g.A, g.lda, g.W, g.ldw, g.C, g.ldc, g.bias, g.M, g.N, g.K, g.batch_a, g.batch_w,
+                            g.batch_c);
 }
 
 // Which tile: the products are sums in order, so K is not split, and the tiles differ in how many
