@@ -41,3 +41,166 @@ def test_float32_product_is_that_of_the_plain_kernel(M, N, Kd):
     for h in range(3):
         K().gemm_simt(heads_a[:, h].contiguous(), heads_w[h], one)
         assert torch.equal(out[:, h], one)
+
+
+def step(lens, starts=None, page=16, slots=None):
+    """A packed step of requests with the given tokens, pages in order."""
+    from servelab_b200.engine.batch import BatchEntry, StepContext
+    starts = starts or [0] * len(lens)
+    entries, at = [], 0
+    for i, (n, s) in enumerate(zip(lens, starts)):
+        pages = -(-(s + n) // page)
+        entries.append(BatchEntry(tokens=[0] * n, start=s, want=(), block_tables=[list(range(at, at + pages))],
+                                  state_slot=slots[i] if slots else i))
+        at += pages
+    return StepContext.pack(entries, 1, DEV), at
+
+
+def odd_view(t):
+    """The same rows at an address and a row stride that 16-byte accesses do not take."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 3, dtype=t.dtype, device=t.device)
+    wide[:, 1:1 + t.shape[1]] = t
+    return wide[:, 1:1 + t.shape[1]]
+
+
+# ---------------------------------------- heads' norms, rotation and cache write in pieces
+HEADS = {   # q heads, kv heads, key size, value size, rotated, halves, norm, unit norm, row norm, biases, mixed values
+    "rotated_halves": (16, 4, 128, 128, 64, True, 0, 0, False, False, None),
+    "normed_pairs": (6, 2, 64, 32, 48, False, 64, 0, False, False, "mix"),
+    "part_normed_kept": (3, 3, 96, 64, 16, False, 40, 0, False, True, "keep"),
+    "unit_after_rotation": (8, 1, 256, 512, 256, True, 0, 256, False, False, None),
+    "row_normed_biases": (16, 4, 128, 64, 0, False, 0, 0, True, True, None),
+    "row_normed_wide": (40, 8, 96, 64, 0, False, 0, 0, True, True, None),
+    "many_heads": (40, 8, 128, 128, 128, True, 128, 0, False, True, None),
+}
+
+
+@pytest.mark.parametrize("name", HEADS)
+@pytest.mark.parametrize("lens", [[1], [3, 1, 40], [700]])
+def test_heads_in_pieces_are_those_of_the_general_kernel(name, lens):
+    """The general kernel runs on rows at odd addresses; both work in float32 and differ in the order of a head's sum
+    of squares: one rounding to bfloat16 (2^-8 of a value) and 2^-16 of the largest where a rotation cancels."""
+    H, G, D, Dv, rot, halves, norm, unit, row, biased, mixed = HEADS[name]
+    g = gen(len(lens) + H)
+    ctx, pages = step(lens, [7 * i for i in range(len(lens))])
+    T, width = sum(lens), H * D + G * (D + Dv)
+    proj = (torch.randn(T, width, device=DEV, generator=g) * 2).bfloat16()
+    nq, nk = (H * D, G * D) if row else (D, D)
+    qw, kw = (1 + 0.1 * torch.randn(n, device=DEV, generator=g) for n in (nq, nk))
+    bias = [torch.randn(n, device=DEV, generator=g) for n in (H * D, G * D, G * Dv)] if biased else [None] * 3
+    freq = 10000.0 ** (-torch.arange(rot // 2, device=DEV) / max(rot // 2, 1)).float()
+    first = torch.randn(T, G * Dv, device=DEV, generator=g).bfloat16()
+    lam = torch.tensor([0.3], device=DEV)
+    got = []
+    for p in (proj, odd_view(proj)):
+        q = torch.zeros(T, H * D, device=DEV, dtype=torch.bfloat16)
+        kc = torch.zeros(pages, G, 16, D, device=DEV, dtype=torch.bfloat16)
+        vc = torch.zeros(pages, G, 16, Dv, device=DEV, dtype=torch.bfloat16)
+        keep = torch.zeros(T, G * Dv, device=DEV, dtype=torch.bfloat16)
+        K().head_prep(p, ctx, ctx.block_tables[0], 16, q_off=0, num_heads=H, q_dim=D, q_norm_w=qw, q_norm_dims=norm,
+                      q_rot_off=0, k_off=H * D, num_kv_heads=G, k_dim=D, k_norm_w=kw, k_norm_dims=norm, k_rot_off=0,
+                      v_off=H * D + G * D, v_dim=Dv, freq=freq if rot else None, rot_dims=rot, rot_mag=1.1, eps=1e-6,
+                      q_out=q, k_cache=kc, v_cache=vc, lam=lam if mixed == "mix" else None,
+                      v_first=first if mixed == "mix" else None, v_keep=keep if mixed == "keep" else None,
+                      rot_half=halves, q_unit_dims=unit, k_unit_dims=unit, q_bias=bias[0], k_bias=bias[1],
+                      v_bias=bias[2], row_norm=row)
+        got.append([t.float() for t in (q, kc, vc, keep)])
+    assert K().head_prep_status() == 0
+    for a, b in zip(*got):
+        assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 2.0 ** -16 * b.abs().max()).all()
+    assert got[0][0].abs().max() > 0 and got[0][1].abs().max() > 0 and got[0][2].abs().max() > 0
+
+
+@pytest.mark.parametrize("lens", [[2, 30], [600]])
+@pytest.mark.parametrize("H,D,rot,R", [(16, 128, 64, 256), (5, 48, 32, 96), (8, 64, 64, 448)])
+def test_latent_rows_in_pieces_are_those_of_the_general_kernel(H, D, rot, R, lens):
+    """A latent attention's rows: one long key (normed latent, rotated rest), queries whose unrotated part is skipped."""
+    g = gen(H + len(lens))
+    ctx, pages = step(lens)
+    T, q_head = sum(lens), D + rot
+    proj = torch.randn(T, H * q_head + R + rot, device=DEV, generator=g).bfloat16()
+    kw = 1 + 0.1 * torch.randn(R, device=DEV, generator=g)
+    freq = 10000.0 ** (-torch.arange(rot // 2, device=DEV) / (rot // 2)).float()
+    got = []
+    for p in (proj, odd_view(proj)):
+        q = torch.zeros(T, H * (R + rot), device=DEV, dtype=torch.bfloat16)
+        kc = torch.zeros(pages, 1, 16, R + rot, device=DEV, dtype=torch.bfloat16)
+        K().head_prep(p, ctx, ctx.block_tables[0], 16, q_off=0, num_heads=H, q_dim=q_head, q_norm_w=None, q_norm_dims=0,
+                      q_rot_off=D, q_out=q[:, R:], q_head_stride=R + rot, q_skip=D, k_off=H * q_head, num_kv_heads=1,
+                      k_dim=R + rot, k_norm_w=kw, k_norm_dims=R, k_rot_off=R, v_off=-1, v_dim=0, freq=freq,
+                      rot_dims=rot, rot_mag=1.0, eps=1e-6, k_cache=kc, v_cache=None)
+        got.append([q.float(), kc.float()])
+    for a, b in zip(*got):
+        assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 2.0 ** -16 * b.abs().max()).all() and a.abs().max() > 0
+
+
+@pytest.mark.parametrize("T,N,group", [(1, 8, 1), (5, 2048, 1), (300, 1000, 1), (33, 1024, 64)])
+def test_sigmoid_gate_in_pieces(T, N, group):
+    g = gen(T)
+    x, z = (torch.randn(T, n, device=DEV, generator=g).bfloat16() for n in (N, N // group))
+    fast, plain = torch.empty_like(x), torch.empty_like(x)
+    K().sigmoid_gate(x, z, fast, group)
+    K().sigmoid_gate(odd_view(x), odd_view(z), plain, group)
+    assert torch.equal(fast, plain)
+
+
+# ------------------------------------------------------------ convolution, norms with a gate
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lens", [[256], [1, 2, 300, 7], [129, 128, 5]])
+def test_convolution_of_runs_is_that_of_single_tokens(dtype, taps, lens):
+    """Portions from 256 tokens on take runs of tokens a thread; rows at an odd address the kernel that takes them one
+    by one.  The same products in the same order: the same bits, in the rows and in the records."""
+    g = gen(taps + len(lens))
+    C = 264
+    ctx, _ = step(lens)
+    T = sum(lens)
+    proj = torch.randn(T, C + 8, device=DEV, generator=g).to(dtype)
+    w, b_in, b_out = (torch.randn(*s, device=DEV, generator=g) for s in ((taps, C), (C,), (C,)))
+    record = torch.randn(len(lens), (taps - 1) * C + 4, device=DEV, generator=g)
+    got = []
+    for p in (proj, odd_view(proj)):
+        out, state = torch.zeros(T, C, device=DEV, dtype=dtype), record.clone()
+        K().short_conv(p, w, state, ctx, out, b_in, b_out, activation="silu")
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,groups,size", [(1, 1, 4), (7, 3, 100), (33, 8, 256), (5, 4, 512), (9, 2, 1024), (3, 2, 1028)])
+def test_gated_norms_against_64_bits(dtype, T, groups, size):
+    """Sums of up to 1,028 squares in float32: 1e-6 of a value, and the result's rounding."""
+    g, n = gen(T + size), groups * size
+    x, lam, w = (torch.randn(*s, device=DEV, generator=g) for s in ((T, 2 * n), (1,), (n,)))
+    gate = torch.randn(T, n, device=DEV, generator=g).to(dtype)
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 4e-6
+
+    def rms(v):
+        v = v.reshape(T, groups, size)
+        return (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6)).reshape(T, n)
+    d, z = x.double(), gate.double()
+    pairs = d.view(T, groups, 2, size)
+    for maps, rows in ((1, d[:, :n]), (2, pairs[:, :, 0] - lam.double() * pairs[:, :, 1])):
+        out = torch.empty(T, n, device=DEV, dtype=dtype)
+        K().group_norm_gate(x[:, :n] if maps == 1 else x, groups, size, out, eps=1e-6, weight=w, factor=0.7, gate=gate,
+                            gate_activation="silu", maps=maps, lam=lam)
+        want = 0.7 * rms(rows) * w.double() * z * torch.sigmoid(z)
+        assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
+    out = torch.empty(T, n, device=DEV, dtype=dtype)
+    K().gate_group_norm(x[:, :n], gate, groups, out, eps=1e-6, weight=w, factor=1.5)
+    want = 1.5 * rms(d[:, :n] * z * torch.sigmoid(z)) * w.double()
+    assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [4, 1024, 1028, 2048, 3584, 4100])
+def test_sum_of_two_norms_against_64_bits(dtype, n):
+    g = gen(n)
+    a, b = (torch.randn(5, n, device=DEV, generator=g) * 3 for _ in range(2))
+    wa, wb = (torch.randn(n, device=DEV, generator=g) for _ in range(2))
+    out = torch.empty(5, n, device=DEV, dtype=dtype)
+    K().norm_sum2(a, b, wa, wb, 1e-6, 0.5, out)
+    u, v = ((t.double() / torch.sqrt((t.double() ** 2).mean(-1, keepdim=True) + 1e-6)) * w.double()
+            for t, w in ((a, wa), (b, wb)))
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    assert ((out.double() - 0.5 * (u + v)).abs() <= tol * (u + v).abs() + 2e-6 * (u.abs() + v.abs()) + 1e-7).all()
