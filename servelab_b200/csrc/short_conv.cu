@@ -144,6 +144,112 @@ __global__ void __launch_bounds__(256) qk_conv_cache_kernel(
     }
 }
 
+// A portion of a prompt: a thread owns 4 channels of SC_RUN neighbouring tokens, so that a projected row is
+// read (SC_RUN + TAPS - 1) / SC_RUN times instead of TAPS times and the taps once; all its rows are in flight
+// before the first is used.  Tokens near a request's start take the rows before them from its record.
+// What bounds it is memory and, with SiLU, the exponentials and divisions.  3,072 channels, 4 taps: 2,048
+// tokens 16.8 -> 8.9 us; 2,912 tokens with SiLU 26.1 -> 18.3.  (8 channels a thread: 161 registers, slower.)
+constexpr int SC_RUN = 8;
+template <typename T> __device__ __forceinline__ void load4(const T* p, float (&v)[4]);
+template <> __device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) { load_vec<float, 4>(p, v); }
+template <> __device__ __forceinline__ void load4<bf16>(const bf16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
+    v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { store_vec<float, 4>(p, v); }
+__device__ __forceinline__ void store4(bf16* p, const float (&v)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) conv_run_kernel(
+    const T* __restrict__ proj, int ldp, const float* __restrict__ taps_w, const float* __restrict__ state,
+    const int* __restrict__ state_slots, const int* __restrict__ cu_q, const int* __restrict__ seq_of_token,
+    const int* __restrict__ positions, const int* __restrict__ block_table, int max_pages, int page_size,
+    int num_pages, float temp_coef, int temp_every, T* __restrict__ q_out, int ldq, T* __restrict__ k_cache,
+    int q_size, int Hkv, int D, int num_tokens, long long state_stride, const float* __restrict__ in_bias,
+    const float* __restrict__ out_bias, int act) {
+    constexpr int HIST = TAPS - 1;
+    const int C = q_size + Hkv * D;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int t0 = blockIdx.y * SC_RUN;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (c >= C) return;
+    const int run_seq = seq_of_token[t0], last_seq = seq_of_token[min(t0 + SC_RUN, num_tokens) - 1];
+    const int first_of_run = cu_q[run_seq];
+    struct __align__(4 * sizeof(T)) Four { T v[4]; };
+    Four raw[SC_RUN + HIST];
+#pragma unroll
+    for (int r = 0; r < SC_RUN + HIST; ++r) {
+        const int t = t0 - HIST + r;
+        if (t >= 0 && t < num_tokens) raw[r] = *reinterpret_cast<const Four*>(proj + (size_t)t * ldp + c);
+    }
+    float w[TAPS][4], add[4] = {0.f, 0.f, 0.f, 0.f}, first[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) load4<float>(taps_w + (size_t)i * C + c, w[i]);
+    if (in_bias != nullptr) load4<float>(in_bias + c, add);
+    if (out_bias != nullptr) load4<float>(out_bias + c, first);
+    auto finish = [&](int t, int s, float (&y)[4]) {
+        if (act == 1) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) y[v] = y[v] / (1.0f + expf(-y[v]));
+        }
+        if (c < q_size) {
+            if (temp_coef != 0.f) {
+                const float f = 1.f + temp_coef * logf(floorf((float)(positions[t] + 1) / (float)temp_every) + 1.f);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) y[v] *= f;
+            }
+            store4(q_out + (size_t)t * ldq + c, y);
+        } else if (k_cache != nullptr) {
+            const int cc = c - q_size, kvh = cc / D, d = cc - kvh * D, pos = positions[t];
+            const int page = block_table[(size_t)s * max_pages + pos / page_size];
+            if (page >= num_pages) atomicCAS(&conv_cache_status_word, 0, 1);
+            else if (page >= 0)
+                store4(k_cache + (((size_t)page * Hkv + kvh) * page_size + pos % page_size) * D + d, y);
+        }
+    };
+    if (t0 + SC_RUN <= num_tokens && t0 - first_of_run >= HIST && last_seq == run_seq) {
+        // (nearly every run: one request's tokens with all rows before them in this step)
+#pragma unroll
+        for (int r = 0; r < SC_RUN; ++r) {
+            float y[4] = {first[0], first[1], first[2], first[3]};
+#pragma unroll
+            for (int i = 0; i < TAPS; ++i) {
+                float u[4];
+                load4<T>(raw[r + i].v, u);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) y[v] = fmaf(w[i][v], u[v] + add[v], y[v]);
+            }
+            finish(t0 + r, run_seq, y);
+        }
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < SC_RUN; ++r) {
+        const int t = t0 + r;
+        if (t >= num_tokens) break;
+        const int s = seq_of_token[t], j = t - cu_q[s];
+        float y[4] = {first[0], first[1], first[2], first[3]};
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) {
+            float u[4];
+            if (j - HIST + i >= 0) {
+                load4<T>(raw[r + i].v, u);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) u[v] += add[v];
+            } else {
+                load4<float>(state + (size_t)state_slots[s] * state_stride + (size_t)(j + i) * C + c, u);
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) y[v] = fmaf(w[i][v], u[v], y[v]);
+        }
+        finish(t, s, y);
+    }
+}
+
 // new record = last taps - 1 rows of (old record, this step's portion), per request and channel
 template <typename T>
 __global__ void __launch_bounds__(256) conv_state_update_kernel(
@@ -199,7 +305,15 @@ static int launch_conv(const T* proj, int ldp, const float* taps_w, int taps, fl
                      (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)state |
                        (uintptr_t)taps_w | (uintptr_t)in_bias | (uintptr_t)out_bias) & 15) == 0;
     int rc;
-    if (vec) {
+    // (a run of tokens a thread from SC_RUN_MIN_TOKENS on: with fewer there are too few threads to fill the device)
+    constexpr int SC_RUN_MIN_TOKENS = 256;
+    if (vec && !inline_update && taps >= 2 && taps <= 4 && T_tokens >= SC_RUN_MIN_TOKENS) {
+        auto kernel = taps == 2 ? conv_run_kernel<T, 2> : taps == 3 ? conv_run_kernel<T, 3> : conv_run_kernel<T, 4>;
+        rc = slb_launch(kernel, dim3((C / 4 + 127) / 128, (T_tokens + SC_RUN - 1) / SC_RUN), dim3(128), 0, st, proj,
+                        ldp, taps_w, state, state_slots, cu_q, seq_of_token, positions, block_table, max_pages, page_size,
+                        num_pages, temp_coef, temp_every, q_out, ldq, k_cache, q_size, Hkv, D, T_tokens, state_stride,
+                        in_bias, out_bias, act);
+    } else if (vec) {
         const int threads = C / V >= 256 ? 256 : 64;
         rc = slb_launch(qk_conv_cache_kernel<T, V>, dim3((C / V + threads - 1) / threads, T_tokens), dim3(threads),
                         0, st, proj, ldp, taps_w, taps, state, state_slots, cu_q, seq_of_token, positions,
