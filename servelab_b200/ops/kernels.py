@@ -1147,6 +1147,9 @@ def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
                M, N, Kd, B, a.stride(1), w.stride(0), out.stride(1), _stream()), "gemm_simt_batched")
 
 
+# Steps of this many tokens: this package's kernel for many tokens, the vendor's product for widths it does not
+# take.  Measured us (kernel for few tokens / vendor, with the copy to float32 / this) at 32 experts of 2,048: 512
+# tokens 13.8 / 21.6 / 13.3, 2,048 tokens 44 / 49 / 13.6; 16 of 1,024: 5.9 / 16.4 / 7.4 and 16.3 / 25.1 / 7.5.
 router_vendor_min_tokens = 512
 
 
@@ -1154,6 +1157,13 @@ def router_logits(x: torch.Tensor, w_f32: torch.Tensor) -> torch.Tensor:
     """float32 logits x . w^T of a float32 router matrix (activations float32 or bfloat16); a
     token's sums run in a fixed order."""
     M, Kd = x.shape
+    if (x.dtype == _BF16 and M >= router_vendor_min_tokens and Kd % 32 == 0 and x.stride(0) % 8 == 0
+            and w_f32.stride(0) % 4 == 0 and (x.data_ptr() | w_f32.data_ptr()) % 16 == 0):
+        out = torch.empty((M, w_f32.shape[0]), dtype=_F32, device=x.device)
+        L.check(L.core().slb_router_logits_tile_bf16(
+            x.data_ptr(), x.stride(0), w_f32.data_ptr(), w_f32.stride(0), out.data_ptr(), out.stride(0), M,
+            w_f32.shape[0], Kd, _stream()), "router_logits")
+        return out
     if x.dtype == _BF16 and M >= router_vendor_min_tokens:
         # a large step in the bfloat16 path: the vendor's float32 product (no reduced-precision
         # mode: torch's default for float32 products) on the widened rows
@@ -1212,12 +1222,16 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
             and inter % 8 == 0 and n_out % 8 == 0 and hasattr(torch, "_grouped_mm")):
         # Large steps: the vendor's grouped product over the rows sorted by expert (the plan's list
         # and offsets stay on the device), as the dense products of large steps go to the vendor's
-        # GEMM; gathering and scattering rows are copies.
+        # GEMM; the weighted sum reads a token's rows where the product left them.
         from .profile import mark
-        nt = (plan.numel() - 4 * E - 1 - P) // 2
+        at = plan.numel() - 2 * P
         ends = plan[E + 1:2 * E + 1]                                   # cumulative row counts
-        order = plan[3 * E + 1 + 2 * nt:3 * E + 1 + 2 * nt + P]        # pairs sorted by expert
-        xs = x.index_select(0, torch.div(order, top, rounding_mode="floor"))
+        order = plan[at:at + P]                                        # pairs sorted by expert
+        if x.stride(0) % 8 or x.data_ptr() % 16:
+            x = x.clone(memory_format=torch.contiguous_format)
+        xs = torch.empty((P, h), dtype=x.dtype, device=x.device)
+        L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, h, xs.data_ptr(),
+                                        xs.stride(0), _stream()), "moe_gather")
         gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
         mark("library grouped gemm")
         act = torch.empty((P, inter), dtype=x.dtype, device=x.device)
@@ -1228,13 +1242,11 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
                       weights.view(-1).index_select(0, order) if weight_inputs else None)
         ys = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)
         mark("library grouped gemm")
-        y = torch.empty_like(ys)
-        y.index_copy_(0, order.long(), ys)
         out = torch.empty((T, n_out), dtype=x.dtype, device=x.device)
-        L.check(lib.slb_moe_combine_bf16_rows(
-            y.data_ptr(), y.stride(0), _p(out_weights), _p(shared),
-            shared.stride(0) if shared is not None else 0, out.data_ptr(), out.stride(0), T, top, n_out,
-            _stream()), "moe_combine")
+        L.check(lib.slb_moe_combine_bf16_sorted(
+            ys.data_ptr(), ys.stride(0), _p(out_weights), _p(shared),
+            shared.stride(0) if shared is not None else 0, out.data_ptr(), out.stride(0), plan.data_ptr(), E, T, top,
+            n_out, _stream()), "moe_combine")
         return out
     act = torch.empty((P, inter), dtype=x.dtype, device=x.device)
     sfx = _suffix(x.dtype)

@@ -148,7 +148,9 @@ _CORE_SIGNATURES = {
     "slb_moe_down_mma_bf16": [P, I, P, I, P, I, P, I, I, I, I, I, P],
     "slb_moe_combine_f32": [P, I, P, P, I, P, I, I, I, I, P],
     "slb_moe_combine_bf16": [P, I, P, P, I, P, I, I, I, I, P],
-    "slb_moe_combine_bf16_rows": [P, I, P, P, I, P, I, I, I, I, P],
+    "slb_moe_combine_bf16_sorted": [P, I, P, P, I, P, I, P, I, I, I, I, P],
+    "slb_moe_gather_bf16": [P, I, P, I, I, I, I, P, I, P],
+    "slb_router_logits_tile_bf16": [P, I, P, I, P, I, I, I, I, P],
 }
 
 # optional entry points: declared when the library exports them

@@ -204,3 +204,32 @@ def test_sum_of_two_norms_against_64_bits(dtype, n):
             for t, w in ((a, wa), (b, wb)))
     tol = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
     assert ((out.double() - 0.5 * (u + v)).abs() <= tol * (u + v).abs() + 2e-6 * (u.abs() + v.abs()) + 1e-7).all()
+
+
+# ------------------------------------------------------------------------- routed experts
+@pytest.mark.parametrize("M,E,Kd", [(512, 32, 2048), (513, 5, 32), (700, 33, 1056), (640, 64, 96)])
+def test_router_logits_of_many_tokens(M, E, Kd):
+    """Float32 sums of up to 2,048 products, an eighth of them at a time: 3e-7 of the result's norm."""
+    g = gen(M + E)
+    x, w = torch.randn(M, Kd + 8, device=DEV, generator=g).bfloat16()[:, :Kd], torch.randn(E, Kd, device=DEV, generator=g)
+    want = x.double() @ w.double().T
+    assert (K().router_logits(x, w).double() - want).norm() <= 1e-6 * want.norm()
+
+
+@pytest.mark.parametrize("P,E", [(1, 1), (3, 7), (256, 32), (8191, 32), (64, 1024), (20001, 60)])
+def test_plan_of_the_experts_rows(P, E):
+    from servelab_b200.ops import library as L
+    ids = torch.randint(0, E, (P,), device=DEV, dtype=torch.int32, generator=gen(P))
+    lib = L.core()
+    plan = torch.full((lib.slb_moe_plan_ints(P, E),), -7, dtype=torch.int32, device=DEV)
+    L.check(lib.slb_moe_plan(ids.data_ptr(), P, E, plan.data_ptr(), K()._stream()), "moe_plan")
+    tiles = -(-P // lib.slb_moe_tile_rows()) + E
+    p, counts = plan.cpu().long(), torch.bincount(ids.cpu().long(), minlength=E)
+    assert torch.equal(p[:E], counts) and torch.equal(p[E:2 * E + 1], torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+    at = 3 * E + 1
+    want = [(e, r) for e in range(E) for r in range(0, int(counts[e]), lib.slb_moe_tile_rows())]
+    got = list(zip(p[at:at + tiles].tolist(), p[at + tiles:at + 2 * tiles].tolist()))
+    assert got[:len(want)] == want and all(e == -1 for e, _ in got[len(want):])
+    order, where = p[at + 2 * tiles:at + 2 * tiles + P], p[at + 2 * tiles + P:]
+    assert len(where) == P and torch.equal(order.sort().values, torch.arange(P)) and torch.equal(where[order], torch.arange(P))
+    assert (ids.cpu().long()[order].diff() >= 0).all()
