@@ -31,6 +31,14 @@
 #define MOE_BN 64
 #define MOE_BK 16
 
+// Rows of a product's tile: few where an expert gets few, so that the tensor-core form's stages are small and
+// all its blocks are resident at once (the last wave of a second round is nearly empty).
+static int moe_tile_rows(int P, int E) { return P <= 8 * E ? 16 : P <= 40 * E ? 32 : MOE_BM; }
+static int moe_num_tiles(int P, int E) {
+    const int rows = moe_tile_rows(P, E);
+    return (P + rows - 1) / rows + E;
+}
+
 // ------------------------------------------------------------------- route
 __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 #pragma unroll
@@ -310,13 +318,13 @@ __global__ void __launch_bounds__(256) router_logits_tile_kernel(const bf16* __r
 
 // -------------------------------------------------------------------- plan
 // One block.  plan = [counts E | offsets E + 1 | unused E | tile_expert NT | tile_row0 NT |
-// sorted P | where P] (int32), NT = ceil(P / MOE_BM) + E; where[sorted[i]] = i.  Counts and ranks in
+// sorted P | where P] (int32), NT = ceil(P / tile rows) + E; where[sorted[i]] = i.  Counts and ranks in
 // shared memory, one atomic a pair; a thread works on PLAN_RUN pairs at a time with their loads in
 // flight together.  (Counting and sorting through atomics on global memory, the tiles listed by one
 // thread: 16.1 us for 8,192 pairs, 6.9 for 256.)
 #define PLAN_RUN 8
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ ids, int P, int E,
-                                                        int num_tiles, int* __restrict__ plan) {
+                                                        int num_tiles, int tile_rows, int* __restrict__ plan) {
     __shared__ int count[MOE_MAX_EXPERTS], start[MOE_MAX_EXPERTS];
     __shared__ int2 warp_total[32];
     int* offsets = plan + E;
@@ -339,7 +347,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
     }
     __syncthreads();
     // rows and tiles before every expert (thread = expert)
-    const int n = tid < E ? count[tid] : 0, tiles = (n + MOE_BM - 1) / MOE_BM;
+    const int n = tid < E ? count[tid] : 0, tiles = (n + tile_rows - 1) / tile_rows;
     int rows_upto = n, tiles_upto = tiles;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -365,7 +373,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
         if (tid == E - 1) offsets[E] = rows_upto;
         for (int i = 0; i < tiles; ++i) {
             tile_expert[tiles_upto - tiles + i] = tid;
-            tile_row0[tiles_upto - tiles + i] = i * MOE_BM;
+            tile_row0[tiles_upto - tiles + i] = i * tile_rows;
         }
     }
     for (int i = all_tiles + tid; i < num_tiles; i += 1024) tile_expert[i] = -1;
@@ -418,7 +426,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
 template <typename T, typename TC, int MODE>
 __global__ void __launch_bounds__(256) moe_product_kernel(
     const T* __restrict__ A, int lda, const T* __restrict__ W, long long w_expert_stride, int ldw,
-    TC* __restrict__ C, int ldc, const int* __restrict__ plan, int E, int num_tiles, int P, int top,
+    TC* __restrict__ C, int ldc, const int* __restrict__ plan, int E, int num_tiles, int tile_rows, int P, int top,
     int N, int K, int act, float limit, float alpha, const float* __restrict__ in_weights) {
     __shared__ __align__(16) float As[MOE_BK][MOE_BM + 4];
     __shared__ __align__(16) float Ws[MOE_BK][MOE_BN + 4];
@@ -433,7 +441,7 @@ __global__ void __launch_bounds__(256) moe_product_kernel(
     const int e = tile_expert[blockIdx.y];
     if (e < 0) return;
     const int r0 = tile_row0[blockIdx.y];
-    const int nrows = min(MOE_BM, counts[e] - r0);
+    const int nrows = min(tile_rows, counts[e] - r0);
     const int tid = threadIdx.x;
     if (tid < MOE_BM) rows[tid] = tid < nrows ? sorted[offsets[e] + r0 + tid] : -1;
     __syncthreads();
@@ -503,26 +511,31 @@ __global__ void __launch_bounds__(256) moe_product_kernel(
 }
 
 // ------------------------------------------------- products on tensor cores
-// The same two products in bfloat16 on mma.sync (m16n8k16, float32 accumulation): a block owns
+// The same two products in bfloat16 on mma.sync (m16n8k16, float32 accumulation): a block owns up to
 // 64 sorted rows of one expert and 64 output columns (MODE 0: 64 gate columns AND their 64 up
-// columns, the activation in the epilogue), a warp 16 rows; A rows (gathered by the plan) and W
-// rows arrive by 16-byte cp.async through a two-stage ring of 32-element k-blocks.  Rows, K and
-// the leading dimensions must be multiples of 8 elements.
-#define MM_BM 64
+// columns, the activation in the epilogue), a warp 16 of the columns and all the rows, so that a
+// fragment of the weights is read from shared memory once however many rows there are, and all four
+// warps have work when an expert has a handful of rows.  A rows (gathered by the plan; only those
+// that exist) and W rows arrive by 16-byte cp.async through a ring of STAGES k-blocks.  What bounds it at
+// few rows is the weights' way from memory: the ring keeps (STAGES - 1) k-blocks of every resident
+// block in flight.  Rows, K and the leading dimensions must be multiples of 8 elements.
 #define MM_BN 64
-#define MM_BK 32
-#define MM_LD (MM_BK + 8)
 
-template <int MODE>
+template <int MODE, int BM, int BK> struct MoeStage {
+    bf16 a[BM][BK + 8];
+    bf16 w[MODE == 0 ? 2 : 1][MM_BN][BK + 8];
+};
+
+template <int MODE, int BM, int BK, int STAGES>
 __global__ void __launch_bounds__(128) moe_product_mma_kernel(
     const bf16* __restrict__ A, int lda, const bf16* __restrict__ W, long long w_expert_stride, int ldw,
     void* __restrict__ Cv, int ldc, const int* __restrict__ plan, int E, int num_tiles, int top, int N,
     int K, int act, float limit, float alpha, const float* __restrict__ in_weights) {
     using namespace slb_mma;
-    __shared__ __align__(16) bf16 As[2][MM_BM][MM_LD];
-    __shared__ __align__(16) bf16 Ws[2][MM_BN][MM_LD];
-    __shared__ __align__(16) bf16 Us[MODE == 0 ? 2 : 1][MODE == 0 ? MM_BN : 1][MM_LD];
-    __shared__ int rows[MM_BM];
+    constexpr int NW = MODE == 0 ? 2 : 1, PIECES = BK / 8;
+    extern __shared__ __align__(16) unsigned char mm_smem[];
+    MoeStage<MODE, BM, BK>* ring = reinterpret_cast<MoeStage<MODE, BM, BK>*>(mm_smem);
+    __shared__ int rows[BM];
     pdl_wait();
     const int* counts = plan;
     const int* offsets = plan + E;
@@ -532,92 +545,93 @@ __global__ void __launch_bounds__(128) moe_product_mma_kernel(
     const int e = tile_expert[blockIdx.y];
     if (e < 0) return;
     const int r0 = tile_row0[blockIdx.y];
-    const int nrows = min(MM_BM, counts[e] - r0);
+    const int nrows = min(BM, counts[e] - r0);
+    const int mtiles = (nrows + 15) >> 4;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid < MM_BM) rows[tid] = tid < nrows ? sorted[offsets[e] + r0 + tid] : -1;
+    if (tid < BM) rows[tid] = tid < nrows ? sorted[offsets[e] + r0 + tid] : -1;
     __syncthreads();
     const bf16* We = W + (size_t)e * w_expert_stride;
     const int n0 = blockIdx.x * MM_BN;
 
-    auto load = [&](int stage, int k0) {
-        // 64 rows x 4 chunks of 8 elements for each of A, W (and U)
-        for (int idx = tid; idx < MM_BM * 4; idx += 128) {
-            const int r = idx >> 2, c = idx & 3;
-            const int gk = k0 + c * 8;
-            const int pr = rows[r];
-            const bool oka = pr >= 0 && gk < K;
-            cp_async16(&As[stage][r][c * 8], A + (oka ? (size_t)(MODE == 0 ? pr / top : pr) * lda + gk : 0), oka);
-            const bool okw = n0 + r < N && gk < K;
-            cp_async16(&Ws[stage][r][c * 8], We + (okw ? (size_t)(n0 + r) * ldw + gk : 0), okw);
-            if (MODE == 0)
-                cp_async16(&Us[stage][r][c * 8], We + (okw ? (size_t)(N + n0 + r) * ldw + gk : 0), okw);
+    auto load = [&](int kb) {
+        MoeStage<MODE, BM, BK>& st = ring[kb % STAGES];
+        const int k0 = kb * BK;
+#pragma unroll
+        for (int idx = tid; idx < NW * MM_BN * PIECES; idx += 128) {
+            const int r = idx / PIECES, c = (idx % PIECES) * 8, u = r / MM_BN, n = n0 + r % MM_BN;
+            const bool ok = n < N && k0 + c < K;
+            cp_async16(&st.w[u][r % MM_BN][c], We + (ok ? (size_t)(u * N + n) * ldw + k0 + c : 0), ok);
+        }
+        for (int idx = tid; idx < mtiles * 16 * PIECES; idx += 128) {
+            const int r = idx / PIECES, c = (idx % PIECES) * 8, pr = rows[r];
+            const bool ok = pr >= 0 && k0 + c < K;
+            cp_async16(&st.a[r][c], A + (ok ? (size_t)(MODE == 0 ? pr / top : pr) * lda + k0 + c : 0), ok);
         }
     };
 
-    float acc[MM_BN / 8][4], acu[MODE == 0 ? MM_BN / 8 : 1][4];
+    float acc[NW][BM / 16][2][4];
 #pragma unroll
-    for (int j = 0; j < MM_BN / 8; ++j)
+    for (int u = 0; u < NW; ++u)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) acc[j][x] = 0.f;
+        for (int m = 0; m < BM / 16; ++m)
 #pragma unroll
-    for (int j = 0; j < (MODE == 0 ? MM_BN / 8 : 1); ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) acu[j][x] = 0.f;
+                for (int x = 0; x < 4; ++x) acc[u][m][j][x] = 0.f;
 
-    const int nk = (K + MM_BK - 1) / MM_BK;
-    load(0, 0);
-    cp_async_commit();
-    const bool active = warp * 16 < nrows;
+    const int nk = (K + BK - 1) / BK;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < nk) load(s);
+        cp_async_commit();
+    }
     for (int kb = 0; kb < nk; ++kb) {
-        if (kb + 1 < nk) {
-            load((kb + 1) & 1, (kb + 1) * MM_BK);
-            cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const int st = kb & 1;
-        if (active) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                                   // block kb is there; block kb - 1 has been read by all
+        if (kb + STAGES - 1 < nk) load(kb + STAGES - 1);
+        cp_async_commit();
+        const MoeStage<MODE, BM, BK>& st = ring[kb % STAGES];
 #pragma unroll
-            for (int kk = 0; kk < MM_BK / 16; ++kk) {
+        for (int kk = 0; kk < BK / 16; ++kk) {
+            unsigned b[NW][4];
+#pragma unroll
+            for (int u = 0; u < NW; ++u)
+                ldmatrix_x4(b[u], &st.w[u][warp * 16 + (lane >> 4) * 8 + (lane & 7)][kk * 16 + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+            for (int m = 0; m < BM / 16; ++m) {
+                if (m >= mtiles) break;
                 unsigned a[4];
-                ldmatrix_x4(a, &As[st][warp * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]);
+                ldmatrix_x4(a, &st.a[m * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]);
 #pragma unroll
-                for (int jp = 0; jp < MM_BN / 16; ++jp) {
-                    unsigned b[4];
-                    ldmatrix_x4(b, &Ws[st][jp * 16 + (lane >> 4) * 8 + (lane & 7)][kk * 16 + ((lane >> 3) & 1) * 8]);
-                    mma_bf16(acc[2 * jp], a, b[0], b[1]);
-                    mma_bf16(acc[2 * jp + 1], a, b[2], b[3]);
-                    if (MODE == 0) {
-                        ldmatrix_x4(b, &Us[st][jp * 16 + (lane >> 4) * 8 + (lane & 7)][kk * 16 + ((lane >> 3) & 1) * 8]);
-                        mma_bf16(acu[2 * jp], a, b[0], b[1]);
-                        mma_bf16(acu[2 * jp + 1], a, b[2], b[3]);
-                    }
+                for (int u = 0; u < NW; ++u) {
+                    mma_bf16(acc[u][m][0], a, b[u][0], b[u][1]);
+                    mma_bf16(acc[u][m][1], a, b[u][2], b[u][3]);
                 }
             }
         }
-        __syncthreads();
     }
-    if (!active) return;
     const int tig = lane & 3;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int pr = rows[warp * 16 + (lane >> 2) + 8 * h];
-        if (pr < 0) continue;
-        const float iw = MODE == 0 && in_weights != nullptr ? in_weights[pr] : 1.f;
+    for (int m = 0; m < BM / 16; ++m) {
+        if (m >= mtiles) break;
 #pragma unroll
-        for (int j = 0; j < MM_BN / 8; ++j) {
-            const int gn = n0 + j * 8 + tig * 2;
-            if (gn >= N) continue;                        // (N is even: both columns exist or neither)
-            float v0 = acc[j][2 * h], v1 = acc[j][2 * h + 1];
-            if (MODE == 0) {
-                auto rounded = [&](float x) { return __bfloat162float(__float2bfloat16_rn(x * iw)); };
-                v0 = act_mul_of(act, rounded(v0), rounded(acu[j][2 * h]), limit, alpha);
-                v1 = act_mul_of(act, rounded(v1), rounded(acu[j][2 * h + 1]), limit, alpha);
-                *reinterpret_cast<unsigned*>(reinterpret_cast<bf16*>(Cv) + (size_t)pr * ldc + gn) = pack_bf16(v0, v1);
-            } else {
-                *reinterpret_cast<float2*>(reinterpret_cast<float*>(Cv) + (size_t)pr * ldc + gn) = make_float2(v0, v1);
+        for (int h = 0; h < 2; ++h) {
+            const int pr = rows[m * 16 + (lane >> 2) + 8 * h];
+            if (pr < 0) continue;
+            const float iw = MODE == 0 && in_weights != nullptr ? in_weights[pr] : 1.f;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int gn = n0 + warp * 16 + j * 8 + tig * 2;
+                if (gn >= N) continue;                    // (N is even: both columns exist or neither)
+                float v0 = acc[0][m][j][2 * h], v1 = acc[0][m][j][2 * h + 1];
+                if (MODE == 0) {
+                    auto rounded = [&](float x) { return __bfloat162float(__float2bfloat16_rn(x * iw)); };
+                    v0 = act_mul_of(act, rounded(v0), rounded(acc[NW - 1][m][j][2 * h]), limit, alpha);
+                    v1 = act_mul_of(act, rounded(v1), rounded(acc[NW - 1][m][j][2 * h + 1]), limit, alpha);
+                    *reinterpret_cast<unsigned*>(reinterpret_cast<bf16*>(Cv) + (size_t)pr * ldc + gn) = pack_bf16(v0, v1);
+                } else {
+                    *reinterpret_cast<float2*>(reinterpret_cast<float*>(Cv) + (size_t)pr * ldc + gn) = make_float2(v0, v1);
+                }
             }
         }
     }
@@ -720,7 +734,6 @@ static int launch_moe_combine(const TY* y, int ldy, const float* weights, const 
     return slb_launch(moe_combine_kernel<T, TY, 1>, grid, dim3(256), 0, st, y, ldy, weights, shared, lds, out, ldo, top, N, where);
 }
 
-static int moe_num_tiles(int P, int E) { return (P + MOE_BM - 1) / MOE_BM + E; }
 
 template <typename T>
 static int launch_moe_gate_up(const T* x, int ldx, const T* w_gu, int ldw, T* out, int lda,
@@ -731,7 +744,7 @@ static int launch_moe_gate_up(const T* x, int ldx, const T* w_gu, int ldw, T* ou
     const int nt = moe_num_tiles(P, E);
     if (nt > 65535) return SLB_ERR_TOO_LARGE;
     return slb_launch(moe_product_kernel<T, T, 0>, dim3((I + MOE_BN - 1) / MOE_BN, nt), dim3(256), 0, st, x,
-                      ldx, w_gu, (long long)2 * I * ldw, ldw, out, lda, plan, E, nt, P, top, I, K, act, limit, alpha, in_weights);
+                      ldx, w_gu, (long long)2 * I * ldw, ldw, out, lda, plan, E, nt, moe_tile_rows(P, E), P, top, I, K, act, limit, alpha, in_weights);
 }
 
 template <typename T>
@@ -742,7 +755,7 @@ static int launch_moe_down(const T* act, int lda, const T* w_down, int ldw, floa
     const int nt = moe_num_tiles(P, E);
     if (nt > 65535) return SLB_ERR_TOO_LARGE;
     return slb_launch(moe_product_kernel<T, float, 1>, dim3((N + MOE_BN - 1) / MOE_BN, nt), dim3(256), 0, st,
-                      act, lda, w_down, (long long)N * ldw, ldw, y, ldy, plan, E, nt, P, top, N, I, 0, 0.f, 0.f, (const float*)nullptr);
+                      act, lda, w_down, (long long)N * ldw, ldw, y, ldy, plan, E, nt, moe_tile_rows(P, E), P, top, N, I, 0, 0.f, 0.f, (const float*)nullptr);
 }
 
 template <int MODE>
@@ -755,8 +768,27 @@ static int launch_moe_mma(const bf16* A, int lda, const bf16* W, long long strid
         return SLB_ERR_BAD_ARG;
     const int nt = moe_num_tiles(P, E);
     if (nt > 65535) return SLB_ERR_TOO_LARGE;
-    return slb_launch(moe_product_mma_kernel<MODE>, dim3((N + MM_BN - 1) / MM_BN, nt), dim3(128), 0, st, A, lda,
-                      W, stride, ldw, C, ldc, plan, E, nt, top, N, K, act, limit, alpha, in_weights);
+    const dim3 grid((N + MM_BN - 1) / MM_BN, nt);
+#define MMF(BM, BK, ST)                                                                                               \
+    do {                                                                                                              \
+        static unsigned long long configured = 0;                                                                     \
+        constexpr size_t smem = sizeof(MoeStage<MODE, BM, BK>) * ST;                                                  \
+        const int rc = slb_configure(&configured, moe_product_mma_kernel<MODE, BM, BK, ST>, smem);                    \
+        if (rc != 0) return rc;                                                                                       \
+        return slb_launch(moe_product_mma_kernel<MODE, BM, BK, ST>, grid, dim3(128), smem, st, A, lda, W, stride, ldw, \
+                          C, ldc, plan, E, nt, top, N, K, act, limit, alpha, in_weights);                             \
+    } while (0)
+    // Measured us, gate|up and down, 32 experts of 2,048 x 1,408 of 1 / 16 / 64 / 128 / 250 / 1,000 tokens, 4 experts
+    // each: two stages of 32 with rows of warps and tiles of 64 rows 45.6 + 19.5 / 68.5 + 41.3 / 88.2 + 45.7 / 97.5 + 51.0
+    // / 111 + 56 / 275 + 126; as below 20.2 + 13.5 / 57.0 + 32.5 / 70.1 + 38.1 / 86.9 + 49.5 / 114 + 53 / 244 + 129.  (At
+    // 64 tokens 369 + 185 MB of weights: 56 + 28 us of the measured bandwidth.)  A third stage pays while few blocks
+    // are resident, or while a block computes for long.
+    const int rows = moe_tile_rows(P, E);
+    if (rows == 16 && P <= E) MMF(16, 64, 3);
+    if (rows == 16) MMF(16, 64, 2);
+    if (rows == 32) MMF(32, 64, 3);
+    MMF(64, 64, 2);
+#undef MMF
 }
 
 extern "C" {
@@ -769,7 +801,7 @@ int slb_moe_down_mma_bf16(const bf16* act, int lda, const bf16* w_down, int ldw,
                           const int* plan, int E, int P, int top, int N, int I, cudaStream_t st) {
     return launch_moe_mma<1>(act, lda, w_down, (long long)N * ldw, ldw, y, ldy, plan, E, P, top, N, I, st);
 }
-int slb_moe_tile_rows() { return MOE_BM; }
+int slb_moe_tile_rows(int P, int E) { return moe_tile_rows(P, E); }
 static int launch_moe_route(const float* logits, int ldl, int T, int E, int groups, int keep, int top,
                             float route_scale, int renormalize, int score_fn, const float* correction,
                             int group_best, float norm_eps, int* ids, float* weights, cudaStream_t st) {
@@ -829,7 +861,7 @@ int slb_moe_plan_ints(int P, int E) { return 3 * E + 1 + 2 * moe_num_tiles(P, E)
 int slb_moe_plan(const int* ids, int P, int E, int* plan, cudaStream_t st) {
     if (P <= 0) return 0;
     if (E <= 0 || E > MOE_MAX_EXPERTS) return SLB_ERR_BAD_ARG;
-    return slb_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, st, ids, P, E, moe_num_tiles(P, E), plan);
+    return slb_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, st, ids, P, E, moe_num_tiles(P, E), moe_tile_rows(P, E), plan);
 }
 int slb_moe_gate_up_f32(const float* x, int ldx, const float* w_gu, int ldw, float* out, int lda,
                         const int* plan, int E, int P, int top, int I, int K, int act, float limit, float alpha,

@@ -99,7 +99,7 @@ _CORE_SIGNATURES = {
     "slb_delta_chunk_bf16": [P, I, P],
     "slb_gated_recurrence_f32": [P, I, I, P],
     "slb_gated_recurrence_bf16": [P, I, I, P],
-    "slb_moe_tile_rows": [],
+    "slb_moe_tile_rows": [I, I],
     "slb_moe_route": [P, I, I, I, I, I, I, F, I, P, P, P],
     "slb_moe_route_scored": [P, I, I, I, I, I, I, F, I, I, P, I, F, P, P, P],
     "slb_gated_act_f32": [P, P, I, I, I, I, I, I, F, F, P, P],

@@ -223,13 +223,38 @@ def test_plan_of_the_experts_rows(P, E):
     lib = L.core()
     plan = torch.full((lib.slb_moe_plan_ints(P, E),), -7, dtype=torch.int32, device=DEV)
     L.check(lib.slb_moe_plan(ids.data_ptr(), P, E, plan.data_ptr(), K()._stream()), "moe_plan")
-    tiles = -(-P // lib.slb_moe_tile_rows()) + E
+    rows = lib.slb_moe_tile_rows(P, E)
+    tiles = -(-P // rows) + E
     p, counts = plan.cpu().long(), torch.bincount(ids.cpu().long(), minlength=E)
     assert torch.equal(p[:E], counts) and torch.equal(p[E:2 * E + 1], torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
     at = 3 * E + 1
-    want = [(e, r) for e in range(E) for r in range(0, int(counts[e]), lib.slb_moe_tile_rows())]
+    want = [(e, r) for e in range(E) for r in range(0, int(counts[e]), rows)]
     got = list(zip(p[at:at + tiles].tolist(), p[at + tiles:at + 2 * tiles].tolist()))
     assert got[:len(want)] == want and all(e == -1 for e, _ in got[len(want):])
     order, where = p[at + 2 * tiles:at + 2 * tiles + P], p[at + 2 * tiles + P:]
     assert len(where) == P and torch.equal(order.sort().values, torch.arange(P)) and torch.equal(where[order], torch.arange(P))
     assert (ids.cpu().long()[order].diff() >= 0).all()
+
+
+@pytest.mark.parametrize("T,E,top,h,I", [(1, 8, 2, 64, 40), (3, 4, 4, 128, 72), (33, 8, 2, 200, 64), (64, 8, 2, 64, 136),
+                                         (100, 5, 3, 72, 64), (300, 4, 2, 128, 64)])
+def test_experts_products_at_few_and_many_rows(T, E, top, h, I):
+    """Tiles of 16, 32 and 64 rows (up to 8, 40 and more rows an expert) against 64 bits: two roundings to bfloat16 of
+    the first product, one of the activation, one of the result."""
+    g = gen(T)
+    x = torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    if T > 50:
+        ids[:, 0] = 1                                     # one expert with more rows than a tile
+        ids[:, 1:] = torch.where(ids[:, 1:] == 1, 0, ids[:, 1:])
+    w = torch.rand(T, top, device=DEV, generator=g)
+    got = K().moe_experts(x, ids, w, wg, wd, None).double()
+    want = torch.zeros_like(got)
+    for t in range(T):
+        for k in range(top):
+            e = int(ids[t, k])
+            gu = wg[e].double() @ x[t].double()
+            act = gu[:I] * torch.sigmoid(gu[:I]) * gu[I:]
+            want[t] += w[t, k].double() * (wd[e].double() @ act)
+    assert (got - want).norm() <= 2.0 ** -7 * want.norm()
