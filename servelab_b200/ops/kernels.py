@@ -1470,8 +1470,7 @@ class _DecayChunkArgs(_ct.Structure):
 
 class _GatedChunkArgs(_ct.Structure):
     _fields_ = [("a", _DecayAttnArgs), ("tile_seq", _ct.c_void_p), ("tile_row0", _ct.c_void_p),
-                ("num_tiles", _ct.c_int), ("work", _ct.c_void_p), ("qdec", _ct.c_void_p), ("kdec", _ct.c_void_p),
-                ("dtot", _ct.c_void_p), ("scores", _ct.c_void_p)]
+                ("num_tiles", _ct.c_int), ("work", _ct.c_void_p)]
 
 
 # Learned decays: steps that bring portions of prompts in bfloat16 take the chunked kernels (float32
@@ -1533,17 +1532,13 @@ def decay_attention(proj: torch.Tensor, ctx, state: torch.Tensor, decay: Optiona
         c = _GatedChunkArgs()
         c.a = a
         c.tile_seq, c.tile_row0, c.num_tiles = tile_seq.data_ptr(), tile_row0.data_ptr(), n
-        dev = proj.device
-        work = torch.empty((max(n, 1), num_heads, head_dim, value_dim), dtype=_F32, device=dev)
-        qk_dec = torch.empty((2, proj.shape[0], num_heads * head_dim), dtype=_F32, device=dev)
-        dtot = torch.empty((max(n, 1), num_heads, head_dim), dtype=_F32, device=dev)
-        scores = torch.empty((max(n, 1), num_heads, chunk, chunk), dtype=_F32, device=dev)
-        c.work, c.dtot, c.scores = work.data_ptr(), dtot.data_ptr(), scores.data_ptr()
-        c.qdec, c.kdec = qk_dec[0].data_ptr(), qk_dec[1].data_ptr()
+        work = torch.empty((max(n, 1), num_heads, L.core().slb_decay_gated_chunk_work_floats(head_dim)), dtype=_F32,
+                           device=proj.device)
+        c.work = work.data_ptr()
         fn = getattr(L.core(), "slb_decay_gated_chunk_" + _suffix(proj.dtype))
         L.check(fn(_ct.byref(c), ctx.num_seqs, _stream()), "decay_attention (gated chunks)")
         global launch_count
-        launch_count += 3
+        launch_count += 1
         return
     if (decay_attention_chunked and plain and proj.dtype == torch.bfloat16 and not ctx.decode_only
             and head_dim <= L.core().slb_decay_chunk_max_dim()
