@@ -288,17 +288,18 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const DeltaChunkA
     // the values of a chunk: two (token, column) pairs a thread, kept in registers on their way
     const T* vp = reinterpret_cast<const T*>(a.proj) + (size_t)q0 * a.ld + a.v_off + h * Dv + e0;
     const int ve = tid % DC_EV, vj = tid / DC_EV;
-    float v0, v1;
+    T v0, v1;                                        // (as they lie in memory: a conversion would wait for the load)
     auto load_v = [&](int k) {
         const int t = k * DC_C + vj;
         const bool live = e0 + ve < Dv;
-        v0 = live && t < qlen ? to_float(vp[(size_t)t * a.ld + ve]) : 0.f;
-        v1 = live && t + 16 < qlen ? to_float(vp[(size_t)(t + 16) * a.ld + ve]) : 0.f;
+        v0 = v1 = from_float<T>(0.f);
+        if (live && t < qlen) v0 = vp[(size_t)t * a.ld + ve];
+        if (live && t + 16 < qlen) v1 = vp[(size_t)(t + 16) * a.ld + ve];
     };
     auto store_v = [&](int k) {
         float* Vt = Vts + (k & 1) * DC_EV * DC_LM + ve * DC_LM + vj;
-        Vt[0] = v0;
-        Vt[16] = v1;
+        Vt[0] = to_float(v0);
+        Vt[16] = to_float(v1);
     };
     load_v(0);
     store_v(0);
@@ -386,11 +387,11 @@ static int launch_delta_chunk(const DeltaChunkArgs& c, int num_seqs, cudaStream_
     if (a.D <= 128) {
         rc = slb_configure(&conf2, delta_chunk_scan_kernel<T, 2>, dc_scan_smem(128, 2));
         if (rc != 0) return rc;
-        return slb_launch(delta_chunk_scan_kernel<T, 2>, dim3(num_seqs, a.H, vz), dim3(256), dc_scan_smem(a.D, 2), st, c);
+        return slb_launch_after(delta_chunk_scan_kernel<T, 2>, dim3(num_seqs, a.H, vz), dim3(256), dc_scan_smem(a.D, 2), st, c);
     }
     rc = slb_configure(&conf3, delta_chunk_scan_kernel<T, 1>, dc_scan_smem(DR_MAX_D, 1));
     if (rc != 0) return rc;
-    return slb_launch(delta_chunk_scan_kernel<T, 1>, dim3(num_seqs, a.H, vz), dim3(256), dc_scan_smem(a.D, 1), st, c);
+    return slb_launch_after(delta_chunk_scan_kernel<T, 1>, dim3(num_seqs, a.H, vz), dim3(256), dc_scan_smem(a.D, 1), st, c);
 }
 
 extern "C" {
