@@ -258,3 +258,25 @@ def test_experts_products_at_few_and_many_rows(T, E, top, h, I):
             act = gu[:I] * torch.sigmoid(gu[:I]) * gu[I:]
             want[t] += w[t, k].double() * (wd[e].double() @ act)
     assert (got - want).norm() <= 2.0 ** -7 * want.norm()
+
+
+# ------------------------------------------------------- state space in chunks
+@pytest.mark.parametrize("lens", [[17], [63, 64], [65, 16, 200], [130, 1, 700]])
+@pytest.mark.parametrize("H,P,N,G", [(4, 64, 128, 2), (2, 72, 64, 1), (3, 8, 64, 3), (2, 136, 128, 1)])
+def test_chunks_in_pieces_are_those_of_the_general_kernels(H, P, N, G, lens):
+    """Rows at an odd address go to the general kernels, whose weighted x is rounded in another order before its split
+    (2^-17 of every term)."""
+    g, T = gen(H + len(lens)), sum(lens)
+    ctx, _ = step(lens)
+    rows = torch.randn(T, H * P + 2 * G * N, device=DEV, generator=g).bfloat16()
+    dt, bias = torch.randn(T, H, device=DEV, generator=g) - 2, torch.randn(H, device=DEV, generator=g)
+    rate, skip = torch.rand(H, device=DEV, generator=g) * 4 + 0.1, torch.randn(H, device=DEV, generator=g)
+    record = torch.randn(len(lens), H * N * P + 4, device=DEV, generator=g)
+    got = []
+    for u in (rows, odd_view(rows)):
+        state, out = record.clone(), torch.zeros(T, H * P, device=DEV)
+        K().state_space(ctx, u, dt, state, out, num_heads=H, value_dim=P, state_dim=N, groups=G, dt_bias=bias, rate=rate,
+                        skip=skip)
+        got.append((out, state))
+    for a, b in zip(*got):
+        assert (a - b).norm() <= 2.0 ** -17 * b.norm() and b.norm() > 0
