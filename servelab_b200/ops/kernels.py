@@ -536,7 +536,9 @@ decode_ws_force_splits = 0     # measurements: launch this many splits instead o
 # about 3 us).  In the arrival-counter form (the twin) a split has about
 # `decode_ws_split_coef` * sqrt(tiles) tiles: there one block combines every split.
 decode_ws_split_coef = 0.8
-decode_ws_unsplit_tiles = 6    # (us at 256 / 512 keys, batch 8: 5.4 / 8.4 with 12, 5.4 / 6.0 with 6, 5.9 / 6.0 with 3)
+decode_ws_unsplit_tiles = 4    # (us at 256 / 512 keys, batch 8: 5.4 / 8.4 with 12, 5.4 / 6.0 with 6, 5.9 / 6.0 with 3; 8
+                               # layers of the 0.5B shape at batch 8, 230 / 300 / 360 keys: 239 / 247 / 254 us a step
+                               # with 6, 237 / 236 / 238 with 4)
 
 _DECODE_COUNTERS = 1 << 16     # arrival counters held per device (256 KiB)
 _decode_counters: Dict[int, torch.Tensor] = {}
@@ -683,7 +685,11 @@ def tc_decode_splits(n_out: int, k: int, groups: int = 1) -> int:
     kblocks = -(-k // 64)
     slots = tc_blocks_per_sm * _num_sms()
     want = max(1, slots // tiles) if tiles < slots else 1      # all blocks resident at once
-    return max(1, min(want, kblocks // 4 if kblocks >= 8 else 1))
+    # a split streams two k-blocks at least: what a narrow product of a small model takes is the wait for its first
+    # tiles and the way through its epilogue, so fewer k-blocks a block pay although more results are added (8 layers
+    # of the 0.5B shape at batch 1 / 8 / 32 / 64 with four at least: 232 / 262 / 284 / 311 us a step, with two 219 /
+    # 247 / 274 / 305, with one 219 / 238 / 277 / -; the 7B shape's products have enough row tiles)
+    return max(1, min(want, kblocks // 2 if kblocks >= 8 else 1))
 
 
 # rows of gates, then as many of ups, and so on: the layout for which the tcgen05 product
