@@ -28,7 +28,7 @@
 // tp_model.py:48-53,67-68,115-119), left to the library there.
 #include <cuda.h>
 
-#include "common.cuh"
+#include "gated_act.cuh"
 
 namespace {
 
@@ -439,7 +439,9 @@ __global__ void gemm_tc_reduce_kernel(const float* __restrict__ partial, TO* __r
 //              stream (the norm on the branch's result), and z[tok, n] = bfloat16(tanh(*pre_alpha *
 //              resid[tok, n]) * norm_weight[n] + pre_b[n]) is the finished normed row of the next
 //              sublayer; no sums of squares are written and the consumer applies no factor.
-enum { EPI_STORE = 0, EPI_ROPE = 1, EPI_RESID = 2, EPI_DYT = 3 };      // EPI_DYT: EPI_RESID in Dynamic Tanh mode
+//   EPI_SWIGLU: W's rows are gates and ups alternating in runs of 64 (a tile holds 64 pairs): the products are
+//              rounded to bfloat16, then out[tok, n / 2] = silu(gate) up, as the activation's own kernel does it
+enum { EPI_STORE = 0, EPI_ROPE = 1, EPI_RESID = 2, EPI_DYT = 3, EPI_SWIGLU = 4 };      // EPI_DYT: EPI_RESID in Dynamic Tanh mode
 #define EPI_IS_RESID(e) ((e) == EPI_RESID || (e) == EPI_DYT)
 
 struct ResidEpilogue {
@@ -843,6 +845,14 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
                 for (int c = 0; c < 4; ++c) v[c] += (&bs.x)[c];
                 if constexpr (EPI == EPI_STORE) {
                     if (in) store4_bf16(out + (size_t)tok * ldo + n4, v);
+                } else if constexpr (EPI == EPI_SWIGLU) {
+                    float act[4];                         // (lanes 0..15: gates, 16..31: the ups of the same pairs)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float mine = __bfloat162float(__float2bfloat16_rn(v[c]));
+                        act[c] = silu_mul_fast(mine, __shfl_down_sync(0xffffffffu, mine, 16));
+                    }
+                    if (lane < 16) store4_bf16(out + (size_t)tok * ldo + (n0 >> 1) + r4, act);
                 } else if constexpr (EPI_IS_RESID(EPI)) {
                     float sq = 0.f;
                     if (in) {
@@ -953,6 +963,13 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
             if (rs.sumsq != nullptr) sum *= rstd_s[tok];
             if constexpr (EPI == EPI_STORE) {
                 if (n < N) out[(size_t)tok * ldo + n] = __float2bfloat16_rn(sum + (bias ? bias[n] : 0.f));
+            } else if constexpr (EPI == EPI_SWIGLU) {
+                pair_vals[parity][row] = __bfloat162float(__float2bfloat16_rn(sum));
+                asm volatile("bar.sync 1, 128;" ::: "memory");           // the four epilogue warps
+                if (row < 64)
+                    out[(size_t)tok * ldo + (n0 >> 1) + row] =
+                        __float2bfloat16_rn(silu_mul_fast(pair_vals[parity][row], pair_vals[parity][row + 64]));
+                parity ^= 1;
             } else if constexpr (EPI_IS_RESID(EPI)) {
                 float r = 0.f;
                 if (n < N) {
@@ -1106,7 +1123,7 @@ int run_cluster(const bf16* x, int ldx, const bf16* W, int ldw, bf16* out, int l
         return p == nullptr || ((uintptr_t)p % bytes == 0 && ((size_t)ld * elem_bytes) % bytes == 0);
     };
     bool wide_ok = N % 4 == 0 && aligned(bias, 0, 4, 16);
-    if (EPI == EPI_STORE) wide_ok = wide_ok && aligned(out, ldo, 2, 8);
+    if (EPI == EPI_STORE || EPI == EPI_SWIGLU) wide_ok = wide_ok && aligned(out, ldo, 2, 8);
     if (EPI_IS_RESID(EPI))
         wide_ok = wide_ok && aligned(res.resid, res.ld, 4, 16) && aligned(res.z, res.ldz, 2, 8) &&
                   aligned(res.norm_weight, 0, 4, 16);
@@ -1162,17 +1179,20 @@ int check_cluster_args(const bf16* x, int ldx, const bf16* W, int ldw, int M, in
 extern "C" {
 
 // out[M, N] = x . W^T (+ bias), bfloat16, the K splits of a row tile as one cluster (at most 8):
-// no workspace, no second kernel.  scale_sumsq: as for slb_gemm_tc_decode_bf16.
+// no workspace, no second kernel.  scale_sumsq, swiglu: as for slb_gemm_tc_decode_bf16.
 int slb_gemm_tc_cluster_bf16(const bf16* x, int ldx, const bf16* W, int ldw, bf16* out, int ldo,
-                             const float* bias, int M, int N, int K, int splits, int max_stages,
+                             const float* bias, int M, int N, int K, int splits, int max_stages, int swiglu,
                              const float* scale_sumsq, int scale_tiles, float scale_eps, int tok_group,
                              cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
-    if (ldo < N || out == nullptr) return SLB_ERR_BAD_ARG;
+    if (ldo < (swiglu ? N / 2 : N) || out == nullptr || (swiglu && (N % TC_BM || bias != nullptr))) return SLB_ERR_BAD_ARG;
     const int rc = check_cluster_args(x, ldx, W, ldw, M, N, K, splits, tok_group);
     if (rc != 0) return rc;
     if (scale_sumsq != nullptr && scale_tiles <= 0) return SLB_ERR_BAD_ARG;
     const RowScale rs = {scale_sumsq, scale_tiles, (float)K, scale_eps};
+    if (swiglu)
+        return run_cluster<EPI_SWIGLU>(x, ldx, W, ldw, out, ldo, nullptr, M, N, K, splits, max_stages, RopeEpilogue{},
+                                       ResidEpilogue{}, rs, tok_group, st);
     return run_cluster<EPI_STORE>(x, ldx, W, ldw, out, ldo, bias, M, N, K, splits, max_stages, RopeEpilogue{},
                                   ResidEpilogue{}, rs, tok_group, st);
 }

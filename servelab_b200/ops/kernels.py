@@ -752,7 +752,7 @@ def tc_cluster_splits(n_out: int, k: int, groups: int = 1) -> int:
 
 
 def gemm_tc_cluster(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
-                    bias: Optional[torch.Tensor] = None, splits: int = 0) -> torch.Tensor:
+                    bias: Optional[torch.Tensor] = None, splits: int = 0, swiglu: bool = False) -> torch.Tensor:
     """out[M,N] = x . w^T (+ bias) in bfloat16 for up to 64 tokens, like
     ``gemm_tc_decode``, but the K splits of a row tile form a thread-block cluster and
     add their results up through one another's shared memory: no partial sums in
@@ -764,10 +764,10 @@ def gemm_tc_cluster(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     groups = tc_token_groups(M, w)
     splits = splits or tc_cluster_splits(N, Kd, groups)
     if out is None:
-        out = torch.empty((M, N), dtype=_BF16, device=x.device)
+        out = torch.empty((M, N // 2 if swiglu else N), dtype=_BF16, device=x.device)
     L.check(L.core().slb_gemm_tc_cluster_bf16(
         x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _p(bias),
-        M, N, Kd, splits, _cluster_stages(M, groups), sumsq, tiles, eps,
+        M, N, Kd, splits, _cluster_stages(M, groups), 1 if swiglu else 0, sumsq, tiles, eps,
         tc_token_group if groups > 1 else 0, _stream()), "gemm_tc_cluster")
     return out
 

@@ -280,3 +280,16 @@ def test_chunks_in_pieces_are_those_of_the_general_kernels(H, P, N, G, lens):
         got.append((out, state))
     for a, b in zip(*got):
         assert (a - b).norm() <= 2.0 ** -17 * b.norm() and b.norm() > 0
+
+
+# ------------------------------------------------ activation in the cluster product's epilogue
+@pytest.mark.parametrize("M", [1, 2, 16, 17, 40, 64])
+@pytest.mark.parametrize("inter,Kd,splits", [(64, 512, 2), (192, 1024, 8), (128, 520, 3)])
+def test_cluster_product_with_activation_is_product_then_activation(M, inter, Kd, splits):
+    g = gen(M + inter)
+    x, w = torch.randn(M, Kd, device=DEV, generator=g).bfloat16(), (torch.randn(2 * inter, Kd, device=DEV, generator=g) * 0.05).bfloat16()
+    fused = K().gemm_tc_cluster(x, w, splits=splits, swiglu=True)
+    gu, act = K().gemm_tc_cluster(x, w, splits=splits), torch.empty(M, inter, device=DEV, dtype=torch.bfloat16)
+    K().swiglu(gu, act, K().SWIGLU_BLOCK)
+    assert torch.equal(fused, act) and act.float().abs().max() > 0
+    assert K().gemm_tc_status() == 0
