@@ -293,3 +293,20 @@ def test_cluster_product_with_activation_is_product_then_activation(M, inter, Kd
     K().swiglu(gu, act, K().SWIGLU_BLOCK)
     assert torch.equal(fused, act) and act.float().abs().max() > 0
     assert K().gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("D", [60, 64, 68, 128])
+@pytest.mark.parametrize("Hh,Dv", [(1, 8), (2, 20), (6, 200)])
+def test_walk_over_the_chunks_against_the_recurrence(D, Hh, Dv):
+    """Both widths of a slice of value columns (few and many slices in the launch), the key sizes with loops of
+    fixed length and their neighbours.  float32 sums of at most 70 x D products against 64 bits: 3e-5 of the
+    largest value, the bound the other sizes are held to."""
+    import test_gpu_sumolorn as case
+    from servelab_b200.ops import kernels
+    lens = [31, 32, 70]
+    proj, z, bias = case._gated_case(5, Hh, D, Dv, sum(lens), torch.bfloat16, z_shift=1.0)
+    want = case._gated_want(proj, z, bias, Hh, D, Dv, lens, 4.0, D ** -0.5)
+    state = torch.zeros(3, Hh * D * Dv, device="cuda")
+    out = case._run_gated_chunked(kernels, proj.cuda(), z.cuda(), bias.cuda(), state, Hh, D, Dv,
+                                  [[(0, 0, 31), (1, 31, 32), (2, 63, 70)]], 4.0, D ** -0.5)
+    assert (out.double().cpu() - want).abs().max() < 3e-5 * max(1.0, float(want.abs().max()))
