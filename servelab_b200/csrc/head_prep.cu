@@ -199,6 +199,7 @@ struct HeadPrepKind {
     int units, items;        // vectors; warps' worth of vectors
     int norm, rot, unit;     // pieces that are normed, first piece that is rotated, pieces of the unit norm
     int skip;                // pieces that are not written
+    int drop;                // elements before `off` of a vector that are not read (a bias has them too)
 };
 struct HeadPrepPlan { HeadPrepKind kind[3]; int items; };
 
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
                     float v[8], b[8];
                     unpack8(raw[j][c], v);
                     if (bias != nullptr) {
-                        load8_weights(bias + unit[j] * kd.stride + piece * 8, b);
+                        load8_weights(bias + unit[j] * kd.stride + kd.drop + piece * 8, b);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) v[e] += b[e];
                     }
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
                 unpack8(raw[j][c], v[c]);
                 if (bias != nullptr && u < kd.units && piece < kd.pieces) {
                     float b[8];
-                    load8_weights(bias + u * kd.stride + piece * 8, b);
+                    load8_weights(bias + u * kd.stride + kd.drop + piece * 8, b);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[c][e] += b[e];
                 }
@@ -479,6 +480,7 @@ static bool head_prep_kind(HeadPrepKind* kd, int off, int D, int units, int norm
     kd->rot = (rot_off - drop) / 8;
     kd->unit = unit / 8;
     kd->skip = (skip - drop) / 8;
+    kd->drop = drop;
     return true;
 }
 

@@ -111,16 +111,19 @@ def test_heads_in_pieces_are_those_of_the_general_kernel(name, lens):
     assert got[0][0].abs().max() > 0 and got[0][1].abs().max() > 0 and got[0][2].abs().max() > 0
 
 
+@pytest.mark.parametrize("biased", [False, True])
 @pytest.mark.parametrize("lens", [[2, 30], [600]])
 @pytest.mark.parametrize("H,D,rot,R", [(16, 128, 64, 256), (5, 48, 32, 96), (8, 64, 64, 448)])
-def test_latent_rows_in_pieces_are_those_of_the_general_kernel(H, D, rot, R, lens):
-    """A latent attention's rows: one long key (normed latent, rotated rest), queries whose unrotated part is skipped."""
+def test_latent_rows_in_pieces_are_those_of_the_general_kernel(H, D, rot, R, lens, biased):
+    """A latent attention's rows: one long key (normed latent, rotated rest), queries whose unrotated part is skipped
+    (a bias has that part too)."""
     g = gen(H + len(lens))
     ctx, pages = step(lens)
     T, q_head = sum(lens), D + rot
     proj = torch.randn(T, H * q_head + R + rot, device=DEV, generator=g).bfloat16()
     kw = 1 + 0.1 * torch.randn(R, device=DEV, generator=g)
     freq = 10000.0 ** (-torch.arange(rot // 2, device=DEV) / (rot // 2)).float()
+    qb, kb = (torch.randn(n, device=DEV, generator=g) if biased else None for n in (H * q_head, R + rot))
     got = []
     for p in (proj, odd_view(proj)):
         q = torch.zeros(T, H * (R + rot), device=DEV, dtype=torch.bfloat16)
@@ -128,7 +131,7 @@ def test_latent_rows_in_pieces_are_those_of_the_general_kernel(H, D, rot, R, len
         K().head_prep(p, ctx, ctx.block_tables[0], 16, q_off=0, num_heads=H, q_dim=q_head, q_norm_w=None, q_norm_dims=0,
                       q_rot_off=D, q_out=q[:, R:], q_head_stride=R + rot, q_skip=D, k_off=H * q_head, num_kv_heads=1,
                       k_dim=R + rot, k_norm_w=kw, k_norm_dims=R, k_rot_off=R, v_off=-1, v_dim=0, freq=freq,
-                      rot_dims=rot, rot_mag=1.0, eps=1e-6, k_cache=kc, v_cache=None)
+                      rot_dims=rot, rot_mag=1.0, eps=1e-6, k_cache=kc, v_cache=None, q_bias=qb, k_bias=kb)
         got.append([q.float(), kc.float()])
     for a, b in zip(*got):
         assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 2.0 ** -16 * b.abs().max()).all() and a.abs().max() > 0
