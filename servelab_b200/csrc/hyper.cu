@@ -321,9 +321,13 @@ static int launch_gate_group_norm(const float* x, int ldx, const T* gate, int ld
     if (groups <= 0 || groups > 65535 || size <= 0 || gate == nullptr || gate_act < 1 || gate_act > 2 ||
         ldx < groups * size || ldg < groups * size || ldo < groups * size)
         return SLB_ERR_BAD_ARG;
-    const int rc = try_group_norm_warp<T, true>(x, ldx, 1, nullptr, w, eps, factor, gate, ldg, gate_act, out, ldo, T_,
-                                                groups, size, st);
-    if (rc != 1) return rc;
+    // (bfloat16 only: the two kernels add a part's squares in different orders, and a float32 row must not depend on
+    // how many rows the step has)
+    if constexpr (sizeof(T) == 2) {
+        const int rc = try_group_norm_warp<T, true>(x, ldx, 1, nullptr, w, eps, factor, gate, ldg, gate_act, out, ldo,
+                                                    T_, groups, size, st);
+        if (rc != 1) return rc;
+    }
     const uintptr_t half = (uintptr_t)gate | (uintptr_t)out;
     const bool vec = ((size | ldx | ldg | ldo) & 3) == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 &&
                      (half & (4 * sizeof(T) - 1)) == 0;

@@ -196,6 +196,33 @@ def test_gated_norms_against_64_bits(dtype, T, groups, size):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("size", [4, 100, 256, 512, 1024])
+@pytest.mark.parametrize("T", [255, 256, 257])
+def test_gate_before_norm_of_many_parts(dtype, size, T):
+    """Bfloat16 calls of 2,048 parts and more have a kernel of their own: 64-bit sums (1e-6 of a value and its
+    rounding), and the general form on rows at odd addresses (a rounding to bfloat16 apart).  A float32 row is the
+    same bits in a call of a few rows."""
+    groups, g = 8, gen(T + size)
+    n = groups * size
+    x, w = torch.randn(T, n, device=DEV, generator=g), torch.randn(n, device=DEV, generator=g)
+    gate = torch.randn(T, n, device=DEV, generator=g).to(dtype)
+
+    def run(x, gate):
+        out = torch.empty(x.shape[0], n, device=DEV, dtype=dtype)
+        K().gate_group_norm(x, gate, groups, out, eps=1e-6, weight=w, factor=1.5)
+        return out
+    out, z = run(x, gate), gate.double()
+    v = (x.double() * z * torch.sigmoid(z)).view(T, groups, size)
+    want = 1.5 * (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6)).view(T, n) * w.double()
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 4e-6
+    assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
+    odd = run(odd_view(x), odd_view(gate)).double()
+    assert ((out.double() - odd).abs() <= 2 * tol * want.abs() + 2e-6).all()
+    if dtype == torch.float32:
+        assert torch.equal(out[-7:], run(x[-7:], gate[-7:]))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n", [4, 1024, 1028, 2048, 3584, 4100])
 def test_sum_of_two_norms_against_64_bits(dtype, n):
     g = gen(n)
