@@ -359,13 +359,14 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
     }
     if (lane == 31) warp_total[warp] = make_int2(rows_upto, tiles_upto);
     __syncthreads();
-    int all_tiles = 0;
+    int all_tiles = 0, all_rows = 0;
     for (int i = 0; i < 32; ++i) {
         if (i < warp) {
             rows_upto += warp_total[i].x;
             tiles_upto += warp_total[i].y;
         }
         all_tiles += warp_total[i].y;
+        all_rows += warp_total[i].x;
     }
     if (tid < E) {
         plan[tid] = n;
@@ -377,6 +378,9 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
         }
     }
     for (int i = all_tiles + tid; i < num_tiles; i += 1024) tile_expert[i] = -1;
+    // (a pair whose id is no expert's is in no expert's rows; the list's end then names pair 0, so that whoever reads
+    // the whole list, as the gather of rows does, stays in range)
+    for (int i = all_rows + tid; i < P; i += 1024) sorted[i] = 0;
     __syncthreads();
     // (a product's result is written per pair, so the order within an expert changes no value)
     for (int p0 = tid; p0 < P; p0 += PLAN_RUN * 1024) {

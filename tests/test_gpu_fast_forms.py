@@ -266,6 +266,29 @@ def test_plan_of_the_experts_rows(P, E):
     assert (ids.cpu().long()[order].diff() >= 0).all()
 
 
+def test_pairs_without_an_expert_add_nothing_in_large_steps():
+    """The list of a plan has an entry for every pair, also where ids are no expert's: in range, and the step's sum is
+    that of the other pairs (the zero weights beside valid ids: the same products, the same bits)."""
+    from servelab_b200.ops import library as L
+    T, E, top, h, I, g = 300, 8, 4, 1024, 2048, gen(5)
+    x = torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    w = torch.rand(T, top, device=DEV, generator=g)
+    bad = torch.rand(T, top, device=DEV, generator=g) < 0.2
+    lib, P = L.core(), T * top
+    plan = torch.full((lib.slb_moe_plan_ints(P, E),), -7, dtype=torch.int32, device=DEV)
+    holes = torch.where(bad, -1, ids)
+    L.check(lib.slb_moe_plan(holes.data_ptr(), P, E, plan.data_ptr(), K()._stream()), "moe_plan")
+    order, rows = plan[-2 * P:-P].cpu(), int(plan[2 * E])
+    assert rows == P - int(bad.sum()) and (order[rows:] == 0).all()
+    assert torch.equal(order[:rows].sort().values, (~bad).view(-1).nonzero().view(-1).int().cpu())
+    for weighted in (False, True):
+        got = K().moe_experts(x, holes, w, wg, wd, None, weight_inputs=weighted)
+        want = K().moe_experts(x, ids, torch.where(bad, 0.0, w), wg, wd, None, weight_inputs=weighted)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("T,E,top,h,I", [(1, 8, 2, 64, 40), (3, 4, 4, 128, 72), (33, 8, 2, 200, 64), (64, 8, 2, 64, 136),
                                          (100, 5, 3, 72, 64), (300, 4, 2, 128, 64)])
 def test_experts_products_at_few_and_many_rows(T, E, top, h, I):
