@@ -1163,8 +1163,8 @@ def router_logits(x: torch.Tensor, w_f32: torch.Tensor) -> torch.Tensor:
     """float32 logits x . w^T of a float32 router matrix (activations float32 or bfloat16); a
     token's sums run in a fixed order."""
     M, Kd = x.shape
-    if (x.dtype == _BF16 and M >= router_vendor_min_tokens and Kd % 32 == 0 and x.stride(0) % 8 == 0
-            and w_f32.stride(0) % 4 == 0 and (x.data_ptr() | w_f32.data_ptr()) % 16 == 0):
+    if (x.dtype == _BF16 and M >= router_vendor_min_tokens and Kd % 32 == 0 and x.stride(1) == 1 and w_f32.stride(1) == 1
+            and x.stride(0) % 8 == 0 and w_f32.stride(0) % 4 == 0 and (x.data_ptr() | w_f32.data_ptr()) % 16 == 0):
         out = torch.empty((M, w_f32.shape[0]), dtype=_F32, device=x.device)
         L.check(L.core().slb_router_logits_tile_bf16(
             x.data_ptr(), x.stride(0), w_f32.data_ptr(), w_f32.stride(0), out.data_ptr(), out.stride(0), M,
@@ -1233,7 +1233,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         at = plan.numel() - 2 * P
         ends = plan[E + 1:2 * E + 1]                                   # cumulative row counts
         order = plan[at:at + P]                                        # pairs sorted by expert
-        if x.stride(0) % 8 or x.data_ptr() % 16:
+        if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
             x = x.clone(memory_format=torch.contiguous_format)
         xs = torch.empty((P, h), dtype=x.dtype, device=x.device)
         L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, h, xs.data_ptr(),

@@ -246,6 +246,23 @@ def test_router_logits_of_many_tokens(M, E, Kd):
     assert (K().router_logits(x, w).double() - want).norm() <= 1e-6 * want.norm()
 
 
+def test_large_steps_of_the_experts_take_rows_of_any_stride():
+    """Every second column of a wider matrix: the library's products took such rows, and so must the steps that read
+    them themselves."""
+    g = gen(3)
+    x, w = torch.randn(600, 512, device=DEV, generator=g).bfloat16(), torch.randn(16, 512, device=DEV, generator=g)
+    want = x[:, ::2].double() @ w[:, ::2].double().T
+    for a, b in ((x[:, ::2], w[:, ::2].contiguous()), (x[:, ::2].contiguous(), w[:, ::2])):
+        assert (K().router_logits(a, b).double() - want).norm() <= 1e-6 * want.norm()
+    T, E, top, h, I = 300, 8, 4, 1024, 2048
+    x = torch.randn(T, 2 * h, device=DEV, generator=g).bfloat16()
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    p = torch.rand(T, top, device=DEV, generator=g)
+    wide, packed = (K().moe_experts(v, ids, p, wg, wd, None) for v in (x[:, ::2], x[:, ::2].contiguous()))
+    assert torch.equal(wide, packed)
+
+
 @pytest.mark.parametrize("P,E", [(1, 1), (3, 7), (256, 32), (8191, 32), (64, 1024), (20001, 60)])
 def test_plan_of_the_experts_rows(P, E):
     from servelab_b200.ops import library as L
