@@ -38,6 +38,9 @@
 #define GC_LA 36                             // row stride of A
 #define GC_MAX_D 256
 
+// 0, or 1: the wait for a chunk's record gave up and the request's rows of that launch are not written
+SLB_DEFINE_STATUS_WORD(gated_chunk_status_word, slb_decay_gated_chunk_status)
+
 struct GatedChunkArgs {
     DecayAttnArgs a;
     const int* tile_seq; const int* tile_row0; int num_tiles;
@@ -274,7 +277,13 @@ __global__ void __launch_bounds__(512, 1) gated_chunk_walk_kernel(const GatedChu
     const bool wide = (Dv & 3) == 0 && (a.ldo & 3) == 0 && ((uintptr_t)a.out & 15) == 0;
     for (int k = 0; k < count; ++k) {
         const bool there = slb_mma::mbar_wait(&bars[k & 1], (k >> 1) & 1);
-        if (!__syncthreads_and(there)) return;       // (the copy never came: nothing of ours is in flight but it)
+        if (!__syncthreads_and(there)) {             // the copy did not come in time: say so, and give it its limit once
+            if (tid == 0) {                          // more before the block's shared memory goes to another
+                atomicCAS(&gated_chunk_status_word, 0, 1);
+                slb_mma::mbar_wait(&bars[k & 1], (k >> 1) & 1);
+            }
+            return;
+        }
         const bool more = k + 1 < count;
         if (more && tid == 256) fetch(k + 1);
         if (more) load_v(k + 1);

@@ -30,6 +30,9 @@
 #define DC_EV 16
 #define DC_LM 36                             // row stride of Y, P, Q and of the [value][token] operands
 
+// 0, or 1: the wait for a chunk's record gave up and the request's rows of that launch are not written
+SLB_DEFINE_STATUS_WORD(delta_chunk_status_word, slb_delta_chunk_status)
+
 struct DeltaChunkArgs {
     DeltaRuleArgs a;
     const int* tile_seq; const int* tile_row0; int num_tiles;
@@ -307,7 +310,13 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const DeltaChunkA
     const int m0 = (warp >> 1) * 16, n0 = (warp & 1) * 8;
     for (int k = 0; k < count; ++k) {
         const bool there = slb_mma::mbar_wait(&bars[k % STAGES], (k / STAGES) & 1);
-        if (!__syncthreads_and(there)) return;       // (the copy never came: nothing of ours is in flight but it)
+        if (!__syncthreads_and(there)) {             // the copy did not come in time: say so, and give it its limit once
+            if (tid == 0) {                          // more before the block's shared memory goes to another
+                atomicCAS(&delta_chunk_status_word, 0, 1);
+                slb_mma::mbar_wait(&bars[k % STAGES], (k / STAGES) & 1);
+            }
+            return;
+        }
         const bool more = k + 1 < count;
         if (STAGES == 2 && more && tid == 0) fetch(k + 1);
         if (more) load_v(k + 1);

@@ -1563,6 +1563,11 @@ def decay_attention(proj: torch.Tensor, ctx, state: torch.Tensor, decay: Optiona
     L.check(fn(_ct.byref(a), ctx.num_seqs, _stream()), "decay_attention")
 
 
+def decay_gated_chunk_status(reset: bool = False) -> int:
+    """0 unless a bounded wait of the walk over a learned decay's chunks gave up."""
+    return L.core().slb_decay_gated_chunk_status(1 if reset else 0)
+
+
 def attention_kv_maps(ctx, q, k_cache, v_cache, out, block_table, num_heads: int, num_kv_heads: int,
                       maps: int, k_dim: int, v_dim: int, page_size: int, scale: float, window: int = 0) -> None:
     """The plain kernel with ``maps`` attention maps a head: q [T, H, maps, k_dim], cached key rows
@@ -1787,6 +1792,11 @@ def delta_rule(ctx, proj: torch.Tensor, state: torch.Tensor, out: torch.Tensor, 
         L.check(getattr(lib, "slb_delta_rule_" + suffix)(_ct.byref(a), ctx.num_seqs, _stream()), "delta_rule")
     group_norm_gate(o, num_heads, value_dim, out, eps=norm_eps, weight=norm_w,
                     gate=proj[:, g_off:g_off + num_heads * value_dim], gate_activation="sigmoid")
+
+
+def delta_chunk_status(reset: bool = False) -> int:
+    """0 unless a bounded wait of the scan over a delta rule's chunks gave up."""
+    return L.core().slb_delta_chunk_status(1 if reset else 0)
 
 
 # --------------------------------------------------- gated linear recurrence (a number a channel)

@@ -97,6 +97,7 @@ _CORE_SIGNATURES = {
     "slb_delta_chunk_work_floats": [I],
     "slb_delta_chunk_f32": [P, I, P],
     "slb_delta_chunk_bf16": [P, I, P],
+    "slb_delta_chunk_status": [I],
     "slb_gated_recurrence_f32": [P, I, I, P],
     "slb_gated_recurrence_bf16": [P, I, I, P],
     "slb_moe_tile_rows": [I, I],
@@ -135,6 +136,7 @@ _CORE_SIGNATURES = {
     "slb_decay_gated_chunk_max_dim": [],
     "slb_decay_gated_chunk_tokens": [],
     "slb_decay_gated_chunk_work_floats": [I],
+    "slb_decay_gated_chunk_status": [I],
     "slb_decay_gated_chunk_f32": [P, I, P],
     "slb_decay_gated_chunk_bf16": [P, I, P],
     "slb_router_logits_f32": [P, I, P, I, P, I, I, I, I, P],

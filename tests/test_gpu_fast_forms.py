@@ -380,3 +380,23 @@ def test_walk_over_the_chunks_against_the_recurrence(D, Hh, Dv):
     out = case._run_gated_chunked(kernels, proj.cuda(), z.cuda(), bias.cuda(), state, Hh, D, Dv,
                                   [[(0, 0, 31), (1, 31, 32), (2, 63, 70)]], 4.0, D ** -0.5)
     assert (out.double().cpu() - want).abs().max() < 3e-5 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("D,Dv", [(64, 64), (128, 40), (192, 64)])
+def test_scans_over_chunks_report_waits_that_gave_up(D, Dv):
+    """Two and one record a block (key sizes up to 128 and above), requests of one and of several chunks: no wait
+    gives up, every row is written."""
+    lens, H, g = [32, 70, 129], 2, gen(D)
+    ctx, _ = step(lens)
+    T = sum(lens)
+    proj = torch.randn(T, H * (3 * D + 2 * Dv), device=DEV, generator=g).bfloat16()
+    z, bias, norm = (torch.randn(*s, device=DEV, generator=g) for s in ((T, H * D), (H * D,), (H * Dv,)))
+    out = torch.full((T, H * Dv), float("nan"), device=DEV, dtype=torch.bfloat16)
+    K().delta_rule(ctx, proj, torch.zeros(3, H * D * Dv, device=DEV), out, r_off=0, k_off=H * D, v_off=2 * H * D,
+                   a_off=H * (2 * D + Dv), g_off=H * (3 * D + Dv), num_heads=H, head_dim=D, value_dim=Dv, a_bias=bias,
+                   gate_z=z, decay_coef=0.6, unit_eps=1e-6, norm_w=norm, norm_eps=1e-5)
+    rows = torch.full((T, H * Dv), float("nan"), device=DEV)
+    K().decay_attention(proj, ctx, torch.zeros(3, H * D * Dv, device=DEV), None, rows, q_off=0, k_off=H * D, v_off=2 * H * D,
+                        num_heads=H, head_dim=D, value_dim=Dv, gate_z=z, gate_tau=4.0)
+    assert out.isfinite().all() and rows.isfinite().all()
+    assert K().delta_chunk_status() == 0 and K().decay_gated_chunk_status() == 0
