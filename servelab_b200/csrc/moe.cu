@@ -9,7 +9,7 @@
 //   slb_moe_route_scored  the same with sigmoid scores, an offset per expert that enters the choice
 //                      only, groups that score as the sum of their best few, and a constant in the
 //                      denominator of the renormalised weights, each an argument.
-//   slb_moe_plan       (token, choice) pairs sorted by expert: counts, offsets, the list, and the
+//   slb_moe_plan(_simt)  (token, choice) pairs sorted by expert: counts, offsets, the list, and the
 //                      row tiles of the products (tile -> expert, first row), of a length that
 //                      depends only on the number of pairs and experts (a fixed grid).
 //   slb_moe_gate_up    act[pair] = silu(W_gate[e] x) * (W_up[e] x) for the pair's expert e, or another gated
@@ -31,13 +31,13 @@
 #define MOE_BN 64
 #define MOE_BK 16
 
-// Rows of a product's tile: few where an expert gets few, so that the tensor-core form's stages are small and
-// all its blocks are resident at once (the last wave of a second round is nearly empty).
+// Rows of a tile of the tensor-core product: few where an expert gets few, so that its stages are small and
+// all its blocks are resident at once (the last wave of a second round is nearly empty).  The product on CUDA
+// cores has tiles of MOE_BM rows whatever they hold: a smaller one would cost it as much.
 static int moe_tile_rows(int P, int E) { return P <= 8 * E ? 16 : P <= 40 * E ? 32 : MOE_BM; }
-static int moe_num_tiles(int P, int E) {
-    const int rows = moe_tile_rows(P, E);
-    return (P + rows - 1) / rows + E;
-}
+static int moe_num_tiles(int P, int E, int rows) { return (P + rows - 1) / rows + E; }
+static int moe_num_tiles(int P, int E) { return moe_num_tiles(P, E, moe_tile_rows(P, E)); }
+static int moe_plan_ints(int P, int E, int rows) { return 3 * E + 1 + 2 * moe_num_tiles(P, E, rows) + 2 * P; }
 
 // ------------------------------------------------------------------- route
 __device__ __forceinline__ void warp_argmax(float& v, int& i) {
@@ -430,8 +430,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
 template <typename T, typename TC, int MODE>
 __global__ void __launch_bounds__(256) moe_product_kernel(
     const T* __restrict__ A, int lda, const T* __restrict__ W, long long w_expert_stride, int ldw,
-    TC* __restrict__ C, int ldc, const int* __restrict__ plan, int E, int num_tiles, int tile_rows, int P, int top,
-    int N, int K, int act, float limit, float alpha, const float* __restrict__ in_weights) {
+    TC* __restrict__ C, int ldc, const int* __restrict__ plan, int E, int num_tiles, int P, int top, int N, int K, int act, float limit, float alpha, const float* __restrict__ in_weights) {
     __shared__ __align__(16) float As[MOE_BK][MOE_BM + 4];
     __shared__ __align__(16) float Ws[MOE_BK][MOE_BN + 4];
     __shared__ __align__(16) float Us[MODE == 0 ? MOE_BK : 1][MOE_BN + 4];
@@ -445,7 +444,7 @@ __global__ void __launch_bounds__(256) moe_product_kernel(
     const int e = tile_expert[blockIdx.y];
     if (e < 0) return;
     const int r0 = tile_row0[blockIdx.y];
-    const int nrows = min(tile_rows, counts[e] - r0);
+    const int nrows = min(MOE_BM, counts[e] - r0);
     const int tid = threadIdx.x;
     if (tid < MOE_BM) rows[tid] = tid < nrows ? sorted[offsets[e] + r0 + tid] : -1;
     __syncthreads();
@@ -745,10 +744,10 @@ static int launch_moe_gate_up(const T* x, int ldx, const T* w_gu, int ldw, T* ou
                               float alpha, const float* in_weights, cudaStream_t st) {
     if (P <= 0) return 0;
     if (E <= 0 || top <= 0 || I <= 0 || K <= 0 || act < 0 || act > 2 || (act == 2 && !(limit > 0.f))) return SLB_ERR_BAD_ARG;
-    const int nt = moe_num_tiles(P, E);
+    const int nt = moe_num_tiles(P, E, MOE_BM);
     if (nt > 65535) return SLB_ERR_TOO_LARGE;
     return slb_launch(moe_product_kernel<T, T, 0>, dim3((I + MOE_BN - 1) / MOE_BN, nt), dim3(256), 0, st, x,
-                      ldx, w_gu, (long long)2 * I * ldw, ldw, out, lda, plan, E, nt, moe_tile_rows(P, E), P, top, I, K, act, limit, alpha, in_weights);
+                      ldx, w_gu, (long long)2 * I * ldw, ldw, out, lda, plan, E, nt, P, top, I, K, act, limit, alpha, in_weights);
 }
 
 template <typename T>
@@ -756,10 +755,10 @@ static int launch_moe_down(const T* act, int lda, const T* w_down, int ldw, floa
                            const int* plan, int E, int P, int top, int N, int I, cudaStream_t st) {
     if (P <= 0) return 0;
     if (E <= 0 || top <= 0 || I <= 0 || N <= 0) return SLB_ERR_BAD_ARG;
-    const int nt = moe_num_tiles(P, E);
+    const int nt = moe_num_tiles(P, E, MOE_BM);
     if (nt > 65535) return SLB_ERR_TOO_LARGE;
     return slb_launch(moe_product_kernel<T, float, 1>, dim3((N + MOE_BN - 1) / MOE_BN, nt), dim3(256), 0, st,
-                      act, lda, w_down, (long long)N * ldw, ldw, y, ldy, plan, E, nt, moe_tile_rows(P, E), P, top, N, I, 0, 0.f, 0.f, (const float*)nullptr);
+                      act, lda, w_down, (long long)N * ldw, ldw, y, ldy, plan, E, nt, P, top, N, I, 0, 0.f, 0.f, (const float*)nullptr);
 }
 
 template <int MODE>
@@ -861,11 +860,20 @@ int slb_router_logits_tile_bf16(const bf16* x, int ldx, const float* w, int ldw,
     return slb_launch(router_logits_tile_kernel, dim3((M + RL_TOK - 1) / RL_TOK, (E + RL_EXP - 1) / RL_EXP), dim3(256),
                       smem, st, x, ldx, w, ldw, logits, ldl, M, E, K);
 }
-int slb_moe_plan_ints(int P, int E) { return 3 * E + 1 + 2 * moe_num_tiles(P, E) + 2 * P; }
-int slb_moe_plan(const int* ids, int P, int E, int* plan, cudaStream_t st) {
+static int launch_moe_plan(const int* ids, int P, int E, int rows, int* plan, cudaStream_t st) {
     if (P <= 0) return 0;
     if (E <= 0 || E > MOE_MAX_EXPERTS) return SLB_ERR_BAD_ARG;
-    return slb_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, st, ids, P, E, moe_num_tiles(P, E), moe_tile_rows(P, E), plan);
+    return slb_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, st, ids, P, E, moe_num_tiles(P, E, rows), rows, plan);
+}
+// the plan of the products on tensor cores and of the library's ...
+int slb_moe_plan_ints(int P, int E) { return moe_plan_ints(P, E, moe_tile_rows(P, E)); }
+int slb_moe_plan(const int* ids, int P, int E, int* plan, cudaStream_t st) {
+    return launch_moe_plan(ids, P, E, moe_tile_rows(P, E), plan, st);
+}
+// ... and of those on CUDA cores
+int slb_moe_plan_simt_ints(int P, int E) { return moe_plan_ints(P, E, MOE_BM); }
+int slb_moe_plan_simt(const int* ids, int P, int E, int* plan, cudaStream_t st) {
+    return launch_moe_plan(ids, P, E, MOE_BM, plan, st);
 }
 int slb_moe_gate_up_f32(const float* x, int ldx, const float* w_gu, int ldw, float* out, int lda,
                         const int* plan, int E, int P, int top, int I, int K, int act, float limit, float alpha,

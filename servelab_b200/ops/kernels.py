@@ -1221,11 +1221,16 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     n_out = w_down.shape[1]
     P = T * top
     lib = L.core()
-    plan = torch.empty(lib.slb_moe_plan_ints(P, E), dtype=torch.int32, device=x.device)
-    L.check(lib.slb_moe_plan(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
-    if (x.dtype == _BF16 and moe_vendor_grouped and P >= moe_vendor_min_pairs
-            and h * inter >= moe_vendor_min_expert_elements and h % 8 == 0
-            and inter % 8 == 0 and n_out % 8 == 0 and hasattr(torch, "_grouped_mm")):
+    vendor = (x.dtype == _BF16 and moe_vendor_grouped and P >= moe_vendor_min_pairs
+              and h * inter >= moe_vendor_min_expert_elements and h % 8 == 0
+              and inter % 8 == 0 and n_out % 8 == 0 and hasattr(torch, "_grouped_mm"))
+    # bfloat16 with rows of whole 16-byte chunks: the tensor-core products; else CUDA cores
+    mma = (x.dtype == _BF16 and moe_tensor_cores and h % 8 == 0 and inter % 8 == 0 and n_out % 2 == 0
+           and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+    form = "" if vendor or mma else "_simt"                # (the tiles' rows differ)
+    plan = torch.empty(getattr(lib, f"slb_moe_plan{form}_ints")(P, E), dtype=torch.int32, device=x.device)
+    L.check(getattr(lib, "slb_moe_plan" + form)(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
+    if vendor:
         # Large steps: the vendor's grouped product over the rows sorted by expert (the plan's list
         # and offsets stay on the device), as the dense products of large steps go to the vendor's
         # GEMM; the weighted sum reads a token's rows where the product left them.
@@ -1256,9 +1261,6 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         return out
     act = torch.empty((P, inter), dtype=x.dtype, device=x.device)
     sfx = _suffix(x.dtype)
-    # bfloat16 with rows of whole 16-byte chunks: the tensor-core products; else CUDA cores
-    mma = (x.dtype == _BF16 and moe_tensor_cores and h % 8 == 0 and inter % 8 == 0 and n_out % 2 == 0
-           and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
     up_sfx = "mma_bf16" if mma else sfx
     L.check(getattr(lib, "slb_moe_gate_up_" + up_sfx)(
         x.data_ptr(), x.stride(0), w_gate_up.data_ptr(), w_gate_up.stride(1), act.data_ptr(), act.stride(0),

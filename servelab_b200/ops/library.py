@@ -143,6 +143,8 @@ _CORE_SIGNATURES = {
     "slb_router_logits_bf16": [P, I, P, I, P, I, I, I, I, P],
     "slb_moe_plan_ints": [I, I],
     "slb_moe_plan": [P, I, I, P, P],
+    "slb_moe_plan_simt_ints": [I, I],
+    "slb_moe_plan_simt": [P, I, I, P, P],
     "slb_moe_gate_up_f32": [P, I, P, I, P, I, P, I, I, I, I, I, I, F, F, P, P],
     "slb_moe_gate_up_bf16": [P, I, P, I, P, I, P, I, I, I, I, I, I, F, F, P, P],
     "slb_moe_down_f32": [P, I, P, I, P, I, P, I, I, I, I, I, P],

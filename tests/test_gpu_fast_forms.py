@@ -283,6 +283,40 @@ def test_plan_of_the_experts_rows(P, E):
     assert (ids.cpu().long()[order].diff() >= 0).all()
 
 
+@pytest.mark.parametrize("P,E", [(1, 1), (256, 32), (1000, 32), (1280, 32), (5000, 32)])
+def test_plan_of_the_products_on_cuda_cores_has_full_tiles(P, E):
+    """One tile an expert up to 64 rows, however few rows the experts get: a smaller tile would cost them as much."""
+    from servelab_b200.ops import library as L
+    ids = torch.randint(0, E, (P,), device=DEV, dtype=torch.int32, generator=gen(P))
+    ids[:P // 3] = 0                                      # a crowded expert
+    lib = L.core()
+    plan = torch.full((lib.slb_moe_plan_simt_ints(P, E),), -7, dtype=torch.int32, device=DEV)
+    L.check(lib.slb_moe_plan_simt(ids.data_ptr(), P, E, plan.data_ptr(), K()._stream()), "moe_plan")
+    p, tiles, at = plan.cpu().tolist(), -(-P // 64) + E, 3 * E + 1
+    counts = torch.bincount(ids.cpu().long(), minlength=E).tolist()
+    want = [(e, r) for e in range(E) for r in range(0, counts[e], 64)]
+    got = list(zip(p[at:at + tiles], p[at + tiles:at + 2 * tiles]))
+    assert len(p) == at + 2 * tiles + 2 * P
+    assert got[:len(want)] == want and all(e == -1 for e, _ in got[len(want):])
+
+
+@pytest.mark.parametrize("T,E,top,h,I", [(9, 8, 2, 36, 20), (100, 8, 3, 60, 28), (300, 5, 2, 44, 36)])
+def test_experts_products_on_cuda_cores(T, E, top, h, I):
+    """Float32, few and many rows an expert, one expert with more rows than a tile: sums of at most 60 products in
+    order against 64 bits, 2e-6 of the norm."""
+    g = gen(T + E)
+    x = torch.randn(T, h, device=DEV, generator=g)
+    wg, wd = (torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5 for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    ids[:, 0] = 1
+    ids[:, 1:] = torch.where(ids[:, 1:] == 1, 0, ids[:, 1:])
+    w = torch.rand(T, top, device=DEV, generator=g)
+    gu = torch.einsum("tkih,th->tki", wg.double()[ids.long()], x.double())
+    act = gu[..., :I] * torch.sigmoid(gu[..., :I]) * gu[..., I:]
+    want = torch.einsum("tk,tkhi,tki->th", w.double(), wd.double()[ids.long()], act)
+    assert (K().moe_experts(x, ids, w, wg, wd, None).double() - want).norm() <= 2e-6 * want.norm()
+
+
 def test_pairs_without_an_expert_add_nothing_in_large_steps():
     """The list of a plan has an entry for every pair, also where ids are no expert's: in range, and the step's sum is
     that of the other pairs (the zero weights beside valid ids: the same products, the same bits)."""
