@@ -34,7 +34,12 @@
 // Rows of a tile of the tensor-core product: few where an expert gets few, so that its stages are small and
 // all its blocks are resident at once (the last wave of a second round is nearly empty).  The product on CUDA
 // cores has tiles of MOE_BM rows whatever they hold: a smaller one would cost it as much.
-static int moe_tile_rows(int P, int E) { return P <= 8 * E ? 16 : P <= 40 * E ? 32 : MOE_BM; }
+// The line at 32 rows an expert, us of a step with tiles of 32 / 64 rows at 28, 36, 44 rows each: 128 experts of
+// 2,048 x 768 313 / 293, 398 / 323, 460 / 353; 32 of 2,048 x 1,408 149 / 185, 206 / 189, 230 / 195; 64 of
+// 1,024 x 512 79 / 71, 94 / 77, 106 / 83.  With few experts there are too few tiles to fill the device and the
+// smaller ones stay ahead for longer, at 36, 50, 64: 16 of 1,024 x 512 38 / 47, 40 / 49, 44 / 54; 8 of 2,048 x 1,408
+// 76 / 86, 80 / 98, 82 / 101.
+static int moe_tile_rows(int P, int E) { return P <= 8 * E ? 16 : P <= (E <= 16 ? 64 : 32) * E ? 32 : MOE_BM; }
 static int moe_num_tiles(int P, int E, int rows) { return (P + rows - 1) / rows + E; }
 static int moe_num_tiles(int P, int E) { return moe_num_tiles(P, E, moe_tile_rows(P, E)); }
 static int moe_plan_ints(int P, int E, int rows) { return 3 * E + 1 + 2 * moe_num_tiles(P, E, rows) + 2 * P; }

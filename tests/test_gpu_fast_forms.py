@@ -317,6 +317,13 @@ def test_experts_products_on_cuda_cores(T, E, top, h, I):
     assert (K().moe_experts(x, ids, w, wg, wd, None).double() - want).norm() <= 2e-6 * want.norm()
 
 
+def test_rows_of_a_tile_follow_the_rows_an_expert_gets():
+    from servelab_b200.ops import library as L
+    rows = L.core().slb_moe_tile_rows
+    assert [rows(32 * n, 32) for n in (1, 8, 9, 32, 33, 200)] == [16, 16, 32, 32, 64, 64]
+    assert [rows(16 * n, 16) for n in (8, 9, 64, 65)] == [16, 32, 32, 64]
+
+
 def test_pairs_without_an_expert_add_nothing_in_large_steps():
     """The list of a plan has an entry for every pair, also where ids are no expert's: in range, and the step's sum is
     that of the other pairs (the zero weights beside valid ids: the same products, the same bits)."""
@@ -343,7 +350,7 @@ def test_pairs_without_an_expert_add_nothing_in_large_steps():
 @pytest.mark.parametrize("T,E,top,h,I", [(1, 8, 2, 64, 40), (3, 4, 4, 128, 72), (33, 8, 2, 200, 64), (64, 8, 2, 64, 136),
                                          (100, 5, 3, 72, 64), (300, 4, 2, 128, 64)])
 def test_experts_products_at_few_and_many_rows(T, E, top, h, I):
-    """Tiles of 16, 32 and 64 rows (up to 8, 40 and more rows an expert) against 64 bits: two roundings to bfloat16 of
+    """Tiles of 16, 32 and 64 rows (up to 8, 64 and more rows of a few experts) against 64 bits: two roundings to bfloat16 of
     the first product, one of the activation, one of the result."""
     g = gen(T)
     x = torch.randn(T, h, device=DEV, generator=g).bfloat16()
