@@ -150,12 +150,13 @@ def test_sigmoid_gate_in_pieces(T, N, group):
 # ------------------------------------------------------------ convolution, norms with a gate
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("taps", [2, 3, 4])
-@pytest.mark.parametrize("lens", [[256], [1, 2, 300, 7], [129, 128, 5]])
-def test_convolution_of_runs_is_that_of_single_tokens(dtype, taps, lens):
-    """Portions from 256 tokens on take runs of tokens a thread; rows at an odd address the kernel that takes them one
-    by one.  The same products in the same order: the same bits, in the rows and in the records."""
+@pytest.mark.parametrize("C,lens", [(264, [256]), (264, [1, 2, 300, 7]), (264, [129, 128, 5]), (1032, [3053]),
+                                    (1032, [1, 2, 3100, 7]), (520, [6100, 9, 130, 5]), (1032, [129] * 24)])
+def test_convolution_of_runs_is_that_of_single_tokens(dtype, taps, C, lens):
+    """Long portions of large steps (3 Mi elements, 128 tokens a request) take runs of tokens a thread; other steps, and
+    rows at an odd address, the kernel that takes them one by one.  The same products in the same
+    order: the same bits, in the rows and in the records."""
     g = gen(taps + len(lens))
-    C = 264
     ctx, _ = step(lens)
     T = sum(lens)
     proj = torch.randn(T, C + 8, device=DEV, generator=g).to(dtype)
