@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(HP_WARPS * 32) head_prep_kernel(const HeadPrep
 // kernel against this one, us: 2,048 tokens of 16 + 4 + 4 heads of 128, half rotated, unit norms 23.7 ->
 // 14.6; 2,912 tokens of 16 + 4 heads of 128 and 4 of 64, norms over the rows, biases 28.0 -> 18.5; 2,082
 // tokens of a latent attention (16 queries of 192, of which 64 are read, a key of 320) 21.0 -> 12.7;
-// 64 single tokens 4.4 -> 4.6 (row norms) and 3.8 -> 3.7.
+// 64 single tokens of 16 + 4 + 4 heads of 128 3.8 -> 3.4.
 #define HPV_ITEMS 4          // vectors (of a lane) that are loaded together
 
 struct HeadPrepKind {
@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
     }
 }
 
+static int max_of(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 static bool pieces(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 // One kind of vector for the kernel in pieces; false: it does not take these sizes.
@@ -487,7 +488,14 @@ static bool head_prep_kind(HeadPrepKind* kd, int off, int D, int units, int norm
 // Whether the kernel in pieces takes these arguments (bfloat16), and how it works on them: sizes and
 // offsets in multiples of 8 elements, rows and weights on 16-byte boundaries, vectors of at most 512
 // (256 where halves turn with one another), a token's vectors in one block's registers where all
-// heads of a row are normed together.
+// heads of a row are normed together.  Steps too small for what it packs stay with the general kernel,
+// which spreads them over more warps.  General kernel / this one, us at 1 / 32 / 128 tokens:
+//   short vectors, several to a warp: 4 + 2 + 2 heads of 64, normed and rotated, 3.2, 3.3, 3.4 / 3.5, 3.6, 3.6; of 32
+//   +15, +12, +12 %; 14 + 2 + 2 of 64 +13, +12, +3 %; 3 + 3 + 3 of 96 and 64 +3, 0, 0 %.  From some 3,200 vectors
+//   on this one is ahead (4 + 2 + 2 of 64, 511 tokens: 5.3 / 4.0).
+//   a long normed row in one block, at 1 / 32 / 64 tokens: 40 + 8 + 8 heads of 128 5.0, 5.4, 9.4 / 5.9, 5.9, 6.0;
+//   16 + 4 + 4 4.1, 4.3, 4.6 / 4.4, 4.5, 4.5; 32 + 8 + 8 of 64 +12, +4, -6 %.  Rows of up to 8 warps' worth of
+//   vectors: -5 % and less.
 static bool head_prep_plan(const HeadPrepArgs& a, int num_tokens, HeadPrepPlan* p, int* warps) {
     const bool has_v = a.v_off >= 0 && a.G > 0;
     if (((a.ld | a.ldq | a.q_head_stride) & 7) || !pieces(a.proj) || !pieces(a.q_out) || !pieces(a.k_cache) ||
@@ -505,6 +513,9 @@ static bool head_prep_plan(const HeadPrepArgs& a, int num_tokens, HeadPrepPlan* 
         !head_prep_kind(&p->kind[2], a.v_off, a.Dv, has_v ? a.G : 0, 0, 0, 0, 0, 0, 0))
         return false;
     p->items = p->kind[0].items + p->kind[1].items + p->kind[2].items;
+    const int units = a.H + a.G + (has_v ? a.G : 0), longest = max_of(a.Dq, a.Dk, has_v ? a.Dv : 0);
+    if (a.row_norm ? num_tokens <= 32 && p->items > 8 : longest <= 96 && (long long)num_tokens * units <= 3200)
+        return false;
     *warps = a.row_norm && (p->items > 4 * HPV_ITEMS || num_tokens < 512) ? 8 : 4;
     return !a.row_norm || p->items <= *warps * HPV_ITEMS;
 }
@@ -554,7 +565,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_vec_kernel(const bf16* __res
 template <typename T>
 static int launch_head_prep(const HeadPrepArgs& a, int num_tokens, cudaStream_t st) {
     if (num_tokens <= 0) return 0;
-    const int maxd = a.Dq > a.Dk ? (a.Dq > a.Dv ? a.Dq : a.Dv) : (a.Dk > a.Dv ? a.Dk : a.Dv);
+    const int maxd = max_of(a.Dq, a.Dk, a.Dv);
     if (a.H < 0 || a.G < 0 || a.Dq < 0 || a.Dk < 0 || maxd <= 0 || (a.rot_dims & 1)) return SLB_ERR_BAD_ARG;
     if (maxd > HP_MAX_D) return SLB_ERR_TOO_LARGE;
     if (a.rot_dims > 0 && (a.freq == nullptr || (a.H > 0 && a.q_rot_off + a.rot_dims > a.Dq) ||
