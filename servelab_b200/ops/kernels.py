@@ -1153,24 +1153,34 @@ def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
                M, N, Kd, B, a.stride(1), w.stride(0), out.stride(1), _stream()), "gemm_simt_batched")
 
 
-# Steps of this many tokens: this package's kernel for many tokens, the vendor's product for widths it does not
-# take.  Measured us (kernel for few tokens / vendor, with the copy to float32 / this) at 32 experts of 2,048: 512
+# bfloat16 steps of this many tokens: this package's kernel for many tokens or the vendor's float32 product.
+# Measured us (kernel for few tokens / vendor, with the copy to float32 / kernel for many) at 32 experts of 2,048: 512
 # tokens 13.8 / 21.6 / 13.3, 2,048 tokens 44 / 49 / 13.6; 16 of 1,024: 5.9 / 16.4 / 7.4 and 16.3 / 25.1 / 7.5.
-router_vendor_min_tokens = 512
+router_many_tokens = 512
+
+
+def router_takes_tiles(tokens: int, experts: int) -> bool:
+    """Whether the kernel for many tokens (a block 16 tokens and 32 experts, one on an SM) is the faster one.  Its
+    time over the vendor's at widths of 1,024 to 7,168, by blocks: up to 384 0.3 to 0.9, 512 0.3 to 0.8 with up to 64
+    experts (which read a token's row twice at most) and 0.98 to 1.09 with more, 768 1.0 to 1.2, 1,024 0.6 to 1.0
+    with 64 experts and 1.2 to 1.6 with more (2,048 tokens of 256 experts: 64 us against 86)."""
+    blocks = -(-tokens // 16) * -(-experts // 32)
+    return blocks <= 3 * _num_sms() or (experts <= 64 and blocks <= 1024)
 
 
 def router_logits(x: torch.Tensor, w_f32: torch.Tensor) -> torch.Tensor:
     """float32 logits x . w^T of a float32 router matrix (activations float32 or bfloat16); a
     token's sums run in a fixed order."""
     M, Kd = x.shape
-    if (x.dtype == _BF16 and M >= router_vendor_min_tokens and Kd % 32 == 0 and x.stride(1) == 1 and w_f32.stride(1) == 1
-            and x.stride(0) % 8 == 0 and w_f32.stride(0) % 4 == 0 and (x.data_ptr() | w_f32.data_ptr()) % 16 == 0):
+    if (x.dtype == _BF16 and M >= router_many_tokens and router_takes_tiles(M, w_f32.shape[0]) and Kd % 32 == 0
+            and x.stride(1) == 1 and w_f32.stride(1) == 1 and x.stride(0) % 8 == 0 and w_f32.stride(0) % 4 == 0
+            and (x.data_ptr() | w_f32.data_ptr()) % 16 == 0):
         out = torch.empty((M, w_f32.shape[0]), dtype=_F32, device=x.device)
         L.check(L.core().slb_router_logits_tile_bf16(
             x.data_ptr(), x.stride(0), w_f32.data_ptr(), w_f32.stride(0), out.data_ptr(), out.stride(0), M,
             w_f32.shape[0], Kd, _stream()), "router_logits")
         return out
-    if x.dtype == _BF16 and M >= router_vendor_min_tokens:
+    if x.dtype == _BF16 and M >= router_many_tokens:
         # a large step in the bfloat16 path: the vendor's float32 product (no reduced-precision
         # mode: torch's default for float32 products) on the widened rows
         from .profile import mark

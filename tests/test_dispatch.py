@@ -86,3 +86,11 @@ def test_switches_change_the_decision(monkeypatch):
     assert L.which_kernel(*_ops(17, h, q)) == "vendor"
     monkeypatch.setattr(L, "tc_max_tokens", 4)
     assert L.which_kernel(*_ops(8, h, q)) == "vendor"
+
+
+def test_router_of_many_experts_and_tokens_stays_with_the_library():
+    """The points at which both sides were measured; the few tokens' kernel is chosen before this rule."""
+    for tokens, experts in ((512, 8), (512, 384), (768, 256), (1024, 192), (2048, 32), (2048, 96), (8192, 32), (8192, 64)):
+        assert K.router_takes_tiles(tokens, experts)
+    for tokens, experts in ((768, 384), (1024, 256), (2048, 128), (2048, 256), (4096, 96), (4096, 192), (8192, 128)):
+        assert not K.router_takes_tiles(tokens, experts)
