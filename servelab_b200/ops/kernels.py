@@ -529,7 +529,7 @@ def decode_attention_split(ctx, q, k_cache, v_cache, out, block_table, num_heads
 decode_ws_stages = 3           # depth of the kernel's shared-memory ring (2..4)
 decode_ws_force_splits = 0     # measurements: launch this many splits instead of the choice below
 # The kernel picks each request's number of splits itself, from the request's own length: one
-# while it has at most `decode_ws_unsplit_tiles` 64-key tiles, and never more splits than were
+# while it has at most `decode_ws_unsplit` 64-key tiles, and never more splits than were
 # launched.  In the cluster form (the default) a split has two tiles at least, and a request
 # takes more splits than one cluster holds only when that saves a block four tiles or more
 # (a tile costs a block about 0.8 us while the GPU is not full, a second level of combining
@@ -539,6 +539,26 @@ decode_ws_split_coef = 0.8
 decode_ws_unsplit_tiles = 4    # (us at 256 / 512 keys, batch 8: 5.4 / 8.4 with 12, 5.4 / 6.0 with 6, 5.9 / 6.0 with 3; 8
                                # layers of the 0.5B shape at batch 8, 230 / 300 / 360 keys: 239 / 247 / 254 us a step
                                # with 6, 237 / 236 / 238 with 4)
+decode_ws_many_unsplit_tiles = 6     # ... and for steps with more (request, kv head) pairs than `decode_ws_few_pairs`
+
+
+def decode_ws_few_pairs(pairs: int, head_dim: int) -> bool:
+    """Whether splitting requests of five and six tiles fills SMs that would idle.  us at 270 / 383 keys, unsplit up
+    to six tiles / up to four: 2 kv heads of 64, 16 requests 5.6, 6.0 / 4.7, 4.9, 64 requests 5.7, 6.2 / 6.2, 6.3;
+    4 of 64, 16 requests 5.6, 6.0 / 4.9, 5.1; 4 of 128 (a tile is twice the bytes), 8 requests 6.1, 6.5 / 5.8, 6.0, 16
+    requests 6.2, 6.7 / 6.5, 6.7, 32 requests 6.5, 6.9 / 7.9, 8.3."""
+    return pairs <= 64 and pairs * head_dim <= 4096
+
+
+def _decode_pairs(num_seqs: int, num_kv_heads: int, group: int) -> int:
+    return num_seqs * num_kv_heads * (-(-group // (8 if group <= 8 else 16)))
+
+
+def decode_ws_unsplit(num_seqs: int, num_kv_heads: int, group: int, head_dim: int) -> int:
+    """Tiles up to which a request of such a step is not split."""
+    few = decode_ws_few_pairs(_decode_pairs(num_seqs, num_kv_heads, group), head_dim)
+    return decode_ws_unsplit_tiles if few else max(decode_ws_unsplit_tiles, decode_ws_many_unsplit_tiles)
+
 
 _DECODE_COUNTERS = 1 << 16     # arrival counters held per device (256 KiB)
 _decode_counters: Dict[int, torch.Tensor] = {}
@@ -556,15 +576,15 @@ def _decode_counter_buffer(device: torch.device) -> torch.Tensor:
 
 
 def decode_ws_splits(num_seqs: int, num_kv_heads: int, group: int, longest_context: int,
-                     max_splits: int, tile_keys: int, cluster: bool = False) -> int:
+                     max_splits: int, tile_keys: int, cluster: bool = False,
+                     unsplit_tiles: Optional[int] = None) -> int:
     """The most splits a request may use (the launch's grid): as many as keep all
     blocks of the step resident at once (two per SM), 1 for short contexts.  ``cluster``:
     the kernel's rule for the cluster form (two tiles a split at least) instead of the one
     for the arrival counter (about ``decode_ws_split_coef`` * sqrt(tiles) tiles a split)."""
-    head_rows = 8 if group <= 8 else 16
-    pairs = num_seqs * num_kv_heads * (-(-group // head_rows))
+    pairs = _decode_pairs(num_seqs, num_kv_heads, group)
     tiles = max(1, -(-longest_context // tile_keys))
-    if tiles <= decode_ws_unsplit_tiles:
+    if tiles <= (decode_ws_unsplit_tiles if unsplit_tiles is None else unsplit_tiles):
         return 1
     slots = 2 * _num_sms()                      # two blocks of three stages fit on an SM
     per = 2 if cluster else max(1, math.ceil(decode_ws_split_coef * math.sqrt(tiles)))
@@ -589,18 +609,19 @@ def decode_attention_takes(head_dim: int, page_size: int) -> bool:
 decode_ws_cluster = True
 
 
-def _decode_launch_shape(ctx, lib, q_device, num_heads, num_kv_heads):
-    """(splits, scratch, counters, cluster) of a launch of the one-launch decode kernel."""
+def _decode_launch_shape(ctx, lib, q_device, num_heads, num_kv_heads, head_dim):
+    """(splits, scratch, counters, cluster, unsplit tiles) of a launch of the one-launch decode kernel."""
     S = ctx.num_seqs
     group = num_heads // num_kv_heads
+    unsplit = decode_ws_unsplit(S, num_kv_heads, group, head_dim)
     splits = decode_ws_force_splits or decode_ws_splits(
         S, num_kv_heads, group, ctx.split_hint_len, lib.slb_decode_attention_ws_max_splits(),
-        lib.slb_decode_attention_ws_tile_keys(), decode_ws_cluster)
+        lib.slb_decode_attention_ws_tile_keys(), decode_ws_cluster, unsplit)
     scratch = counters = None
     cluster = False
     most = lib.slb_decode_attention_ws_max_cluster_splits()
     if splits > 1 and decode_ws_cluster:
-        pairs = S * num_kv_heads * (-(-group // (8 if group <= 8 else 16)))
+        pairs = _decode_pairs(S, num_kv_heads, group)
         if splits > most and pairs * most >= _num_sms():
             splits = most
         if splits > most:
@@ -613,7 +634,7 @@ def _decode_launch_shape(ctx, lib, q_device, num_heads, num_kv_heads):
             nbytes = lib.slb_decode_attention_ws_scratch_bytes(S, num_heads, splits)
             scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=q_device)
             counters = _decode_counter_buffer(q_device)
-    return splits, scratch, counters, cluster
+    return splits, scratch, counters, cluster, unsplit
 
 
 def decode_attention(ctx, q, k_cache, v_cache, out, block_table, num_heads, num_kv_heads,
@@ -628,13 +649,14 @@ def decode_attention(ctx, q, k_cache, v_cache, out, block_table, num_heads, num_
                                head_dim, page_size, scale, window)
         return
     S = ctx.num_seqs
-    splits, scratch, counters, cluster = _decode_launch_shape(ctx, lib, q.device, num_heads, num_kv_heads)
+    splits, scratch, counters, cluster, unsplit = _decode_launch_shape(ctx, lib, q.device, num_heads, num_kv_heads,
+                                                                        head_dim)
     L.check(lib.slb_decode_attention_ws_bf16(
         q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
         out.stride(0), block_table.data_ptr(), block_table.shape[1], ctx.ctx_len.data_ptr(),
         _p(scratch), _p(counters), S, num_heads, num_kv_heads, page_size, k_cache.shape[0],
         float(scale), int(window), splits, int(decode_ws_stages), float(decode_ws_split_coef),
-        int(decode_ws_unsplit_tiles), 1 if cluster else 0, _stream()), "decode_attention")
+        int(unsplit), 1 if cluster else 0, _stream()), "decode_attention")
 
 
 def decode_attention_status(head_dim: int, reset: bool = False) -> int:

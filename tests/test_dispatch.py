@@ -94,3 +94,13 @@ def test_router_of_many_experts_and_tokens_stays_with_the_library():
         assert K.router_takes_tiles(tokens, experts)
     for tokens, experts in ((768, 384), (1024, 256), (2048, 128), (2048, 256), (4096, 96), (4096, 192), (8192, 128)):
         assert not K.router_takes_tiles(tokens, experts)
+
+
+def test_requests_of_five_tiles_are_split_only_while_sms_would_idle():
+    for seqs, kv, group, dim in ((1, 2, 7, 64), (32, 2, 7, 64), (16, 4, 4, 64), (8, 4, 7, 128)):
+        assert K.decode_ws_unsplit(seqs, kv, group, dim) == 4
+        assert K.decode_ws_splits(seqs, kv, group, 300, 64, 64, True, 4) > 1
+    for seqs, kv, group, dim in ((64, 2, 7, 64), (32, 4, 4, 64), (16, 4, 7, 128), (32, 4, 7, 128), (65, 1, 8, 32)):
+        assert K.decode_ws_unsplit(seqs, kv, group, dim) == 6
+        assert K.decode_ws_splits(seqs, kv, group, 384, 64, 64, True, 6) == 1
+        assert K.decode_ws_splits(seqs, kv, group, 385, 64, 64, True, 6) > 1
