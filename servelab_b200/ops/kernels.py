@@ -700,18 +700,29 @@ def tc_token_groups(m: int, w) -> int:
     return -(-m // tc_token_group)
 
 
-def tc_decode_splits(n_out: int, k: int, groups: int = 1) -> int:
-    """K splits so that (row tiles x token groups x splits) is about ``tc_blocks_per_sm``
-    blocks per SM."""
+def _tc_splits(n_out: int, k: int, groups: int, most: int) -> int:
     tiles = -(-n_out // 128) * groups
     kblocks = -(-k // 64)
     slots = tc_blocks_per_sm * _num_sms()
-    want = max(1, slots // tiles) if tiles < slots else 1      # all blocks resident at once
-    # a split streams two k-blocks at least: what a narrow product of a small model takes is the wait for its first
-    # tiles and the way through its epilogue, so fewer k-blocks a block pay although more results are added (8 layers
-    # of the 0.5B shape at batch 1 / 8 / 32 / 64 with four at least: 232 / 262 / 284 / 311 us a step, with two 219 /
-    # 247 / 274 / 305, with one 219 / 238 / 277 / -; the 7B shape's products have enough row tiles)
-    return max(1, min(want, kblocks // 2 if kblocks >= 8 else 1))
+    if tiles >= slots or kblocks < 8:
+        return 1
+
+    def whole(splits):                                         # as many as get k-blocks when each streams as many
+        return -(-kblocks // -(-kblocks // splits))
+    want = min(slots // tiles, most)                           # all blocks resident at once
+    # Two k-blocks a split: what a narrow product of a small model takes is the wait for its first tiles and the way
+    # through its epilogue, so fewer k-blocks a block pay although more results are added (8 layers of the 0.5B shape
+    # at batch 1 / 8 / 32 / 64 with four: 232 / 262 / 284 / 311 us a step, with two 219 / 247 / 274 / 305, with one
+    # 219 / 238 / 277 / -: ahead at 8 requests, behind at 32) -- while most SMs have one block: 64 tokens, K = 896,
+    # 28 tiles 4.4 -> 4.0 us, 36 tiles 4.4 -> 4.7; K = 1,024, 24 tiles 3.9 -> 3.8, 32 tiles 4.0 -> 4.6.  Otherwise four.
+    fine = whole(min(want, kblocks // 2))
+    return fine if 3 * tiles * fine <= 4 * _num_sms() else whole(min(want, kblocks // 4))
+
+
+def tc_decode_splits(n_out: int, k: int, groups: int = 1) -> int:
+    """K splits so that (row tiles x token groups x splits) is about ``tc_blocks_per_sm``
+    blocks per SM and every split has k-blocks of its own."""
+    return _tc_splits(n_out, k, groups, 1 << 30)
 
 
 # rows of gates, then as many of ups, and so on: the layout for which the tcgen05 product
@@ -770,7 +781,8 @@ TC_ROPE_HEAD_DIMS = (16, 32, 64, 128)   # a 128-row tile of the q|k|v product ho
 
 
 def tc_cluster_splits(n_out: int, k: int, groups: int = 1) -> int:
-    return min(tc_decode_splits(n_out, k, groups), TC_MAX_CLUSTER)
+    """The same for splits that form a cluster."""
+    return _tc_splits(n_out, k, groups, TC_MAX_CLUSTER)
 
 
 def gemm_tc_cluster(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,

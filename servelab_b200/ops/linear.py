@@ -68,9 +68,8 @@ cluster_max_tokens_per_block = 8  # tokens a block of the cluster may finish in 
                                   # 17 / 24 / 32 / 48 / 64 requests: 3.04 / 3.47 / 3.43 / 3.95 / 4.43
                                   # against 3.51 / 3.70 / 3.61 / 4.00 / 4.42 -- this package's kernels
                                   # chain through programmatic dependent launch and carry rotation,
-                                  # cache write, residual add and norm in their epilogues.  With few
-                                  # row tiles (the 0.5B shape: 3 K splits, 22 tokens a block at 64
-                                  # requests) the library stays faster: 1.39 against 1.67 ms a step.
+                                  # cache write, residual add and norm in their epilogues.  Small
+                                  # matrices (the 0.5B shape's) are cut into groups of 16 tokens instead.
 cluster_long_k_kblocks = 16      # products whose blocks stream more k-blocks than this ("long K") ...
 cluster_long_k_max_tokens = 64   # ... use the cluster form also from 17 tokens up to here
 fuse_qkv_rope = True       # the q|k|v product of a decode step rotates and writes the cache itself
@@ -82,12 +81,12 @@ def _cluster_ok(x, w, M) -> bool:
         return False
     N, Kd = w.shape
     groups = K.tc_token_groups(M, w)
-    want = K.tc_decode_splits(N, Kd, groups)
-    if want <= 1:
+    splits = K.tc_cluster_splits(N, Kd, groups)
+    if splits <= 1:
         return False
     if groups > 1:
         M = K.tc_token_group                   # (what a block sees)
-    per_block = -(-(-(-Kd // 64)) // min(want, K.TC_MAX_CLUSTER))      # k-blocks of 64 a block streams
+    per_block = -(-(-(-Kd // 64)) // splits)      # k-blocks of 64 a block streams
     if per_block > cluster_max_kblocks:
         return False
     if M <= tc_max_tokens:
@@ -96,7 +95,6 @@ def _cluster_ok(x, w, M) -> bool:
     # its epilogue (tokens rank, rank + splits, ...): the cluster form is taken while that
     # share stays small, or for long K ranges (down), where streaming the weights is most of
     # the time either way (30.8 against 34.1 us with the norm at 64 tokens, 7B shape).
-    splits = min(want, K.TC_MAX_CLUSTER)
     if -(-M // splits) <= cluster_max_tokens_per_block:
         return True
     return per_block > cluster_long_k_kblocks and M <= cluster_long_k_max_tokens

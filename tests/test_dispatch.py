@@ -104,3 +104,15 @@ def test_requests_of_five_tiles_are_split_only_while_sms_would_idle():
         assert K.decode_ws_unsplit(seqs, kv, group, dim) == 6
         assert K.decode_ws_splits(seqs, kv, group, 384, 64, 64, True, 6) == 1
         assert K.decode_ws_splits(seqs, kv, group, 385, 64, 64, True, 6) > 1
+
+
+@pytest.mark.parametrize("n,k,groups,splits", [
+    (896, 896, 1, 7), (1152, 896, 1, 7), (896, 896, 4, 7), (1152, 896, 4, 3), (1024, 1024, 3, 8), (1024, 1024, 4, 4),
+    (640, 1152, 1, 6), (2048, 1152, 1, 6), (2048, 1152, 4, 4), (896, 4864, 1, 8), (9728, 896, 1, 3), (3584, 18944, 1, 8),
+    (4608, 3584, 1, 8), (512, 576, 1, 3), (512, 448, 1, 1), (512, 512, 1, 4)])
+def test_k_splits_have_blocks_of_their_own_and_finer_ones_an_sm(n, k, groups, splits):
+    """Two k-blocks a split while most SMs have one block, else four; no split without any."""
+    assert K.tc_cluster_splits(n, k, groups) == splits
+    kblocks = -(-k // 64)
+    for s in (splits, K.tc_decode_splits(n, k, groups)):
+        assert (s - 1) * -(-kblocks // s) < kblocks
