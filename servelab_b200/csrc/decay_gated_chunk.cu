@@ -20,16 +20,21 @@
 // exponentials, the products and the state (what enters a recurrence stays 32-bit also where the
 // projections are bfloat16).
 //
-// Two launches:
+// Two launches, or four:
 //   1. `prep` per (chunk, head): L for the chunk's tokens and the masked scores A; a record in a work
 //      buffer holds the queries times e^(L_t), the keys times e^(L_last - L_j), A and e^(L_last),
 //      padded as the second launch wants them in shared memory;
 //   2. `walk` per (request, head, slice of EV value columns): the chunks in order with the slice of the
 //      state in shared memory, the next chunk's record fetched by one bulk copy while this one is
 //      worked on; outputs and the new state from the same rows.
-// The state of a chunk never goes to memory (an earlier form with launches for the chunks' own sums, for
-// a scan over them and for the outputs wrote and read it twice: 67 MB each way for 2,048 tokens of 8 heads
-// of 128 x 256).  The result differs from the token-by-token kernel by float32 rounding only, and so does
+//      The state of a chunk never goes to memory;
+//   or, for long requests of few heads and values, whose walk would be a long chain on few SMs:
+//   2. `local` per (chunk, head, 64 value columns): the sum that a chunk adds to the state, into a second buffer;
+//   3. `scan` per (request, head, state element): the buffer is left holding the state that ENTERS every chunk;
+//   4. `out` per (chunk, head, 64 value columns): the outputs.
+//      The states are written and read twice (67 MB each way for 2,048 tokens of 8 heads of 128 x 256), but no
+//      chunk waits for another outside the scan.
+// The result differs from the token-by-token kernel by float32 rounding only, and so does
 // the result of a prompt cut elsewhere.
 #include "decay_attention.cuh"
 #include "mma_util.cuh"
@@ -45,6 +50,7 @@ struct GatedChunkArgs {
     DecayAttnArgs a;
     const int* tile_seq; const int* tile_row0; int num_tiles;
     float* work;                             // [num_tiles][H][gc_floats(D)]
+    float* states;                           // [num_tiles][H][D][Dv] for the form without a walk; null: the walk
 };
 
 // A record: q~ and k~ [32][Dp + 4] (zero rows beyond the chunk's tokens, zero columns beyond D), A [32][36],
@@ -392,6 +398,170 @@ __global__ void __launch_bounds__(512, 1) gated_chunk_walk_kernel(const GatedChu
     }
 }
 
+// ------------------------------------------------------------------ 2b. what a chunk adds to the state
+// Thread (dy, ex): state rows dy, dy + 16, ... and value columns 4 ex .. 4 ex + 3 of the slice.
+#define GC_EV 64
+template <typename T>
+__device__ __forceinline__ void gc_stage_values(const GatedChunkArgs& c, int h, int e0, int t0, int n, float* vs) {
+    const DecayAttnArgs& a = c.a;
+    const T* v = reinterpret_cast<const T*>(a.proj) + (size_t)t0 * a.ld + a.v_off + h * a.Dv + e0;
+#pragma unroll
+    for (int i = 0; i < GC_CHUNK * GC_EV / 256; ++i) {
+        const int j = (threadIdx.x >> 6) + 4 * i, e = threadIdx.x & 63;
+        float x = 0.f;
+        if (j < n && e0 + e < a.Dv) x = to_float(v[(size_t)j * a.ld + e]);
+        vs[j * GC_EV + e] = a.act == 1 ? da_silu(x) : x;
+    }
+}
+template <typename T, int R>
+__global__ void __launch_bounds__(256) gated_chunk_local_kernel(const GatedChunkArgs c) {
+    extern __shared__ __align__(16) float gc_smem[];
+    pdl_wait();
+    pdl_launch_dependents();
+    const DecayAttnArgs& a = c.a;
+    const int tile = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * GC_EV;
+    int t0, n;
+    if (!gc_tile(c, tile, t0, n)) return;
+    const int D = a.D, Dv = a.Dv, LD = gc_ld(D);
+    float* kk = gc_smem;                         // [32][LD]: the record's keys
+    float* vs = kk + GC_CHUNK * LD;              // [32][GC_EV]
+    const float* rec = c.work + ((size_t)tile * a.H + h) * gc_floats(D) + GC_CHUNK * LD;
+    for (int i = threadIdx.x * 4; i < GC_CHUNK * LD; i += 1024)
+        *reinterpret_cast<float4*>(kk + i) = *reinterpret_cast<const float4*>(rec + i);
+    gc_stage_values<T>(c, h, e0, t0, n, vs);
+    __syncthreads();
+    const int ex = threadIdx.x & 15, dy = threadIdx.x >> 4;
+    float acc[R][4];
+#pragma unroll
+    for (int i = 0; i < R; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int j = 0; j < n; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(vs + j * GC_EV + ex * 4);
+        const float* kj = kk + j * LD + dy;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            if (dy + 16 * i >= D) break;
+            const float k = kj[16 * i];
+            acc[i][0] = fmaf(k, v.x, acc[i][0]); acc[i][1] = fmaf(k, v.y, acc[i][1]);
+            acc[i][2] = fmaf(k, v.z, acc[i][2]); acc[i][3] = fmaf(k, v.w, acc[i][3]);
+        }
+    }
+    float* w = c.states + ((size_t)tile * a.H + h) * (size_t)D * Dv + e0 + ex * 4;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int d = dy + 16 * i;
+        if (d >= D) break;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + ex * 4 + u < Dv) w[(size_t)d * Dv + u] = acc[i][u];
+    }
+}
+
+// ------------------------------------------------------------------ 3b. the states that enter the chunks
+#define GC_SCAN_BATCH 16
+__global__ void __launch_bounds__(256) gated_chunk_scan_kernel(const GatedChunkArgs c) {
+    __shared__ int first_s;
+    pdl_wait();
+    pdl_launch_dependents();
+    const DecayAttnArgs& a = c.a;
+    const int s = blockIdx.x, h = blockIdx.y;
+    const int qlen = a.cu_q[s + 1] - a.cu_q[s];
+    if (qlen <= 0) return;
+    const int slot = a.state_slots[s];
+    if (slot < 0 || slot >= a.num_slots) return;
+    if (threadIdx.x == 0) first_s = c.num_tiles;
+    __syncthreads();
+    for (int i = threadIdx.x; i < c.num_tiles; i += 256)       // (a request's chunks are neighbours, in order)
+        if (c.tile_seq[i] == s) { atomicMin(&first_s, i); break; }
+    __syncthreads();
+    const int elems = a.D * a.Dv, idx = blockIdx.z * 256 + threadIdx.x;
+    const int first = first_s, count = (qlen + GC_CHUNK - 1) / GC_CHUNK;
+    if (idx >= elems || first + count > c.num_tiles) return;
+    const int rec = gc_floats(a.D);
+    float* sp = a.state + (size_t)slot * (size_t)a.state_stride + (size_t)h * elems + idx;
+    float* wp = c.states + ((size_t)first * a.H + h) * (size_t)elems + idx;
+    const float* gp = c.work + ((size_t)first * a.H + h) * rec + rec - gc_pad(a.D) + idx / a.Dv;
+    const size_t step = (size_t)a.H * elems, gstep = (size_t)a.H * rec;
+    float S = *sp;
+    for (int k0 = 0; k0 < count; k0 += GC_SCAN_BATCH) {
+        float add[GC_SCAN_BATCH], g[GC_SCAN_BATCH];
+#pragma unroll
+        for (int u = 0; u < GC_SCAN_BATCH; ++u) {
+            add[u] = k0 + u < count ? wp[u * step] : 0.f;
+            g[u] = k0 + u < count ? gp[u * gstep] : 1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < GC_SCAN_BATCH; ++u)
+            if (k0 + u < count) {
+                wp[u * step] = S;
+                S = fmaf(g[u], S, add[u]);
+            }
+        wp += GC_SCAN_BATCH * step;
+        gp += GC_SCAN_BATCH * gstep;
+    }
+    *sp = S;
+}
+
+// ------------------------------------------------------------------ 4b. the chunk's outputs
+// Thread (ty, ex): tokens ty and ty + 16 of the chunk, value columns 4 ex .. 4 ex + 3 of the slice.
+template <typename T>
+__global__ void __launch_bounds__(256) gated_chunk_out_kernel(const GatedChunkArgs c) {
+    extern __shared__ __align__(16) float gc_smem[];
+    pdl_wait();
+    pdl_launch_dependents();
+    const DecayAttnArgs& a = c.a;
+    const int tile = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * GC_EV;
+    int t0, n;
+    if (!gc_tile(c, tile, t0, n)) return;
+    const int slot = a.state_slots[c.tile_seq[tile]];
+    if (slot < 0 || slot >= a.num_slots) return;
+    const int D = a.D, Dv = a.Dv, Dp = gc_pad(D), LD = gc_ld(D);
+    float* q = gc_smem;                          // [32][LD]: the record's queries
+    float* A = q + GC_CHUNK * LD;                // [32][GC_LA]
+    float* vs = A + GC_CHUNK * GC_LA;            // [32][GC_EV]
+    float* S = vs + GC_CHUNK * GC_EV;            // [Dp][GC_EV]: the entering state's slice, zeros beyond it
+    const float* rec = c.work + ((size_t)tile * a.H + h) * gc_floats(D);
+    for (int i = threadIdx.x * 4; i < GC_CHUNK * LD; i += 1024)
+        *reinterpret_cast<float4*>(q + i) = *reinterpret_cast<const float4*>(rec + i);
+    for (int i = threadIdx.x * 4; i < GC_CHUNK * GC_LA; i += 1024)
+        *reinterpret_cast<float4*>(A + i) = *reinterpret_cast<const float4*>(rec + 2 * GC_CHUNK * LD + i);
+    gc_stage_values<T>(c, h, e0, t0, n, vs);
+    const float* w = c.states + ((size_t)tile * a.H + h) * (size_t)D * Dv + e0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < Dp * GC_EV; i += 256) {
+        const int d = i / GC_EV, e = i % GC_EV;
+        S[i] = d < D && e0 + e < Dv ? w[(size_t)d * Dv + e] : 0.f;
+    }
+    __syncthreads();
+    const int ex = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float acc[2][4] = {};
+    auto rows = [&](const float* left, int ld, const float* right, int count) {
+        for (int d = 0; d < count; d += 4) {
+            const float4 l0 = *reinterpret_cast<const float4*>(left + ty * ld + d);
+            const float4 l1 = *reinterpret_cast<const float4*>(left + (ty + 16) * ld + d);
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const float4 r = *reinterpret_cast<const float4*>(right + (d + y) * GC_EV + ex * 4);
+                const float a0 = y == 0 ? l0.x : y == 1 ? l0.y : y == 2 ? l0.z : l0.w;
+                const float a1 = y == 0 ? l1.x : y == 1 ? l1.y : y == 2 ? l1.z : l1.w;
+                acc[0][0] = fmaf(a0, r.x, acc[0][0]); acc[0][1] = fmaf(a0, r.y, acc[0][1]);
+                acc[0][2] = fmaf(a0, r.z, acc[0][2]); acc[0][3] = fmaf(a0, r.w, acc[0][3]);
+                acc[1][0] = fmaf(a1, r.x, acc[1][0]); acc[1][1] = fmaf(a1, r.y, acc[1][1]);
+                acc[1][2] = fmaf(a1, r.z, acc[1][2]); acc[1][3] = fmaf(a1, r.w, acc[1][3]);
+            }
+        }
+    };
+    rows(q, LD, S, Dp);
+    rows(A, GC_LA, vs, GC_CHUNK);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int t = ty + 16 * r;
+        if (t >= n) break;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + ex * 4 + u < Dv) a.out[(size_t)(t0 + t) * a.ldo + h * Dv + e0 + ex * 4 + u] = acc[r][u];
+    }
+}
+
 static size_t gc_prep_smem(int D) {
     const size_t three = (size_t)3 * GC_CHUNK * gc_ld(D), sums = (size_t)GC_CHUNK * gc_ld(D) + 4 * GC_PAIRS * 64;
     return (three > sums ? three : sums) * sizeof(float);
@@ -418,6 +588,25 @@ static int launch_gated_walk(const GatedChunkArgs& c, int num_seqs, cudaStream_t
 }
 
 template <typename T>
+static int launch_gated_parallel(const GatedChunkArgs& c, int num_seqs, cudaStream_t st) {
+    const DecayAttnArgs& a = c.a;
+    const int vz = (a.Dv + GC_EV - 1) / GC_EV, ez = (a.D * a.Dv + 255) / 256;
+    if (vz > 65535 || ez > 65535) return SLB_ERR_TOO_LARGE;
+    auto smem = [](int D, bool out) {
+        return ((size_t)GC_CHUNK * (gc_ld(D) + GC_EV) + (out ? GC_CHUNK * GC_LA + gc_pad(D) * GC_EV : 0)) * sizeof(float);
+    };
+    static unsigned long long conf = 0;
+    int rc = slb_configure(&conf, gated_chunk_out_kernel<T>, smem(GC_MAX_D, true));
+    if (rc != 0) return rc;
+    auto local = a.D <= 128 ? gated_chunk_local_kernel<T, 8> : gated_chunk_local_kernel<T, GC_MAX_D / 16>;
+    rc = slb_launch(local, dim3(c.num_tiles, a.H, vz), dim3(256), smem(a.D, false), st, c);
+    if (rc != 0) return rc;
+    rc = slb_launch(gated_chunk_scan_kernel, dim3(num_seqs, a.H, ez), dim3(256), 0, st, c);
+    if (rc != 0) return rc;
+    return slb_launch(gated_chunk_out_kernel<T>, dim3(c.num_tiles, a.H, vz), dim3(256), smem(a.D, true), st, c);
+}
+
+template <typename T>
 static int launch_gated_chunk(const GatedChunkArgs* c_in, int num_seqs, cudaStream_t st) {
     if (num_seqs <= 0 || c_in->num_tiles <= 0) return 0;
     GatedChunkArgs c = *c_in;
@@ -436,6 +625,7 @@ static int launch_gated_chunk(const GatedChunkArgs* c_in, int num_seqs, cudaStre
     if (rc != 0) return rc;
     rc = slb_launch(gated_chunk_prep_kernel<T>, dim3(c.num_tiles, a.H), dim3(256), gc_prep_smem(a.D), st, c);
     if (rc != 0) return rc;
+    if (c.states != nullptr) return launch_gated_parallel<T>(c, num_seqs, st);
     // (the walk is serial in a request's chunks: with few heads and values, slices of 8 columns, so that twice
     // as many SMs share a chunk's work)
     const long long slices = (long long)num_seqs * a.H * ((a.Dv + 15) / 16);
@@ -445,6 +635,16 @@ static int launch_gated_chunk(const GatedChunkArgs* c_in, int num_seqs, cudaStre
 extern "C" {
 int slb_decay_gated_chunk_max_dim() { return GC_MAX_D; }
 int slb_decay_gated_chunk_tokens() { return GC_CHUNK; }
+// 1: chunks of such a step are better worked on side by side (`states` is then wanted).  The walk costs 1.0 us a
+// chunk of the longest request, the form without it two launches more, some 12 us, and the states' way through
+// memory, 13 us for 2^20 elements.  Measured us walked / side by side, one request, by tokens: 4 heads of 64 x 128
+// 2,048 75 / 52, 8,192 280 / 137; 2 of 64 x 64 1,024 41 / 26; 1 of 128 x 128 1,024 53 / 36, 8,192 316 / 104; 8 of
+// 64 x 64 2,048 83 / 57; 8 of 128 x 256 2,048 145 / 224, 8,192 550 / 935 (the latter with a slower first launch).
+// (The mean length stands for the longest: a step that is captured for later ones knows no more.)
+int slb_decay_gated_chunk_side_by_side(int num_tiles, int num_seqs, int H, int D, int Dv) {
+    const double chunks = (double)num_tiles / (num_seqs > 0 ? num_seqs : 1);
+    return 0.95 * chunks > 14.0 + 13.0 / (1 << 20) * ((double)num_tiles * H * D * Dv);
+}
 int slb_decay_gated_chunk_work_floats(int D) { return gc_floats(D); }
 int slb_decay_gated_chunk_f32(const GatedChunkArgs* c, int num_seqs, cudaStream_t st) {
     return launch_gated_chunk<float>(c, num_seqs, st);

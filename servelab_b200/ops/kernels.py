@@ -1522,13 +1522,14 @@ class _DecayChunkArgs(_ct.Structure):
 
 class _GatedChunkArgs(_ct.Structure):
     _fields_ = [("a", _DecayAttnArgs), ("tile_seq", _ct.c_void_p), ("tile_row0", _ct.c_void_p),
-                ("num_tiles", _ct.c_int), ("work", _ct.c_void_p)]
+                ("num_tiles", _ct.c_int), ("work", _ct.c_void_p), ("states", _ct.c_void_p)]
 
 
 # Learned decays: steps that bring portions of prompts in bfloat16 take the chunked kernels (float32
 # arithmetic on the CUDA cores, chunks of 32 tokens) from the same number of tokens a request on.
 decay_gated_chunked = True
 force_gated_chunks = False       # (tests: the chunked kernels also for float32 rows)
+force_side_by_side = None        # (tests: chunks side by side, or walked over; None: by the step's sizes)
 
 
 # Steps that bring portions of prompts in bfloat16 take the chunked tensor-core kernels when the
@@ -1587,10 +1588,15 @@ def decay_attention(proj: torch.Tensor, ctx, state: torch.Tensor, decay: Optiona
         work = torch.empty((max(n, 1), num_heads, L.core().slb_decay_gated_chunk_work_floats(head_dim)), dtype=_F32,
                            device=proj.device)
         c.work = work.data_ptr()
+        side_by_side = (force_side_by_side if force_side_by_side is not None else
+                        L.core().slb_decay_gated_chunk_side_by_side(n, ctx.num_seqs, num_heads, head_dim, value_dim))
+        if side_by_side:
+            states = torch.empty((max(n, 1), num_heads, head_dim, value_dim), dtype=_F32, device=proj.device)
+            c.states = states.data_ptr()
         fn = getattr(L.core(), "slb_decay_gated_chunk_" + _suffix(proj.dtype))
         L.check(fn(_ct.byref(c), ctx.num_seqs, _stream()), "decay_attention (gated chunks)")
         global launch_count
-        launch_count += 1
+        launch_count += 3 if side_by_side else 1
         return
     if (decay_attention_chunked and plain and proj.dtype == torch.bfloat16 and not ctx.decode_only
             and head_dim <= L.core().slb_decay_chunk_max_dim()

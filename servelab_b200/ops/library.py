@@ -136,6 +136,7 @@ _CORE_SIGNATURES = {
     "slb_decay_gated_chunk_max_dim": [],
     "slb_decay_gated_chunk_tokens": [],
     "slb_decay_gated_chunk_work_floats": [I],
+    "slb_decay_gated_chunk_side_by_side": [I, I, I, I, I],
     "slb_decay_gated_chunk_status": [I],
     "slb_decay_gated_chunk_f32": [P, I, P],
     "slb_decay_gated_chunk_bf16": [P, I, P],

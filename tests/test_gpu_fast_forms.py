@@ -424,6 +424,41 @@ def test_walk_over_the_chunks_against_the_recurrence(D, Hh, Dv):
     assert (out.double().cpu() - want).abs().max() < 3e-5 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("D,Dv", [(60, 200), (64, 64), (128, 20), (132, 72), (256, 8)])
+@pytest.mark.parametrize("lens", [[31, 32, 70], [600]])
+def test_chunks_side_by_side_against_the_recurrence(monkeypatch, D, Dv, lens):
+    """The form without a walk over the chunks (up to 128 and more state rows a block, slices of values that end
+    anywhere, more chunks than the scan loads at once), to the bound that the walk is held to; the records it leaves
+    are the walk's bits, whose sums have the same order."""
+    import test_gpu_sumolorn as case
+    from servelab_b200.ops import kernels
+    H, T = 2, sum(lens)
+    proj, z, bias = case._gated_case(5, H, D, Dv, T, torch.bfloat16, z_shift=1.0)
+    want = case._gated_want(proj, z, bias, H, D, Dv, lens, 4.0, D ** -0.5)
+    at, parts = 0, []
+    for i, n in enumerate(lens):
+        parts.append((i, at, n))
+        at += n
+    states = []
+    for form in (True, False):
+        monkeypatch.setattr(kernels, "force_side_by_side", form)
+        states.append(torch.zeros(len(lens), H * D * Dv, device="cuda"))
+        out = case._run_gated_chunked(kernels, proj.cuda(), z.cuda(), bias.cuda(), states[-1], H, D, Dv, [parts], 4.0,
+                                      D ** -0.5)
+        assert (out.double().cpu() - want).abs().max() < 3e-5 * max(1.0, float(want.abs().max()))
+    assert torch.equal(*states)
+
+
+def test_long_requests_of_few_values_have_their_chunks_side_by_side():
+    """The points at which both forms were measured, chunks of 32 tokens."""
+    from servelab_b200.ops import library as L
+    rule = L.core().slb_decay_gated_chunk_side_by_side
+    assert all(rule(*p) for p in ((64, 1, 4, 64, 128), (32, 1, 2, 64, 64), (32, 1, 1, 128, 128), (256, 1, 8, 64, 64),
+                                  (64, 2, 1, 128, 128)))
+    assert not any(rule(*p) for p in ((16, 1, 4, 64, 128), (16, 1, 1, 128, 128), (64, 1, 8, 128, 256), (64, 1, 16, 128, 128),
+                                      (256, 1, 8, 128, 256), (127, 64, 4, 64, 128), (64, 64, 1, 64, 64), (512, 64, 8, 64, 64)))
+
+
 @pytest.mark.parametrize("D,Dv", [(64, 64), (128, 40), (192, 64)])
 def test_scans_over_chunks_report_waits_that_gave_up(D, Dv):
     """Two and one record a block (key sizes up to 128 and above), requests of one and of several chunks: no wait
