@@ -626,10 +626,11 @@ static int launch_gated_chunk(const GatedChunkArgs* c_in, int num_seqs, cudaStre
     rc = slb_launch(gated_chunk_prep_kernel<T>, dim3(c.num_tiles, a.H), dim3(256), gc_prep_smem(a.D), st, c);
     if (rc != 0) return rc;
     if (c.states != nullptr) return launch_gated_parallel<T>(c, num_seqs, st);
-    // (the walk is serial in a request's chunks: with few heads and values, slices of 8 columns, so that twice
-    // as many SMs share a chunk's work)
+    // (the walk is serial in a request's chunks: while slices of 16 columns leave half of the SMs idle, slices of 8
+    // share a chunk's work among twice as many: 512 tokens of 1 head of 128 x 128 34.6 us, 42.9 with 16; 1,024 +
+    // 1,024 of 4 heads of 96 x 96 54 and 69; 256 of 4 heads of 64 x 128 18.3 and 20.6)
     const long long slices = (long long)num_seqs * a.H * ((a.Dv + 15) / 16);
-    return slices < 74 ? launch_gated_walk<T, 8>(c, num_seqs, st) : launch_gated_walk<T, 16>(c, num_seqs, st);
+    return 2 * slices < slb_num_sms() ? launch_gated_walk<T, 8>(c, num_seqs, st) : launch_gated_walk<T, 16>(c, num_seqs, st);
 }
 
 extern "C" {

@@ -90,9 +90,10 @@ static int launch_gemm(const TA* A, int lda, const TW* W, int ldw, TC* C, int ld
 // The same sums in the same order (one FFMA per product, k = 0..K-1: results are bit for bit those of
 // the kernel above), with the operands brought in by cp.async through a ring of G_STAGES tiles.  What
 // bounds it is the FFMA rate (74 TFLOP/s): the kernel above waits for scattered 4-byte loads twice a
-// k-tile.  It reaches 45 TFLOP/s (1,024 x 32,000 x 896), bound by shared-memory reads.  A tile row keeps its k elements side by side (as in memory, so a piece is
-// copied as it is) with 4 floats of padding, which makes the 16-byte reads of 8 neighbouring rows
-// free of bank conflicts; a thread owns rows ty + i TY and columns tx + j TX, so a warp's reads of W
+// k-tile.  It reaches 46 TFLOP/s at 1,024 x 32,000 x 896, bound by shared-memory reads, and 32 and 20 at
+// 257 x 9,728 x 896 and 257 x 896 x 4,864, whose last wave of tiles is ragged.  A tile row keeps its k
+// elements side by side (as in memory, so a piece is copied as it is) with 4 floats of padding, which
+// makes the 16-byte reads of 8 neighbouring rows free of bank conflicts; a thread owns rows ty + i TY and columns tx + j TX, so a warp's reads of W
 // are neighbouring rows and its stores neighbouring columns.
 #define G_STAGES 4
 #define G_PAD 4
@@ -199,8 +200,8 @@ static int launch_f32_tile(const F32Args& g, cudaStream_t st) {
     const int err = slb_configure(&configured, kernel, smem);
     if (err) return err;
     return slb_launch_after(kernel, dim3((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, g.batch),
-                            dim3((BM / TM) * (BN / TN)), smem, st, g.A, g.lda, g.W, g.ldw, g.C, g.ldc, g.bias, g.M, g.N, g.K, g.batch_a, g.batch_w,
-                            g.batch_c);
+                            dim3((BM / TM) * (BN / TN)), smem, st, g.A, g.lda, g.W, g.ldw, g.C, g.ldc, g.bias, g.M, g.N,
+                            g.K, g.batch_a, g.batch_w, g.batch_c);
 }
 
 // Which tile: the products are sums in order, so K is not split, and the tiles differ in how many
@@ -212,12 +213,13 @@ static int launch_f32_tile(const F32Args& g, cudaStream_t st) {
 static int launch_f32(const F32Args& g, cudaStream_t st) {
     struct Tile { int bm, bn; float first, next; };
     static const Tile tiles[] = {{64, 128, 62.f, 45.f}, {32, 128, 39.5f, 26.f}, {32, 64, 23.f, 13.5f}, {16, 64, 19.f, 10.5f}};
+    const int sms = slb_num_sms();
     int best = 0;
     double least = 0.0;
     for (int i = 0; i < 4; ++i) {
         const long long n = (long long)((g.M + tiles[i].bm - 1) / tiles[i].bm) *
                             ((g.N + tiles[i].bn - 1) / tiles[i].bn) * g.batch;
-        const double cost = tiles[i].first + (double)((n + 147) / 148 - 1) * tiles[i].next;
+        const double cost = tiles[i].first + (double)((n + sms - 1) / sms - 1) * tiles[i].next;
         if (i == 0 || cost < least) { least = cost; best = i; }
     }
     switch (best) {

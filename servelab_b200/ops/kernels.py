@@ -1244,9 +1244,11 @@ def moe_route(logits: torch.Tensor, groups: int, keep: int, top: int, route_scal
 
 moe_vendor_grouped = True      # bfloat16 steps of many rows: the vendor's grouped product (off: this package's)
 moe_vendor_min_pairs = 1024    # (token, choice) pairs from which it is taken ...
-moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this many elements a matrix (measured:
-                                           # width 2,048 x 1,408: 2.8 -> 1.1 ms a 2,048-token step of 4 layers;
-                                           # 1,024 x 512: 0.40 -> 0.62 ms with the copies around it)
+moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this many elements a matrix.  Own / vendor,
+                                           # us, 4 experts a token: 32 of 2,048 x 1,408, 128 tokens 136 / 144, 160 144 /
+                                           # 143, 256 178 / 145, 2,048 695 / 208; 16 of 1,024 x 512, 128 tokens 36 /
+                                           # 37, 256 44 / 38, 512 66 / 40, 2,048 160 / 72: the vendor's is ahead of
+                                           # the smaller ones too, which stay with this package's kernel all the same
 moe_tensor_cores = True        # bfloat16: the experts' products on mma.sync (off: CUDA cores, the twin)
 
 
