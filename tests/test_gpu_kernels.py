@@ -851,7 +851,9 @@ def test_gemm_tcgen05_cluster(M, N, Kd, splits):
     out = torch.full((M, N), 9.0, device=DEV, dtype=torch.bfloat16)
     K().gemm_tc_cluster(x, w, out, b, splits)
     assert K().gemm_tc_status(True) == 0, "a bounded wait in the kernel ran out"
-    assert (out.float() - want).abs().max() <= 2e-2
+    # (a value of 8 and more, which the unseeded inputs bring now and then, is rounded by up to 2^-8 of itself; beside
+    # that the float32 sum's 2e-3)
+    assert ((out.float() - want).abs() <= torch.clamp(want.abs() * 2.0 ** -8 + 2e-3, min=2e-2)).all()
     again = torch.empty_like(out)
     K().gemm_tc_cluster(x, w, again, b, splits)
     assert torch.equal(again, out)
