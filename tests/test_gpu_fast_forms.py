@@ -477,3 +477,47 @@ def test_scans_over_chunks_report_waits_that_gave_up(D, Dv):
                         num_heads=H, head_dim=D, value_dim=Dv, gate_z=z, gate_tau=4.0)
     assert out.isfinite().all() and rows.isfinite().all()
     assert K().delta_chunk_status() == 0 and K().decay_gated_chunk_status() == 0
+
+
+# ----------------------------------------------------- more splits in decode steps, and their error
+@pytest.mark.parametrize("N,Kd", [(896, 896), (640, 1152), (896, 4864)])
+def test_finer_k_splits_are_no_less_exact(N, Kd):
+    """Ten inputs, the chosen splits against one: float32 sums in another order under the same rounding to bfloat16,
+    which makes nearly all of the error."""
+    assert K().tc_cluster_splits(N, Kd) > 5
+    total = {0: 0.0, 1: 0.0}
+    for seed in range(10):
+        g = gen(seed)
+        x, w = torch.randn(3, Kd, device=DEV, generator=g).bfloat16(), (torch.randn(N, Kd, device=DEV, generator=g) * 0.05).bfloat16()
+        want = x.double() @ w.double().T
+        for splits in total:
+            total[splits] += float((K().gemm_tc_cluster(x, w, splits=splits).double() - want).norm() / want.norm())
+    assert total[0] <= 1.005 * total[1] and total[1] < 10 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("H,G,D", [(14, 2, 64), (28, 4, 128)])
+def test_split_requests_of_five_tiles_are_no_less_exact(monkeypatch, H, G, D):
+    """Ten inputs, 8 requests of 270 to 384 keys, the chosen splits against none: the same keys with the largest score
+    of a split in place of the request's; the probabilities' and the result's rounding make the error."""
+    lens = [270, 300, 319, 320, 321, 350, 383, 384]
+    ctx, pages = step([1] * 8, [n - 1 for n in lens])
+    assert K().decode_ws_unsplit(8, G, H // G, D) < 5
+    total = {0: 0.0, 1: 0.0}
+    for seed in range(10):
+        g = gen(seed)
+        q, kc, vc = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((8, H * D), (pages, G, 16, D), (pages, G, 16, D)))
+        want, at = [], 0
+        for i, n in enumerate(lens):
+            used = -(-n // 16)
+            k, v = (c[at:at + used].transpose(0, 1).reshape(G, used * 16, D)[:, :n].double() for c in (kc, vc))
+            p = torch.softmax(q[i].double().view(G, H // G, D) @ k.transpose(1, 2) * D ** -0.5, -1)
+            want.append((p @ v).reshape(-1))
+            at += used
+        want = torch.stack(want)
+        for splits in total:
+            monkeypatch.setattr(K(), "decode_ws_force_splits", splits)
+            out = torch.empty(8, H * D, device=DEV, dtype=torch.bfloat16)
+            K().decode_attention(ctx, q, kc, vc, out, ctx.block_tables[0], H, G, D, 16, D ** -0.5, 0)
+            total[splits] += float((out.double() - want).norm() / want.norm())
+    assert total[0] <= 1.03 * total[1] and total[1] < 10 * 2.0 ** -7
+    assert K().decode_attention_status(D) == 0
