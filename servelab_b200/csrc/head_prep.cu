@@ -199,7 +199,6 @@ struct HeadPrepKind {
     int units, items;        // vectors; warps' worth of vectors
     int norm, rot, unit;     // pieces that are normed, first piece that is rotated, pieces of the unit norm
     int skip;                // pieces that are not written
-    int drop;                // elements before `off` of a vector that are not read (a bias has them too)
 };
 struct HeadPrepPlan { HeadPrepKind kind[3]; int items; };
 
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
                     float v[8], b[8];
                     unpack8(raw[j][c], v);
                     if (bias != nullptr) {
-                        load8_weights(bias + unit[j] * kd.stride + kd.drop + piece * 8, b);
+                        load8_weights(bias + unit[j] * kd.stride + piece * 8, b);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) v[e] += b[e];
                     }
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
                 unpack8(raw[j][c], v[c]);
                 if (bias != nullptr && u < kd.units && piece < kd.pieces) {
                     float b[8];
-                    load8_weights(bias + u * kd.stride + kd.drop + piece * 8, b);
+                    load8_weights(bias + u * kd.stride + piece * 8, b);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[c][e] += b[e];
                 }
@@ -461,13 +460,17 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
 static int max_of(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 static bool pieces(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
+// What is not written and enters no sum is not read either (a latent attention's unrotated queries).
+static int head_prep_drop(int norm, int unit, int rot_off, int skip) {
+    return norm == 0 && unit == 0 && rot_off >= skip ? skip : 0;
+}
+
 // One kind of vector for the kernel in pieces; false: it does not take these sizes.
 static bool head_prep_kind(HeadPrepKind* kd, int off, int D, int units, int norm, int rot_off, int rot_dims,
                            int unit, int skip, int rot_half) {
     *kd = HeadPrepKind{};
     if (units == 0) return true;
-    // what is not written and enters no sum is not read either (a latent attention's unrotated queries)
-    const int drop = norm == 0 && unit == 0 && rot_off >= skip ? skip : 0;
+    const int drop = head_prep_drop(norm, unit, rot_off, skip);
     if ((off | D | norm | rot_off | rot_dims | unit | skip) & 7) return false;
     if (rot_half && (rot_dims & 15)) return false;
     kd->off = off + drop;
@@ -481,7 +484,6 @@ static bool head_prep_kind(HeadPrepKind* kd, int off, int D, int units, int norm
     kd->rot = (rot_off - drop) / 8;
     kd->unit = unit / 8;
     kd->skip = (skip - drop) / 8;
-    kd->drop = drop;
     return true;
 }
 
@@ -584,7 +586,10 @@ static int launch_head_prep(const HeadPrepArgs& a, int num_tokens, cudaStream_t 
         const bool wide = plan.kind[0].pieces > 32 || plan.kind[1].pieces > 32 || plan.kind[2].pieces > 32;
         auto kernel = a.row_norm ? (wide ? head_prep_vec_kernel<2, true> : head_prep_vec_kernel<1, true>)
                                  : (wide ? head_prep_vec_kernel<2, false> : head_prep_vec_kernel<1, false>);
-        return slb_launch(kernel, dim3(num_tokens, split), dim3(warps * 32), a.rot_dims * sizeof(float), st, a, plan);
+        HeadPrepArgs read = a;                           // (a bias has the elements too that are not read)
+        if (a.q_bias != nullptr && !a.row_norm)
+            read.q_bias += head_prep_drop(a.q_norm_dims, a.q_unit_dims, a.rot_dims ? a.q_rot_off : 0, a.q_skip);
+        return slb_launch(kernel, dim3(num_tokens, split), dim3(warps * 32), a.rot_dims * sizeof(float), st, read, plan);
     }
     const size_t smem = ((size_t)HP_WARPS * maxd + a.rot_dims) * sizeof(float);
     const int units = a.H + a.G + (a.v_off >= 0 ? a.G : 0);
