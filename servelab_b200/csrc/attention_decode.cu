@@ -123,7 +123,7 @@ __device__ __forceinline__ BoxGeometry box_geometry(int rows) {
     return geo;
 }
 
-// One tile's copies, issued by the calling warp.  Lane b handles box b (box_rows keys of
+// One tile's copies, issued by the calling warp.  Lane b looks box b up (box_rows keys of
 // one page, every panel, in ONE tiled copy each for K and V); `page` is that box's entry
 // of the block table.  Boxes that are not fetched are zero-filled by the whole warp with
 // ordinary stores; lane 0 arrives on `bar` (count 1) with the bytes of all copies.
@@ -150,19 +150,20 @@ __device__ __forceinline__ void produce_tile(unsigned char* Kd, unsigned char* V
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
     }
-    if (lane == 0) {
+    if (slb_elected()) {
         const uint32_t bytes = (uint32_t)__popc(fetched) * (uint32_t)geo.box_bytes * 2u;
         if (bytes) mbar_arrive_expect_tx(bar, bytes); else mbar_arrive(bar);
     }
-    __syncwarp();
-    if (row0 >= 0) {
-        if (evict_first) {                                 // the cache is streamed once a step
-            const uint64_t policy = l2_evict_first_policy();
-            slb_tma::tma_load_3d_hint(Kd + lane * geo.box_bytes, map_k, bar, 0, row0, 0, policy);
-            slb_tma::tma_load_3d_hint(Vd + lane * geo.box_bytes, map_v, bar, 0, row0, 0, policy);
+    const uint64_t policy = l2_evict_first_policy();       // (the cache is streamed once a step)
+    for (int b = 0; b < geo.boxes; ++b) {
+        const int row = __shfl_sync(0xffffffffu, row0, b);
+        if (row < 0 || !slb_elected()) continue;
+        if (evict_first) {
+            slb_tma::tma_load_3d_hint(Kd + b * geo.box_bytes, map_k, bar, 0, row, 0, policy);
+            slb_tma::tma_load_3d_hint(Vd + b * geo.box_bytes, map_v, bar, 0, row, 0, policy);
         } else {
-            tma_load_3d(Kd + lane * geo.box_bytes, map_k, bar, 0, row0, 0);
-            tma_load_3d(Vd + lane * geo.box_bytes, map_v, bar, 0, row0, 0);
+            tma_load_3d(Kd + b * geo.box_bytes, map_k, bar, 0, row, 0);
+            tma_load_3d(Vd + b * geo.box_bytes, map_v, bar, 0, row, 0);
         }
     }
 }

@@ -136,8 +136,8 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // same with the A operand in tensor memory (lane = row, 32-bit columns of two bfloat16)
@@ -146,8 +146,8 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
 
     pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = slb_warp(), lane = threadIdx.x & 31;
     // Blocks are handed out in the order of their linear index: tile by tile from the last
     // (most keys) to the first, all kv heads of a tile together, so that no head's long
     // tiles start late.
@@ -283,8 +283,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
         // Warp 0 fetches the keys, warp 6 the values, each through its own two-stage ring:
         // the keys of a tile may be replaced when its Q.K^T has run (two softmax periods
         // before the new ones are needed), the values when its P.V has.  Lane b looks up the
-        // page of box b, one tile ahead of its use (a dependent global load), and issues the
-        // box's copies (a copy costs the issuing warp 60 to 160 cycles: spread over lanes).
+        // page of box b, one tile ahead of its use (a dependent global load).
         const bool keys = warp == 0;
         const CUtensorMap* map = keys ? &map_k : &map_v;
         unsigned char* ring = smem + (keys ? OFF_K : OFF_V);
@@ -312,38 +311,40 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
                 break;
             }
             const unsigned got = __ballot_sync(0xffffffffu, row >= 0);
-            if (lane == 0) {
+            if (slb_elected()) {
                 const uint32_t bytes = (uint32_t)__popc(got) * (uint32_t)box_rows * 128u * PANELS;
                 if (bytes) mbar_expect_tx(&full[st], bytes); else mbar_arrive(&full[st]);
             }
-            __syncwarp();
-            if (row >= 0) {
+            for (int b = 0; b < boxes; ++b) {
+                const int box_row = __shfl_sync(0xffffffffu, row, b);
+                if (box_row >= 0 && slb_elected()) {
 #pragma unroll
-                for (int p = 0; p < PANELS; ++p)
-                    tma_load_2d(ring + st * KV_TILE_BYTES + p * KV_PANEL_BYTES + lane * box_rows * 128, map,
-                                &full[st], p * 64, row);
+                    for (int p = 0; p < PANELS; ++p)
+                        tma_load_2d(ring + st * KV_TILE_BYTES + p * KV_PANEL_BYTES + b * box_rows * 128, map, &full[st],
+                                    p * 64, box_row);
+                }
             }
             row = next_row;
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                      ((uint32_t)(BM >> 4) << 24);
-            const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                      ((uint32_t)(D >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            // operand descriptors are built once; a step along K or to another panel adds its
-            // byte offset / 16 to the address field
-            const uint64_t q_desc = umma_desc(smem_u32(smem + OFF_Q), 1);
-            const uint64_t k_desc0 = umma_desc(smem_u32(smem + OFF_K), 1);
-            const uint64_t v_desc0 = umma_desc(smem_u32(smem + OFF_V), KV_PANEL_BYTES >> 4);
-            constexpr uint64_t STAGE_STEP = KV_TILE_BYTES >> 4;      // to the second stage
-            // S = Q.K^T of tile t into score buffer t & 1 (which held the scores and then P of
-            // tile t - 2; its P.V has been issued before)
-            auto issue_qk = [&](int t) -> bool {
-                const int st = t & 1;
-                if (!mbar_spin(&k_full[st], (t >> 1) & 1)) { gave_up(status, 0x201, 1, t, ntiles); return false; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
+                                  ((uint32_t)(BM >> 4) << 24);
+        const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
+                                  ((uint32_t)(D >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        // operand descriptors are built once; a step along K or to another panel adds its
+        // byte offset / 16 to the address field
+        const uint64_t q_desc = umma_desc(smem_u32(smem + OFF_Q), 1);
+        const uint64_t k_desc0 = umma_desc(smem_u32(smem + OFF_K), 1);
+        const uint64_t v_desc0 = umma_desc(smem_u32(smem + OFF_V), KV_PANEL_BYTES >> 4);
+        constexpr uint64_t STAGE_STEP = KV_TILE_BYTES >> 4;      // to the second stage
+        // S = Q.K^T of tile t into score buffer t & 1 (which held the scores and then P of
+        // tile t - 2; its P.V has been issued before)
+        auto issue_qk = [&](int t) -> bool {
+            const int st = t & 1;
+            if (!mbar_spin(&k_full[st], (t >> 1) & 1)) { gave_up(status, 0x201, 1, t, ntiles); return false; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (slb_elected()) {
 #pragma unroll
                 for (int p = 0; p < PANELS; ++p)
 #pragma unroll
@@ -352,25 +353,27 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
                                   k_desc0 + st * STAGE_STEP + ((p * KV_PANEL_BYTES + kk * 32) >> 4), idesc_qk,
                                   (p > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&s_full[st]);
-                return true;
-            };
-            bool ok = issue_qk(0);
-            if (ok && ntiles > 1) ok = issue_qk(1);
-            for (int j = 0; j < ntiles && ok; ++j) {
-                const int st = j & 1;
-                if (!mbar_spin(&p_full[st], (j >> 1) & 1)) { gave_up(status, 0x202, 1, j, ntiles); break; }
-                if (!mbar_spin(&v_full[st], (j >> 1) & 1)) { gave_up(status, 0x203, 1, j, ntiles); break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            return true;
+        };
+        bool ok = issue_qk(0);
+        if (ok && ntiles > 1) ok = issue_qk(1);
+        for (int j = 0; j < ntiles && ok; ++j) {
+            const int st = j & 1;
+            if (!mbar_spin(&p_full[st], (j >> 1) & 1)) { gave_up(status, 0x202, 1, j, ntiles); break; }
+            if (!mbar_spin(&v_full[st], (j >> 1) & 1)) { gave_up(status, 0x203, 1, j, ntiles); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (slb_elected()) {
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk)              // 16 keys per step: P 8 columns, V 16 rows
                     umma_bf16_ts(tmem + O_COL, tmem + S_COL + 64 * st + kk * 8,
                                  v_desc0 + st * STAGE_STEP + ((kk * 16 * 128) >> 4), idesc_pv,
                                  (j > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&pv_done[st]);
-                // the scores of tile j + 2 go where P of tile j was: issued after P.V of tile j
-                // (the tensor core executes in issue order), while the softmax of j + 1 runs
-                if (j + 2 < ntiles) ok = issue_qk(j + 2);
             }
+            // the scores of tile j + 2 go where P of tile j was: issued after P.V of tile j
+            // (the tensor core executes in issue order), while the softmax of j + 1 runs
+            if (j + 2 < ntiles) ok = issue_qk(j + 2);
         }
     } else {
         // ---------------------------------------------------------------- softmax + epilogue

@@ -118,8 +118,8 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_decode_kernel(
     uint64_t* accum = empty + TC_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = slb_warp(), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * TC_BM;
     const int splits = gridDim.y, split = blockIdx.y;
     const int kblocks = (K + TC_BK - 1) / TC_BK;
@@ -262,53 +262,64 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_decode_kernel(
         // ------------------------------------------------------------ loader
         // W is written by no kernel, x by the preceding one: the W tiles of the first
         // stages are requested at once, the x tiles after the wait for that kernel.
-        if (lane == 0) {
-            const uint32_t bytes = A_STAGE_BYTES + (uint32_t)ntok16 * TC_BK * 2;
-            const bool w_first = (flags & SLB_FLAG_EVICT_FIRST) != 0;
-            const uint64_t w_policy = w_first ? l2_evict_first_policy() : 0;
-            const int ahead = min(iters, TC_STAGES);
-            for (int i = 0; i < ahead; ++i) {                 // stages are empty at the start
+        const uint32_t bytes = A_STAGE_BYTES + (uint32_t)ntok16 * TC_BK * 2;
+        const bool w_first = (flags & SLB_FLAG_EVICT_FIRST) != 0;
+        const uint64_t w_policy = w_first ? l2_evict_first_policy() : 0;
+        const int ahead = min(iters, TC_STAGES);
+        for (int i = 0; i < ahead; ++i)                       // stages are empty at the start
+            if (slb_elected()) {
                 mbar_expect_tx(&full[i], bytes);
                 load_w_tile(a_stage + i * A_STAGE_BYTES, &map_w, &full[i], (kb_begin + i) * TC_BK, n0, w_first, w_policy);
             }
-            pdl_wait();
-            for (int i = 0; i < ahead; ++i)
+        pdl_wait();
+        for (int i = 0; i < ahead; ++i)
+            if (slb_elected())
                 tma_load_2d(b_stage + i * B_STAGE_BYTES, &map_x, &full[i], (kb_begin + i) * TC_BK, tok_base);
-            for (int i = ahead; i < iters; ++i) {
-                const int s = i % TC_STAGES;
-                if (!mbar_wait(&empty[s], ((i / TC_STAGES) & 1) ^ 1)) {
-                    atomicCAS(status, 0, (1 << 8) | 1);
-                    break;
-                }
+        int s = 0;
+        uint32_t phase = 0;
+        for (int i = ahead; i < iters; ++i) {
+            if (!mbar_wait(&empty[s], phase)) {
+                atomicCAS(status, 0, (1 << 8) | 1);
+                break;
+            }
+            const int k = (kb_begin + i) * TC_BK;
+            if (slb_elected()) {
                 mbar_expect_tx(&full[s], bytes);
-                const int k = (kb_begin + i) * TC_BK;
                 load_w_tile(a_stage + s * A_STAGE_BYTES, &map_w, &full[s], k, n0, w_first, w_policy);
                 tma_load_2d(b_stage + s * B_STAGE_BYTES, &map_x, &full[s], k, tok_base);
+            }
+            if (++s == TC_STAGES) {
+                s = 0;
+                phase ^= 1;
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            // instruction descriptor: D float32, A and B bfloat16, both K-major
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                   ((uint32_t)(ntok16 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-            bool ok = true;
-            for (int i = 0; i < iters && ok; ++i) {
-                const int s = i % TC_STAGES;
-                if (!mbar_wait(&full[s], (i / TC_STAGES) & 1)) {
-                    atomicCAS(status, 0, (2 << 8) | 1);
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t adesc = umma_desc_sw128(smem_u32(a_stage + s * A_STAGE_BYTES));
-                const uint64_t bdesc = umma_desc_sw128(smem_u32(b_stage + s * B_STAGE_BYTES));
-#pragma unroll
-                for (int kk = 0; kk < TC_BK / 16; ++kk)     // 32 bytes further per K = 16 step
-                    umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(&empty[s]);                      // stage free once these MMAs have read it
+        // instruction descriptor: D float32, A and B bfloat16, both K-major
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                               ((uint32_t)(ntok16 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        const uint64_t a_desc = umma_desc_sw128(smem_u32(a_stage)), b_desc = umma_desc_sw128(smem_u32(b_stage));
+        int s = 0;
+        uint32_t phase = 0;
+        for (int i = 0; i < iters; ++i) {
+            if (!mbar_wait(&full[s], phase)) {
+                atomicCAS(status, 0, (2 << 8) | 1);
+                break;
             }
-            if (ok) umma_commit(accum);                      // accumulator complete
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t adesc = a_desc + (uint64_t)(s * (A_STAGE_BYTES >> 4));
+            const uint64_t bdesc = b_desc + (uint64_t)(s * (B_STAGE_BYTES >> 4));
+            if (slb_elected()) {
+#pragma unroll
+                for (int kk = 0; kk < TC_BK / 16; ++kk)       // 32 bytes further per K = 16 step
+                    umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);                        // stage free once these MMAs have read it
+                if (i + 1 == iters) umma_commit(accum);        // accumulator complete
+            }
+            if (++s == TC_STAGES) {
+                s = 0;
+                phase ^= 1;
+            }
         }
     } else {
         // ------------------------------------------------------------ epilogue
@@ -610,7 +621,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
     float (*pair_vals)[TC_BM] = reinterpret_cast<float (*)[TC_BM]>(b_stage);         // [2][128]: 1 KB
     float* sink = reinterpret_cast<float*>(b_stage) + 2 * TC_BM;                     // [192] behind them
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = slb_warp(), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * TC_BM;
     const int splits = gridDim.y, split = blockIdx.y;
     const int kblocks = (K + TC_BK - 1) / TC_BK;
@@ -656,52 +667,63 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
     if (tracer) slb_trace_event(tr, TRACE_ID, SLB_TR_START);
 
     if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t bytes = A_STAGE_BYTES + (uint32_t)ntok16 * TC_BK * 2;
-            const bool w_first = (flags & SLB_FLAG_EVICT_FIRST) != 0;
-            const uint64_t w_policy = w_first ? l2_evict_first_policy() : 0;
-            const int ahead = min(iters, TC_STAGES);
-            for (int i = 0; i < ahead; ++i) {
+        const uint32_t bytes = A_STAGE_BYTES + (uint32_t)ntok16 * TC_BK * 2;
+        const bool w_first = (flags & SLB_FLAG_EVICT_FIRST) != 0;
+        const uint64_t w_policy = w_first ? l2_evict_first_policy() : 0;
+        const int ahead = min(iters, TC_STAGES);
+        for (int i = 0; i < ahead; ++i)                       // stages are empty at the start
+            if (slb_elected()) {
                 mbar_expect_tx(&full[i], bytes);
                 load_w_tile(a_stage + i * A_STAGE_BYTES, &map_w, &full[i], (kb_begin + i) * TC_BK, n0, w_first, w_policy);
             }
-            pdl_wait();
-            for (int i = 0; i < ahead; ++i)
+        pdl_wait();
+        for (int i = 0; i < ahead; ++i)
+            if (slb_elected())
                 tma_load_2d(b_stage + i * B_STAGE_BYTES, &map_x, &full[i], (kb_begin + i) * TC_BK, tok_base);
-            for (int i = ahead; i < iters; ++i) {
-                const int s = i % TC_STAGES;
-                if (!mbar_wait(&empty[s], ((i / TC_STAGES) & 1) ^ 1)) {
-                    atomicCAS(status, 0, (1 << 8) | 2);
-                    break;
-                }
+        int s = 0;
+        uint32_t phase = 0;
+        for (int i = ahead; i < iters; ++i) {
+            if (!mbar_wait(&empty[s], phase)) {
+                atomicCAS(status, 0, (1 << 8) | 2);
+                break;
+            }
+            const int k = (kb_begin + i) * TC_BK;
+            if (slb_elected()) {
                 mbar_expect_tx(&full[s], bytes);
-                const int k = (kb_begin + i) * TC_BK;
                 load_w_tile(a_stage + s * A_STAGE_BYTES, &map_w, &full[s], k, n0, w_first, w_policy);
                 tma_load_2d(b_stage + s * B_STAGE_BYTES, &map_x, &full[s], k, tok_base);
+            }
+            if (++s == TC_STAGES) {
+                s = 0;
+                phase ^= 1;
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                   ((uint32_t)(ntok16 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-            bool ok = true;
-            for (int i = 0; i < iters && ok; ++i) {
-                const int s = i % TC_STAGES;
-                if (!mbar_wait(&full[s], (i / TC_STAGES) & 1)) {
-                    atomicCAS(status, 0, (2 << 8) | 2);
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t adesc = umma_desc_sw128(smem_u32(a_stage + s * A_STAGE_BYTES));
-                const uint64_t bdesc = umma_desc_sw128(smem_u32(b_stage + s * B_STAGE_BYTES));
-#pragma unroll
-                for (int kk = 0; kk < TC_BK / 16; ++kk)
-                    umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(&empty[s]);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                               ((uint32_t)(ntok16 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        const uint64_t a_desc = umma_desc_sw128(smem_u32(a_stage)), b_desc = umma_desc_sw128(smem_u32(b_stage));
+        int s = 0;
+        uint32_t phase = 0;
+        for (int i = 0; i < iters; ++i) {
+            if (!mbar_wait(&full[s], phase)) {
+                atomicCAS(status, 0, (2 << 8) | 2);
+                break;
             }
-            if (ok) umma_commit(accum);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t adesc = a_desc + (uint64_t)(s * (A_STAGE_BYTES >> 4));
+            const uint64_t bdesc = b_desc + (uint64_t)(s * (B_STAGE_BYTES >> 4));
+            if (slb_elected()) {
+#pragma unroll
+                for (int kk = 0; kk < TC_BK / 16; ++kk)       // 32 bytes further per K = 16 step
+                    umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);                        // stage free once these MMAs have read it
+                if (i + 1 == iters) umma_commit(accum);        // accumulator complete
+            }
+            if (++s == TC_STAGES) {
+                s = 0;
+                phase ^= 1;
+            }
         }
         __syncwarp();
     } else {
