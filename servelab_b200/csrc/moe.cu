@@ -906,7 +906,7 @@ int slb_moe_combine_bf16(const float* y, int ldy, const float* weights, const bf
                          bf16* out, int ldo, int T, int top, int N, cudaStream_t st) {
     return launch_moe_combine<bf16, float>(y, ldy, weights, shared, lds, out, ldo, T, top, N, st);
 }
-// the experts' rows in bfloat16, sorted by expert (a library product left them so); the plan says where a
+// the experts' rows in bfloat16, sorted by expert (as a product over sorted rows leaves them); the plan says where a
 // pair's row is
 int slb_moe_combine_bf16_sorted(const bf16* y, int ldy, const float* weights, const bf16* shared, int lds,
                                 bf16* out, int ldo, const int* plan, int E, int T, int top, int N, cudaStream_t st) {
@@ -914,6 +914,14 @@ int slb_moe_combine_bf16_sorted(const bf16* y, int ldy, const float* weights, co
     const int P = T * top;
     return launch_moe_combine<bf16, bf16>(y, ldy, weights, shared, lds, out, ldo, T, top, N, st,
                                           plan + 3 * E + 1 + 2 * moe_num_tiles(P, E) + P);
+}
+// ... in float32
+int slb_moe_combine_bf16_sorted_f32(const float* y, int ldy, const float* weights, const bf16* shared, int lds,
+                                    bf16* out, int ldo, const int* plan, int E, int T, int top, int N, cudaStream_t st) {
+    if (E <= 0 || plan == nullptr) return SLB_ERR_BAD_ARG;
+    const int P = T * top;
+    return launch_moe_combine<bf16, float>(y, ldy, weights, shared, lds, out, ldo, T, top, N, st,
+                                           plan + 3 * E + 1 + 2 * moe_num_tiles(P, E) + P);
 }
 // out[i] = the input row of the i-th pair of the plan's list; rows of whole 16-byte pieces
 int slb_moe_gather_bf16(const bf16* x, int ldx, const int* plan, int E, int P, int top, int K, bf16* out, int ldo,

@@ -881,6 +881,53 @@ def gemm_tc_resid_dyt(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, pos
     return z
 
 
+# ------------------------------------ tcgen05 products of a feed-forward over many tokens
+def gemm_rows_gated_takes(x: torch.Tensor, w: torch.Tensor, block: int) -> bool:
+    """The product with the gated activation in its epilogue: bfloat16 rows of whole 16-byte pieces, gates then ups
+    (``block`` 0, a multiple of 16 of each) or alternating in runs of 64."""
+    inter = w.shape[0] // 2
+    return (x.dtype == _BF16 and w.dtype == _BF16 and x.shape[0] > 0 and w.stride(1) == 1 and x.stride(1) == 1
+            and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0 and block in (0, SWIGLU_BLOCK) and inter % (block or 16) == 0)
+
+
+def gemm_rows_gated_pays(m: int, inter: int, k: int) -> bool:
+    """Whether that product is ahead of the library's and the activation's kernel.  A pair of SMs has 128 features, so
+    matrices with few of them leave SMs idle (1,024 x 512, us at 200 / 512 / 1,000 / 2,048 tokens: library 5.9 / 6.2 / 7.0 /
+    9.0, own 5.9 / 6.7 / 7.2 / 8.2; 512 x 1,536 5.9 / 6.8 / 8.8 / 13.6, own 5.3 / 6.5 / 7.9 / 11.1).  Up to 128 tokens both
+    wait for the weights, and the library's tiles are full at 64 and 128 (2,048 x 2,816 at 33 / 64 / 100 / 128 tokens 9.3 /
+    7.6 / 9.8 / 7.8, own 8.7 / 8.8 / 9.3 / 9.2; 896 x 4,864 8.9 / 9.9 / 8.1 / 7.0, own 7.5 / 8.4 / 7.0 / 7.2), and many
+    features must fill whole rounds of the SMs (148 pairs' tiles of 3,584 x 18,944 at 65 / 128 tokens 52 / 56, own 45 / 45;
+    108 of 5,120 x 13,824 52 / 60, own 56 / 57)."""
+    tiles, pairs = -(-inter // 128), _num_sms() // 2
+    if m <= 16:                                                # (the weight-streaming products' steps)
+        return False
+    if m > 128:
+        return tiles >= 8 or m >= 1500
+    if tiles > pairs:
+        return 10 * tiles >= 9 * pairs * -(-tiles // pairs)
+    if 48 < m <= 64 or m > 112:
+        return k <= 1024 and m <= 64 and tiles >= 8
+    return tiles >= 8
+
+
+def gemm_rows_gated(x: torch.Tensor, w: torch.Tensor, block: int, activation: str = "silu",
+                    limit: Optional[float] = None, alpha: float = 1.0, tile_tokens: int = 0) -> torch.Tensor:
+    """act(x Wg^T) * (x Wu^T) for any number of tokens, one launch (see ``gemm_rows_gated_takes``)."""
+    M, Kd = x.shape
+    inter = w.shape[0] // 2
+    out = torch.empty((M, inter), dtype=_BF16, device=x.device)
+    L.check(L.core().slb_gemm_rows_gated_bf16(
+        x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, inter, Kd, int(block),
+        GATED_ACTIVATIONS[activation], float(limit or 0.0), float(alpha), int(tile_tokens), _stream()), "gemm_rows_gated")
+    return out
+
+
+def gemm_rows_status(reset: bool = False) -> int:
+    """0 while no wait of the products over many tokens has given up (synchronises)."""
+    return L.core().slb_gemm_rows_status(1 if reset else 0)
+
+
 def gemm_tc_status(reset: bool = False) -> int:
     """0 unless a bounded wait inside the tcgen05 kernels ran out, or the q|k|v epilogue met a
     block-table entry outside the cache (synchronises)."""
@@ -1252,6 +1299,30 @@ moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this ma
 moe_tensor_cores = True        # bfloat16: the experts' products on mma.sync (off: CUDA cores, the twin)
 
 
+def _gather_rows(x: torch.Tensor, plan: torch.Tensor, E: int, P: int, top: int) -> torch.Tensor:
+    """The rows of ``x`` in the order of the plan's list of pairs [P, h]."""
+    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+        x = x.clone(memory_format=torch.contiguous_format)
+    xs = torch.empty((P, x.shape[1]), dtype=x.dtype, device=x.device)
+    L.check(L.core().slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, x.shape[1],
+                                         xs.data_ptr(), xs.stride(0), _stream()), "moe_gather")
+    return xs
+
+
+moe_tcgen05 = True             # bfloat16: the experts' products on tcgen05 (off: the vendor's or mma.sync)
+moe_tcgen05_max_experts = 1024
+
+
+def moe_tcgen05_pays(pairs: int, experts: int, elements: int) -> bool:
+    """Whether they are ahead of the others (``elements``: of one matrix of an expert).  Always for large experts; for
+    others from some rows an expert on, since a list of rows and one launch more come with them.  us, others / tcgen05:
+    32 of 2,048 x 1,408, 4 a token, 1 / 16 / 64 / 250 / 2,048 tokens 39 / 97 / 111 / 173 / 210, 29 / 99 / 103 / 109 / 179; 128
+    of 2,048 x 768, 8 a token, 2 / 4 / 8 / 64 / 512 tokens 47 / 65 / 107 / 236 / 348, 49 / 68 / 91 / 201 / 226; 64 of 1,024 x
+    512, 8 a token, 16 / 64 / 128 / 2,048 tokens 45 / 50 / 72 / 302, 52 / 54 / 55 / 119; 8 of 512 x 256, 2 a token, 32 / 64 /
+    512 tokens 17 / 20 / 32, 19 / 19 / 25."""
+    return elements >= 1 << 21 or pairs >= 16 * experts or (elements >= 1 << 20 and pairs >= 64)
+
+
 def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor,
                 w_down: torch.Tensor, shared: Optional[torch.Tensor], activation: str = "silu",
                 limit: Optional[float] = None, alpha: float = 1.0, weight_inputs: bool = False) -> torch.Tensor:
@@ -1273,9 +1344,35 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     # bfloat16 with rows of whole 16-byte chunks: the tensor-core products; else CUDA cores
     mma = (x.dtype == _BF16 and moe_tensor_cores and h % 8 == 0 and inter % 8 == 0 and n_out % 2 == 0
            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
-    form = "" if vendor or mma else "_simt"                # (the tiles' rows differ)
+    own = (x.dtype == _BF16 and moe_tcgen05 and moe_tensor_cores and 0 < P and E <= moe_tcgen05_max_experts and h % 8 == 0
+           and inter % 16 == 0 and n_out % 4 == 0 and moe_tcgen05_pays(P, E, h * inter)
+           and all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (w_gate_up, w_down)))
+    form = "" if own or vendor or mma else "_simt"         # (the tiles' rows differ)
     plan = torch.empty(getattr(lib, f"slb_moe_plan{form}_ints")(P, E), dtype=torch.int32, device=x.device)
     L.check(getattr(lib, "slb_moe_plan" + form)(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
+    if own:
+        # Rows sorted by expert, each expert's in tiles of up to 256; a token's results are summed where the second
+        # product left them: in float32, in the steps of many rows of large experts in bfloat16 (their way through
+        # memory is what they cost: 67 MB for 8,192 rows of 2,048).
+        at = plan.numel() - 2 * P
+        order = plan[at:at + P]
+        xs = _gather_rows(x, plan, E, P, top)
+        act = torch.empty((P, inter), dtype=x.dtype, device=x.device)
+        offsets = plan.data_ptr() + 4 * E
+        L.check(lib.slb_gemm_rows_experts_bf16(
+            xs.data_ptr(), h, w_gate_up.data_ptr(), h, act.data_ptr(), inter, offsets, E, P, inter, h, 1, 0, *act_args,
+            _p(weights if weight_inputs else None), order.data_ptr() if weight_inputs else None, _stream()),
+            "gemm_rows_experts")
+        half = P >= moe_vendor_min_pairs and h * inter >= moe_vendor_min_expert_elements
+        ys = torch.empty((P, n_out), dtype=_BF16 if half else _F32, device=x.device)
+        L.check(lib.slb_gemm_rows_experts_bf16(
+            act.data_ptr(), inter, w_down.data_ptr(), inter, ys.data_ptr(), n_out, offsets, E, P, n_out, inter, 0,
+            0 if half else 1, 0, 0.0, 0.0, None, None, _stream()), "gemm_rows_experts")
+        out = torch.empty((T, n_out), dtype=x.dtype, device=x.device)
+        combine = lib.slb_moe_combine_bf16_sorted if half else lib.slb_moe_combine_bf16_sorted_f32
+        L.check(combine(ys.data_ptr(), n_out, _p(out_weights), _p(shared), shared.stride(0) if shared is not None else 0,
+                        out.data_ptr(), out.stride(0), plan.data_ptr(), E, T, top, n_out, _stream()), "moe_combine")
+        return out
     if vendor:
         # Large steps: the vendor's grouped product over the rows sorted by expert (the plan's list
         # and offsets stay on the device), as the dense products of large steps go to the vendor's
@@ -1284,11 +1381,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         at = plan.numel() - 2 * P
         ends = plan[E + 1:2 * E + 1]                                   # cumulative row counts
         order = plan[at:at + P]                                        # pairs sorted by expert
-        if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
-            x = x.clone(memory_format=torch.contiguous_format)
-        xs = torch.empty((P, h), dtype=x.dtype, device=x.device)
-        L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, h, xs.data_ptr(),
-                                        xs.stride(0), _stream()), "moe_gather")
+        xs = _gather_rows(x, plan, E, P, top)
         gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
         mark("library grouped gemm")
         act = torch.empty((P, inter), dtype=x.dtype, device=x.device)

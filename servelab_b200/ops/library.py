@@ -60,6 +60,9 @@ _CORE_SIGNATURES = {
     "slb_add_rmsnorm_parts_bf16": [P, P, I, LL, P, P, P, P, I, I, F, P],
     "slb_qkv_rope_cache_parts_bf16": [P, I, LL, I, P, P, P, P, I, I, I, P, I, P, I, P, P, I, I, I, I, P],
     "slb_gemm_tc_status": [I],
+    "slb_gemm_rows_gated_bf16": [P, I, P, I, P, I, I, I, I, I, I, F, F, I, P],
+    "slb_gemm_rows_experts_bf16": [P, I, P, I, P, I, P, I, I, I, I, I, I, I, F, F, P, P, P],
+    "slb_gemm_rows_status": [I],
     "slb_ln_add_norm_f32": [P, I, P, I, P, P, F, P, P, F, P, I, P, I, I, P],
     "slb_ln_add_norm_bf16": [P, I, P, I, P, P, F, P, P, F, P, I, P, I, I, P],
     "slb_head_prep_f32": [P, I, P],
@@ -155,6 +158,7 @@ _CORE_SIGNATURES = {
     "slb_moe_combine_f32": [P, I, P, P, I, P, I, I, I, I, P],
     "slb_moe_combine_bf16": [P, I, P, P, I, P, I, I, I, I, P],
     "slb_moe_combine_bf16_sorted": [P, I, P, P, I, P, I, P, I, I, I, I, P],
+    "slb_moe_combine_bf16_sorted_f32": [P, I, P, P, I, P, I, P, I, I, I, I, P],
     "slb_moe_gather_bf16": [P, I, P, I, I, I, I, P, I, P],
     "slb_router_logits_tile_bf16": [P, I, P, I, P, I, I, I, I, P],
 }

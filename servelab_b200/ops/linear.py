@@ -31,6 +31,8 @@ tc_wide_max_tokens = 64    # ... and up to this many for products wide enough to
 # ms a step without, 3.28 / 3.10 with "rope", 3.22 / 3.04 with both).
 defer_split_sums = {"rope": True, "norm": True}
 fuse_swiglu = True         # the gate|up product of a decode step applies the activation itself
+fuse_gated = True          # ... and so does that of every other step (gemm_rows.cu; off: the library's product, then the
+                           # activation's kernel)
 # The product that closes a residual branch (o, down) of a decode step also does the add and
 # the RMS norm that follow it: its epilogue updates the float32 stream and writes the normed
 # rows without their factor 1 / rms, which the next product (q|k|v, gate|up) applies in its own
@@ -139,6 +141,9 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, block: int, activatio
         # (K splits: the activation in the cluster's epilogue; 8 layers of the 0.5B shape: 215 us a step with the
         # activation's own launch)
         return K.gemm_tc_cluster(x, w_gate_up, swiglu=True)
+    if (fuse_gated and K.gemm_rows_gated_takes(xt, w_gate_up, block)
+            and K.gemm_rows_gated_pays(M, inter, w_gate_up.shape[1])):
+        return K.gemm_rows_gated(K.plain_unless(None, x), w_gate_up, block, activation, limit, alpha)
     gu = linear(x, w_gate_up)
     act = torch.empty((M, inter), dtype=x.dtype, device=x.device)
     if activation == "silu":

@@ -521,3 +521,88 @@ def test_split_requests_of_five_tiles_are_no_less_exact(monkeypatch, H, G, D):
             total[splits] += float((out.double() - want).norm() / want.norm())
     assert total[0] <= 1.03 * total[1] and total[1] < 10 * 2.0 ** -7
     assert K().decode_attention_status(D) == 0
+
+
+# ------------------------------------------------------------- products of a feed-forward over many tokens
+def _act64(g, u, act):
+    if act == "gelu_tanh":
+        return torch.nn.functional.gelu(g, approximate="tanh") * u
+    if act == "swish_clamped":
+        g, u = g.clamp(max=1.3), u.clamp(-1.3, 1.3) + 1
+        return g * torch.sigmoid(1.7 * g) * u
+    return g * torch.sigmoid(g) * u
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "swish_clamped"])
+@pytest.mark.parametrize("T,I,Kd,block,nt", [(1, 64, 8, 64, 0), (33, 64, 64, 64, 32), (257, 192, 200, 64, 96), (300, 112, 72, 0, 256),
+                                             (700, 16, 128, 0, 160), (2048, 4864, 896, 64, 0), (480, 1408, 2048, 0, 0)])
+def test_gated_product_of_many_tokens(T, I, Kd, block, nt, act):
+    """Against 64 bits, in tiles that do not divide tokens, features or K: the result is rounded once (2^-9 relative), and
+    float32 sums of K products and a hardware exponential and reciprocal before it change it by less than a quarter of
+    that: 2.5e-3 of the norm."""
+    g = gen(T + I)
+    x = torch.randn(T, Kd, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(2 * I, Kd, device=DEV, generator=g) * Kd ** -0.5).bfloat16()
+    assert K().gemm_rows_gated_takes(x, w, block)
+    got = K().gemm_rows_gated(x, w, block, act, 1.3, 1.7, tile_tokens=nt).double()
+    y = x.double() @ w.double().T
+    gu = y.view(T, I // 64, 2, 64).transpose(1, 2).reshape(T, 2, I) if block else y.view(T, 2, I)
+    want = _act64(gu[:, 0], gu[:, 1], act)
+    assert (got - want).norm() <= 2.5e-3 * want.norm() and K().gemm_rows_status() == 0
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 300, 33], [256, 257, 0, 17, 513, 1, 2, 31], [700, 2400, 5], [0, 0, 1]])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_experts_products_over_sorted_rows(counts, weighted):
+    """Experts without rows, with one, with whole tiles and one more; both results of the second product; rows of no
+    expert stay as they are.  Bound as above (float32 rows: 2^-20 for sums of 112 products)."""
+    from servelab_b200.ops import library as L
+    g, E, h, I = gen(sum(counts)), len(counts), 72, 112
+    P = sum(counts) + 5
+    offs = torch.tensor([0] + counts, device=DEV).cumsum(0).int()
+    x = torch.randn(P, h, device=DEV, generator=g).bfloat16()
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    order, rw = torch.randperm(P, device=DEV, generator=g).int(), torch.rand(P, device=DEV, generator=g)
+    act = torch.full((P, I), float("nan"), device=DEV, dtype=torch.bfloat16)
+    lib, st = L.core(), K()._stream()
+    L.check(lib.slb_gemm_rows_experts_bf16(x.data_ptr(), h, wg.data_ptr(), h, act.data_ptr(), I, offs.data_ptr(), E, P, I, h, 1,
+                                           0, 0, 0.0, 0.0, rw.data_ptr() if weighted else None,
+                                           order.data_ptr() if weighted else None, st), "experts")
+    at = 0
+    for e, n in enumerate(counts):
+        y = x[at:at + n].double() @ wg[e].double().T * (rw[order[at:at + n].long()].double()[:, None] if weighted else 1.0)
+        want = _act64(y[:, :I], y[:, I:], "silu")
+        assert (act[at:at + n].double() - want).norm() <= 2.5e-3 * want.norm()
+        at += n
+    assert act[at:].isnan().all()
+    act[at:] = 0
+    for dtype, bound in ((torch.bfloat16, 2.5e-3), (torch.float32, 1e-6)):
+        out = torch.full((P, h), float("nan"), device=DEV, dtype=dtype)
+        L.check(lib.slb_gemm_rows_experts_bf16(act.data_ptr(), I, wd.data_ptr(), I, out.data_ptr(), h, offs.data_ptr(), E, P, h,
+                                               I, 0, int(dtype == torch.float32), 0, 0.0, 0.0, None, None, st), "experts")
+        at = 0
+        for e, n in enumerate(counts):
+            want = act[at:at + n].double() @ wd[e].double().T
+            assert (out[at:at + n].double() - want).norm() <= bound * want.norm()
+            at += n
+        assert out[at:].isnan().all()
+    assert K().gemm_rows_status() == 0
+
+
+@pytest.mark.parametrize("T,E,top,h,I,half", [(70, 8, 4, 256, 64, False), (300, 8, 4, 1024, 2048, True), (3, 4, 2, 2048, 1024, False)])
+def test_routed_experts_on_sorted_rows(T, E, top, h, I, half):
+    """The whole sum, rows read from a wider matrix, with shared rows: against 64 bits with the activation and the result
+    rounded (and an expert's rows, in large steps): 6e-3 of the norm."""
+    g = gen(T)
+    x = torch.randn(T, h + 8, device=DEV, generator=g).bfloat16()[:, 8:]
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    w, shared = torch.rand(T, top, device=DEV, generator=g), torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    assert K().moe_tcgen05_pays(T * top, E, h * I) and half == (T * top >= K().moe_vendor_min_pairs)
+    got = K().moe_experts(x, ids, w, wg, wd, shared).double()
+    want = shared.double()
+    for e in range(E):
+        t, k = torch.where(ids == e)
+        y = x[t].double() @ wg[e].double().T
+        want = want.index_add(0, t, w[t, k].double()[:, None] * (_act64(y[:, :I], y[:, I:], "silu") @ wd[e].double().T))
+    assert (got - want).norm() <= 6e-3 * want.norm()
