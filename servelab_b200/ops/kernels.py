@@ -1318,9 +1318,10 @@ def moe_tcgen05_pays(pairs: int, experts: int, elements: int) -> bool:
     others from some rows an expert on, since a list of rows and one launch more come with them.  us, others / tcgen05:
     32 of 2,048 x 1,408, 4 a token, 1 / 16 / 64 / 250 / 2,048 tokens 39 / 97 / 111 / 173 / 210, 29 / 99 / 103 / 109 / 179; 128
     of 2,048 x 768, 8 a token, 2 / 4 / 8 / 64 / 512 tokens 47 / 65 / 107 / 236 / 348, 49 / 68 / 91 / 201 / 226; 64 of 1,024 x
-    512, 8 a token, 16 / 64 / 128 / 2,048 tokens 45 / 50 / 72 / 302, 52 / 54 / 55 / 119; 8 of 512 x 256, 2 a token, 32 / 64 /
-    512 tokens 17 / 20 / 32, 19 / 19 / 25."""
-    return elements >= 1 << 21 or pairs >= 16 * experts or (elements >= 1 << 20 and pairs >= 64)
+    512, 8 a token, 16 / 64 / 128 / 2,048 tokens 45 / 50 / 72 / 302, 52 / 54 / 55 / 119.  Experts smaller than that stay with
+    one kernel for steps of any size (8 of 512 x 256, 2 a token, 64 / 512 tokens 20 / 32, 19 / 25): its sums are the same
+    whatever the step, and in so small a model a router's choice hangs on them."""
+    return elements >= 1 << 21 or elements >= 1 << 19 and (pairs >= 16 * experts or elements >= 1 << 20 and pairs >= 64)
 
 
 def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor,

@@ -589,7 +589,7 @@ def test_experts_products_over_sorted_rows(counts, weighted):
     assert K().gemm_rows_status() == 0
 
 
-@pytest.mark.parametrize("T,E,top,h,I,half", [(70, 8, 4, 256, 64, False), (300, 8, 4, 1024, 2048, True), (3, 4, 2, 2048, 1024, False)])
+@pytest.mark.parametrize("T,E,top,h,I,half", [(70, 8, 4, 1024, 512, False), (300, 8, 4, 1024, 2048, True), (3, 4, 2, 2048, 1024, False)])
 def test_routed_experts_on_sorted_rows(T, E, top, h, I, half):
     """The whole sum, rows read from a wider matrix, with shared rows: against 64 bits with the activation and the result
     rounded (and an expert's rows, in large steps): 6e-3 of the norm."""
