@@ -26,7 +26,7 @@
 // the block then frees its tensor memory and returns without a result.
 #include <cuda.h>
 
-#include "common.cuh"
+#include "softmax_util.cuh"
 #include "tma_util.cuh"
 
 #if (SLB_KEY_DIM % 64 == 0 && SLB_VALUE_DIM % 64 == 0 && SLB_VALUE_DIM <= 256 && SLB_KEY_DIM <= 448)
@@ -46,10 +46,17 @@ constexpr int K_TILE_BYTES = PANELS_K * KV_PANEL_BYTES;
 constexpr int V_TILE_BYTES = PANELS_V * KV_PANEL_BYTES;
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
-constexpr int OFF_V = OFF_K + 2 * K_TILE_BYTES;            // (tied values: no value ring, the barriers sit here)
-__host__ __device__ constexpr int off_bar(bool tied) { return tied ? OFF_V : OFF_V + 2 * V_TILE_BYTES; }
-__host__ __device__ constexpr size_t attn_smem(bool tied) { return (size_t)off_bar(tied) + 128; }
 constexpr size_t SMEM_LIMIT = 227 * 1024;
+constexpr int OFF_V = OFF_K + 2 * K_TILE_BYTES;
+// Key tiles on their way.  Tied, a tile is given back when its P.V has run, one softmax later than otherwise, and with
+// two the next copy began when its tile was already wanted (keys of 320: 3,700 cycles a tile, 2,500 of them this wait);
+// where tensor memory allows one block an SM there is room for more.
+constexpr int TIED_FIT = (int)((SMEM_LIMIT - 256 - OFF_K) / K_TILE_BYTES);
+constexpr int TIED_STAGES = TMEM_COLS < 512 || TIED_FIT < 3 ? 2 : TIED_FIT < 4 ? 3 : 4;
+__host__ __device__ constexpr int off_bar(bool tied) {
+    return tied ? OFF_K + TIED_STAGES * K_TILE_BYTES : OFF_V + 2 * V_TILE_BYTES;
+}
+__host__ __device__ constexpr size_t attn_smem(bool tied) { return (size_t)off_bar(tied) + 256; }
 constexpr uint32_t SPIN_LIMIT = 1u << 18;     // a poll that suspends takes about 4 us: about a second
 constexpr float RESCALE_THRESHOLD = 8.f;       // log2 of the largest probability tolerated
 
@@ -155,6 +162,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
 }
+// the 64 scores of this thread's row
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&s)[64]) {
+    uint32_t v[2][32];
+    tmem_ld32(taddr, v[0]);
+    tmem_ld32(taddr + 32, v[1]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 64; ++i) s[i] = __uint_as_float(v[i >> 5][i & 31]);
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -166,20 +182,36 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
           "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
-// 2^x in one MUFU instruction (exp2f adds a range fix-up around it; the probabilities
-// here are rounded to bfloat16 anyway, and -inf gives 0)
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+using slb_softmax::fast_exp2;
+using slb_softmax::pack2;
+
+// The cap on the scores, cap_back tanh(s / cap_back): tanh(x) = 1 - 2 / (e^(2x) + 1) ...
+__device__ __forceinline__ void cap_scores(float (&s)[64], float cap_in, float cap_back) {
+#pragma unroll
+    for (int i = 0; i < 64; ++i) s[i] = cap_back * (1.0f - __fdividef(2.0f, fast_exp2(s[i] * cap_in) + 1.0f));
 }
-__device__ __forceinline__ unsigned pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<unsigned*>(&v);
+// ... or its series, s + s (x^2 (-1/3 + x^2 (2/15 + ...))), two scores an instruction
+__device__ __forceinline__ void cap_small_scores(float (&s)[64], float to_x) {
+    using namespace slb_softmax;
+    const uint64_t k = pair_bits(to_x, to_x);
+    const uint64_t c1 = pair_bits(-1.f / 3.f, -1.f / 3.f), c2 = pair_bits(2.f / 15.f, 2.f / 15.f);
+    const uint64_t c3 = pair_bits(-17.f / 315.f, -17.f / 315.f), c4 = pair_bits(62.f / 2835.f, 62.f / 2835.f);
+    const uint64_t c5 = pair_bits(-1382.f / 155925.f, -1382.f / 155925.f);
+#pragma unroll
+    for (int i = 0; i < 64; i += 2) {
+        const uint64_t v = pair_bits(s[i], s[i + 1]), x = mul2(v, k), u = mul2(x, x);
+        uint64_t q = fma2(c5, u, c4);
+        q = fma2(q, u, c3);
+        q = fma2(q, u, c2);
+        q = fma2(q, u, c1);
+        const float2 r = pair_of(fma2(mul2(v, u), q, v));
+        s[i] = r.x;
+        s[i + 1] = r.y;
+    }
 }
 
 __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_kv_tc_kernel(
-    const bf16* __restrict__ q, int ldq, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, int ldo,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_q,
     const int* __restrict__ ctx_len, const int* __restrict__ tile_seq, const int* __restrict__ tile_row0,
@@ -192,15 +224,19 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
     // (which multiplies by scale log2 e) sees the capped score; tanh(x) = 1 - 2 / (e^(2x) + 1).
     // sink: one number a head whose exponential joins the softmax's denominator when a row is finished.
     extern __shared__ __align__(1024) unsigned char smem[];
-    // All barriers come in pairs indexed by tile parity.  s_full[b]: Q.K^T of a tile is done
-    // (its scores are ready and its keys may be replaced); pv_done[b]: its P.V is done (its
-    // values may be replaced, the accumulator may be rescaled or read).
-    uint64_t* k_full = reinterpret_cast<uint64_t*>(smem + off_bar(tied != 0));     // [2]
-    uint64_t* v_full = k_full + 2;                                      // [2]
+    // Barriers of scores, weights, values and results come in pairs indexed by tile parity, those of the keys by their
+    // stage.  s_full[b]: Q.K^T of a tile is done (its scores are ready and, not tied, its keys may be replaced);
+    // pv_done[b]: its P.V is done (its values may be replaced, the accumulator may be rescaled or read); k_free[s]: the
+    // same of a tied tile (the loader may be a tile behind: pv_done could have moved on by two).
+    uint64_t* k_full = reinterpret_cast<uint64_t*>(smem + off_bar(tied != 0));     // [4]
+    uint64_t* k_free = k_full + 4;                                      // [4]
+    uint64_t* v_full = k_free + 4;                                      // [2]
     uint64_t* s_full = v_full + 2;                                      // [2]
     uint64_t* p_full = s_full + 2;                                      // [2], one per score buffer
     uint64_t* pv_done = p_full + 2;                                     // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+    uint64_t* q_full = pv_done + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 1);
+    const int k_stages = tied ? TIED_STAGES : 2;
 
     pdl_wait();
     const int warp = slb_warp(), lane = threadIdx.x & 31;
@@ -238,8 +274,12 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
     const int ntiles = (kend - kbeg + BN - 1) / BN;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             mbar_init(&k_full[i], 1);
+            mbar_init(&k_free[i], 1);
+        }
+        mbar_init(q_full, 1);
+        for (int i = 0; i < 2; ++i) {
             mbar_init(&v_full[i], 1);
             mbar_init(&pv_done[i], 1);
         }
@@ -252,29 +292,6 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
                      ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // K/V stages start as zeros so that rows no copy fills (absent pages) hold finite values
-    for (int i = threadIdx.x; i < (off_bar(tied != 0) - OFF_K) / 16; i += THREADS)
-        reinterpret_cast<uint4*>(smem + OFF_K)[i] = make_uint4(0, 0, 0, 0);
-    // Q tile: the softmax threads copy their rows into the swizzled operand layout
-    if (warp >= 2 && warp < 6) {
-        const int r = (warp & 3) * 32 + lane;
-        unsigned char* qs = smem + OFF_Q;
-        if (r < nrows) {
-            const int tl = r / g, hg = r - tl * g;
-            const bf16* src = q + (size_t)(q0 + tok0 + tl) * ldq + (size_t)((kvh * g + hg) * maps + amap) * DK;
-#pragma unroll
-            for (int c = 0; c < DK / 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src + c * 8);
-                *reinterpret_cast<uint4*>(qs + (c >> 3) * (BM * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < DK / 8; ++c)
-                *reinterpret_cast<uint4*>(qs + (c >> 3) * (BM * 128) + r * 128 + ((c & 7) << 4)) =
-                    make_uint4(0, 0, 0, 0);
-        }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -284,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
         // (tied values: the key tiles are the value tiles, nothing to fetch)
     } else if (warp == 0 || warp == 6) {
         // ---------------------------------------------------------------- loaders
-        // Warp 0 fetches the keys, warp 6 the values, each through its own two-stage ring:
+        // Warp 0 fetches the keys, warp 6 the values, each through its own ring:
         // the keys of a tile may be replaced when its Q.K^T has run (two softmax periods
         // before the new ones are needed), the values when its P.V has.  Lane b looks up the
         // page of box b, one tile ahead of its use (a dependent global load).
@@ -292,7 +309,8 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
         const CUtensorMap* map = keys ? &map_k : &map_v;
         unsigned char* ring = smem + (keys ? OFF_K : OFF_V);
         uint64_t* full = keys ? k_full : v_full;
-        uint64_t* freed = (keys && !tied) ? s_full : pv_done;   // (tied: a key stage also feeds P.V)
+        uint64_t* freed = !keys ? pv_done : tied ? k_free : s_full;      // (tied: a key stage also feeds P.V)
+        const int stages = keys ? k_stages : 2;
         const int panels = keys ? PANELS_K : PANELS_V;
         const int tile_bytes = keys ? K_TILE_BYTES : V_TILE_BYTES;
         const int boxes = BN / box_rows;
@@ -308,15 +326,30 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
             }
             return row;
         };
-        int row = lookup(0);
+        if (keys && slb_elected()) {                         // the queries: whole tokens, a panel a copy (rows beyond the
+            mbar_expect_tx(q_full, PANELS_K * (BM / g) * g * 128);             // tile's are computed and not stored)
+            for (int p = 0; p < PANELS_K; ++p)
+                slb_tma::tma_load_3d(smem + OFF_Q + p * (BM * 128), &map_q, q_full, amap * DK + p * 64, kvh * g, q0 + tok0);
+        }
+        int row = lookup(0), st = 0;
+        uint32_t phase = 1;
         for (int j = 0; j < ntiles; ++j) {
-            const int st = j & 1;
             const int next_row = lookup(j + 1);
-            if (!mbar_wait(&freed[st], ((j >> 1) & 1) ^ 1)) {
+            if (!mbar_wait(&freed[st], phase)) {
                 if (lane == 0) gave_up(status, keys ? 0x101 : 0x102, 0, j, ntiles);
                 break;
             }
             const unsigned got = __ballot_sync(0xffffffffu, row >= 0);
+            if (got != (1u << boxes) - 1u) {               // rows that no copy brings (absent pages) hold zeros
+                for (int b = 0; b < boxes; ++b) {
+                    if (got >> b & 1u) continue;
+                    for (int i = lane; i < panels * box_rows * 8; i += 32)
+                        *reinterpret_cast<uint4*>(ring + st * tile_bytes + i / (box_rows * 8) * KV_PANEL_BYTES +
+                                                  b * box_rows * 128 + i % (box_rows * 8) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
             if (slb_elected()) {
                 const uint32_t bytes = (uint32_t)__popc(got) * (uint32_t)box_rows * 128u * (uint32_t)panels;
                 if (bytes) mbar_expect_tx(&full[st], bytes); else mbar_arrive(&full[st]);
@@ -330,6 +363,10 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
                 }
             }
             row = next_row;
+            if (++st == stages) {
+                st = 0;
+                phase ^= 1;
+            }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
@@ -346,37 +383,47 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
         const uint64_t V_STAGE_STEP = (tied ? K_TILE_BYTES : V_TILE_BYTES) >> 4;
         // S = Q.K^T of tile t into score buffer t & 1 (which held the scores and then P of
         // tile t - 2; its P.V has been issued before)
+        int kst = 0, vst = 0;                                 // stages of the next Q.K^T and (tied) P.V
+        uint32_t k_phase = 0;
         auto issue_qk = [&](int t) -> bool {
-            const int st = t & 1;
-            if (!mbar_spin(&k_full[st], (t >> 1) & 1)) { gave_up(status, 0x201, 1, t, ntiles); return false; }
+            const int buf = t & 1;
+            if (!mbar_spin(&k_full[kst], k_phase)) { gave_up(status, 0x201, 1, t, ntiles); return false; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t k_desc = k_desc0 + (uint64_t)kst * STAGE_STEP;
             if (slb_elected()) {
 #pragma unroll
                 for (int p = 0; p < PANELS_K; ++p)
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)          // 16 elements of a key = 32 bytes per step
-                        umma_bf16(tmem + S_COL + 64 * st, q_desc + ((p * (BM * 128) + kk * 32) >> 4),
-                                  k_desc0 + st * STAGE_STEP + ((p * KV_PANEL_BYTES + kk * 32) >> 4), idesc_qk,
-                                  (p > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(&s_full[st]);
+                        umma_bf16(tmem + S_COL + 64 * buf, q_desc + ((p * (BM * 128) + kk * 32) >> 4),
+                                  k_desc + ((p * KV_PANEL_BYTES + kk * 32) >> 4), idesc_qk, (p > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(&s_full[buf]);
+            }
+            if (++kst == k_stages) {
+                kst = 0;
+                k_phase ^= 1;
             }
             return true;
         };
-        bool ok = issue_qk(0);
+        bool ok = mbar_spin(q_full, 0);
+        if (!ok) gave_up(status, 0x204, 1, 0, ntiles);
+        if (ok) ok = issue_qk(0);
         if (ok && ntiles > 1) ok = issue_qk(1);
         for (int j = 0; j < ntiles && ok; ++j) {
             const int st = j & 1;
             if (!mbar_spin(&p_full[st], (j >> 1) & 1)) { gave_up(status, 0x202, 1, j, ntiles); break; }
             if (!tied && !mbar_spin(&v_full[st], (j >> 1) & 1)) { gave_up(status, 0x203, 1, j, ntiles); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t v_desc = v_desc0 + (uint64_t)(tied ? vst : st) * V_STAGE_STEP;
             if (slb_elected()) {
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk)              // 16 keys per step: P 8 columns, V 16 rows
-                    umma_bf16_ts(tmem + O_COL, tmem + S_COL + 64 * st + kk * 8,
-                                 v_desc0 + st * V_STAGE_STEP + ((kk * 16 * 128) >> 4), idesc_pv,
+                    umma_bf16_ts(tmem + O_COL, tmem + S_COL + 64 * st + kk * 8, v_desc + ((kk * 16 * 128) >> 4), idesc_pv,
                                  (j > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&pv_done[st]);
+                if (tied) umma_commit(&k_free[vst]);
             }
+            if (++vst == k_stages) vst = 0;
             // the scores of tile j + 2 go where P of tile j was: issued after P.V of tile j
             // (the tensor core executes in issue order), while the softmax of j + 1 runs
             if (j + 2 < ntiles) ok = issue_qk(j + 2);
@@ -394,85 +441,63 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
         const float bias2 = sig_bias != nullptr && r < nrows ? sig_bias[kvh * g + r % g] * 1.4426950408889634f : 0.f;
         // (raw scores are multiplied by scale * log2 e below: the slope divided by scale)
         const float slope = slopes != nullptr && r < nrows ? slopes[kvh * g + r % g] * inv_scale : 0.f;
+        // a cap on small scores, c tanh(x) with x = s / c: to x^11, relative error 2e-8 up to |x| = 0.35
+        const float to_x = cap_in * 0.34657359027997264f;    // (cap_in is 2 log2(e) scale / c)
+        const bool live = quarter * 32 < nrows;              // (a warp whose rows are all padding only hands tiles on)
         bool ok = true;
         for (int j = 0; j < ntiles && ok; ++j) {
-            if (!mbar_spin(&s_full[j & 1], (j >> 1) & 1)) { if (lane == 0) gave_up(status, 0x301, 2, j, ntiles); ok = false; break; }
+            if (!(live ? mbar_spin(&s_full[j & 1], (j >> 1) & 1) : mbar_wait(&s_full[j & 1], (j >> 1) & 1))) {
+                if (lane == 0) gave_up(status, 0x301, 2, j, ntiles);
+                ok = false;
+                break;
+            }
+            if (!live) {
+                mbar_arrive(&p_full[j & 1]);
+                continue;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t raw[2][32];
-            tmem_ld32(tmem + lane_base + S_COL + 64 * (j & 1), raw[0]);
-            tmem_ld32(tmem + lane_base + S_COL + 64 * (j & 1) + 32, raw[1]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float s[64];
+            tmem_ld64(tmem + lane_base + S_COL + 64 * (j & 1), s);
             if (cap_in > 0.f) {
+                float big = 0.f;
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const float t = fast_exp2(__uint_as_float(raw[h][i]) * cap_in);
-                        raw[h][i] = __float_as_uint(cap_back * (1.0f - __fdividef(2.0f, t + 1.0f)));
-                    }
+                for (int i = 0; i < 64; ++i) big = fmaxf(big, fabsf(s[i]));
+                // (the exponential and the reciprocal of the general form are what four cycles of the multiply-adds' units
+                // cost: 2,000 cycles a tile, this form 900)
+                if (__any_sync(0xffffffffu, !(big * to_x <= 0.35f)))
+                    cap_scores(s, cap_in, cap_back);
+                else
+                    cap_small_scores(s, to_x);
             }
             const int k0 = kbeg + j * BN;
             if (slopes != nullptr) {
                 const float base = slope * (float)(k0 - pos);
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        raw[h][i] = __float_as_uint(fmaf(slope, (float)(h * 32 + i), __uint_as_float(raw[h][i]) + base));
+                for (int i = 0; i < 64; ++i) s[i] = fmaf(slope, (float)i, s[i] + base);
             }
             // raw scores stay unscaled; masked ones become -inf.  A tile that every row of
             // the block sees completely needs no mask (rows of padding compute garbage that
             // is never stored).
             const bool open = k0 + BN - 1 <= p_first && k0 >= all_first;
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, not one
-            if (open) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(raw[h][i]));
-            } else {
-                const int hi = min(BN, min(kend, pos + 1) - k0);      // visible keys: [lo, hi)
-                const int lo = max(0, pos_first - k0);
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int c = h * 32 + i;
-                        if (!(c >= lo && c < hi)) raw[h][i] = __float_as_uint(-INFINITY);
-                        mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(raw[h][i]));
-                    }
-            }
-            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // scale > 0
+            if (!open) slb_softmax::mask_keys(s, pos_first - k0, min(kend, pos + 1) - k0);
             float alpha = 1.f;
-            float sm[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t packed[32];
             if (sig_bias != nullptr) {
                 // sigmoid(x) = 1 / (1 + 2^(-x log2 e)); a masked score (-inf) gives 2^inf and so 0 (as every
                 // divisor above 2^126 does)
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float e0 = fast_exp2(fmaf(__uint_as_float(raw[h][i]), -scale_log2, -bias2));
-                        const float e1 = fast_exp2(fmaf(__uint_as_float(raw[h][i + 1]), -scale_log2, -bias2));
-                        packed[h * 16 + i / 2] = pack2(__fdividef(1.f, 1.f + e0), __fdividef(1.f, 1.f + e1));
-                    }
-            } else {
-            if (mt > m_ref + RESCALE_THRESHOLD || (m_ref == -INFINITY && mt != -INFINITY)) {
-                alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mt);
-                m_ref = mt;
-            }
-            const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float p0 = fast_exp2(fmaf(__uint_as_float(raw[h][i]), scale_log2, -m_use));
-                    const float p1 = fast_exp2(fmaf(__uint_as_float(raw[h][i + 1]), scale_log2, -m_use));
-                    sm[(i >> 1) & 3] += p0 + p1;
-                    packed[h * 16 + i / 2] = pack2(p0, p1);
+                for (int i = 0; i < 64; i += 2) {
+                    const float e0 = fast_exp2(fmaf(s[i], -scale_log2, -bias2));
+                    const float e1 = fast_exp2(fmaf(s[i + 1], -scale_log2, -bias2));
+                    packed[i / 2] = pack2(__fdividef(1.f, 1.f + e0), __fdividef(1.f, 1.f + e1));
                 }
-            l = l * alpha + ((sm[0] + sm[1]) + (sm[2] + sm[3]));
+            } else {
+                const float mt = slb_softmax::max_of(s) * scale_log2;     // scale > 0
+                if (mt > m_ref + RESCALE_THRESHOLD || (m_ref == -INFINITY && mt != -INFINITY)) {
+                    alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mt);
+                    m_ref = mt;
+                }
+                l = l * alpha + slb_softmax::exponentials(s, scale_log2, m_ref == -INFINITY ? 0.f : m_ref, packed);
             }
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
                 // the accumulator is rescaled (rarely): P.V of the previous tile must be done
@@ -556,7 +581,7 @@ int slb_attention_kv_tc_tile_rows(int group) { return group >= 1 && group <= BM 
 
 }  // extern "C"
 
-static int launch_attention_kv_tc(const bf16* q, int ldq, const bf16* kc, const bf16* vc, int tied, bf16* out, int ldo,
+static int launch_attention_kv_tc(const bf16* q, int ldq, int tokens, const bf16* kc, const bf16* vc, int tied, bf16* out, int ldo,
                                   const int* block_table, int max_pages, const int* cu_q, const int* ctx_len,
                                   const int* tile_seq, const int* tile_row0, int num_tiles, int H, int Hkv, int ps,
                                   int num_pages, float scale, int window, const bf16* gate, int ldg, int maps,
@@ -564,6 +589,7 @@ static int launch_attention_kv_tc(const bf16* q, int ldq, const bf16* kc, const 
                                   const float* sink = nullptr, int chunk = 0, const float* sig_bias = nullptr,
                                   const float* slopes = nullptr, float out_scale = 1.f) {
     if (num_tiles <= 0) return 0;
+    if (tokens <= 0) return SLB_ERR_BAD_ARG;
     if (softcap < 0.f || ((sink != nullptr || slopes != nullptr) && maps != 1)) return SLB_ERR_BAD_ARG;
     if (chunk < 0 || (chunk > 0 && window > 0) || (sig_bias != nullptr && (maps != 1 || sink != nullptr)))
         return SLB_ERR_BAD_ARG;
@@ -581,24 +607,27 @@ static int launch_attention_kv_tc(const bf16* q, int ldq, const bf16* kc, const 
     if (ldq % 8 || ((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) % 16) return SLB_ERR_BAD_ARG;
     if ((long long)num_tiles * Hkv * maps > 0x7fffffffll) return SLB_ERR_TOO_LARGE;
     const int box_rows = ps < BN ? ps : BN;
-    CUtensorMap map_k, map_v;
+    CUtensorMap map_q, map_k, map_v;
     const long long rows = (long long)num_pages * Hkv * ps;
     if (rows > 0x7fffffffll) return SLB_ERR_TOO_LARGE;    // box coordinates are 32-bit
     // (a block-table entry outside [0, num_pages) names rows outside the tensor map: the copy
     // reads zeros there, never memory outside the cache)
-    int rc = slb_tma::make_rows_map(&map_k, kc, maps * DK, rows, box_rows);
+    int rc = slb_tma::make_query_map(&map_q, q, maps * DK, H, tokens, ldq, H / Hkv, BM / (H / Hkv));
+    if (rc != 0) return rc;
+    rc = slb_tma::make_rows_map(&map_k, kc, maps * DK, rows, box_rows);
     if (rc != 0) return rc;
     rc = tied ? slb_tma::make_rows_map(&map_v, kc, DK, rows, box_rows)
               : slb_tma::make_rows_map(&map_v, vc, DV, rows, box_rows);
     if (rc != 0) return rc;
     const size_t smem = attn_smem(tied != 0);
     static unsigned long long configured = 0;              // a bit per device
-    rc = slb_configure(&configured, attention_kv_tc_kernel, attn_smem(false) <= SMEM_LIMIT ? attn_smem(false) : attn_smem(true));
+    rc = slb_configure(&configured, attention_kv_tc_kernel,
+                       attn_smem(false) <= SMEM_LIMIT && attn_smem(false) > attn_smem(true) ? attn_smem(false) : attn_smem(true));
     if (rc != 0) return rc;
     int* status = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&status, tc_attn_status);
     if (e != cudaSuccess) return (int)e;
-    return slb_launch(attention_kv_tc_kernel, dim3((unsigned)num_tiles * Hkv * maps), dim3(THREADS), smem, st, q, ldq,
+    return slb_launch(attention_kv_tc_kernel, dim3((unsigned)num_tiles * Hkv * maps), dim3(THREADS), smem, st, map_q,
                       map_k, map_v, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq, tile_row0, H, Hkv,
                       ps, box_rows, scale * 1.4426950408889634f, window, status, tied, gate, ldg, maps, out32, ldo32,
                       softcap > 0.f ? 2.0f * 1.4426950408889634f * scale / softcap : 0.f,
@@ -606,13 +635,13 @@ static int launch_attention_kv_tc(const bf16* q, int ldq, const bf16* kc, const 
 }
 
 extern "C" {
-// num_pages: pages in k_cache ([num_pages][Hkv][ps][DK]) and v_cache ([..][DV]; ignored with `tied`).
-int slb_attention_kv_tc_bf16(const bf16* q, int ldq, const bf16* kc, const bf16* vc, int tied, bf16* out, int ldo,
+// tokens: rows of q.  num_pages: pages in k_cache ([num_pages][Hkv][ps][DK]) and v_cache ([..][DV]; ignored with `tied`).
+int slb_attention_kv_tc_bf16(const bf16* q, int ldq, int tokens, const bf16* kc, const bf16* vc, int tied, bf16* out, int ldo,
                              const int* block_table, int max_pages, const int* cu_q, const int* ctx_len,
                              const int* tile_seq, const int* tile_row0, int num_tiles, int H, int Hkv, int ps,
                              int num_pages, float scale, int window, const bf16* gate, int ldg,
                              cudaStream_t st) {
-    return launch_attention_kv_tc(q, ldq, kc, vc, tied, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq,
+    return launch_attention_kv_tc(q, ldq, tokens, kc, vc, tied, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq,
                                   tile_row0, num_tiles, H, Hkv, ps, num_pages, scale, window, gate, ldg, 1, nullptr,
                                   0, st);
 }
@@ -620,24 +649,24 @@ int slb_attention_kv_tc_bf16(const bf16* q, int ldq, const bf16* kc, const bf16*
 // sink a head (`sink` [H] float32 or null) in the softmax's denominator; with `chunk` > 0 instead of the
 // window and `sig_bias` ([H] float32 or null) instead of the softmax; with slopes of a distance bias
 // (`slopes` [H] float32 or null) and a factor on the results.
-int slb_attention_kv_tc_capped_bf16(const bf16* q, int ldq, const bf16* kc, const bf16* vc, int tied, bf16* out,
+int slb_attention_kv_tc_capped_bf16(const bf16* q, int ldq, int tokens, const bf16* kc, const bf16* vc, int tied, bf16* out,
                                     int ldo, const int* block_table, int max_pages, const int* cu_q,
                                     const int* ctx_len, const int* tile_seq, const int* tile_row0, int num_tiles,
                                     int H, int Hkv, int ps, int num_pages, float scale, int window, const bf16* gate,
                                     int ldg, float softcap, const float* sink, int chunk, const float* sig_bias,
                                     const float* slopes, float out_scale, cudaStream_t st) {
-    return launch_attention_kv_tc(q, ldq, kc, vc, tied, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq,
+    return launch_attention_kv_tc(q, ldq, tokens, kc, vc, tied, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq,
                                   tile_row0, num_tiles, H, Hkv, ps, num_pages, scale, window, gate, ldg, 1, nullptr,
                                   0, st, softcap, sink, chunk, sig_bias, slopes, out_scale);
 }
 // `maps` attention maps a head: q [T][H][maps][DK], k_cache [num_pages][Hkv][ps][maps * DK], one set
 // of values a kv head, float32 results per map out32 [T][H][maps][DV].
-int slb_attention_kv_tc_maps_bf16(const bf16* q, int ldq, const bf16* kc, const bf16* vc, float* out32, int ldo32,
+int slb_attention_kv_tc_maps_bf16(const bf16* q, int ldq, int tokens, const bf16* kc, const bf16* vc, float* out32, int ldo32,
                                   const int* block_table, int max_pages, const int* cu_q, const int* ctx_len,
                                   const int* tile_seq, const int* tile_row0, int num_tiles, int H, int Hkv, int maps,
                                   int ps, int num_pages, float scale, int window, cudaStream_t st) {
     if (out32 == nullptr) return SLB_ERR_BAD_ARG;
-    return launch_attention_kv_tc(q, ldq, kc, vc, 0, nullptr, 0, block_table, max_pages, cu_q, ctx_len, tile_seq,
+    return launch_attention_kv_tc(q, ldq, tokens, kc, vc, 0, nullptr, 0, block_table, max_pages, cu_q, ctx_len, tile_seq,
                                   tile_row0, num_tiles, H, Hkv, ps, num_pages, scale, window, nullptr, 0, maps, out32,
                                   ldo32, st);
 }
@@ -664,18 +693,18 @@ int slb_attention_kv_tc_status(int reset) {
 
 extern "C" {
 int slb_attention_kv_tc_supported(int, int, int) { return 0; }
-int slb_attention_kv_tc_bf16(const bf16*, int, const bf16*, const bf16*, int, bf16*, int, const int*, int, const int*,
+int slb_attention_kv_tc_bf16(const bf16*, int, int, const bf16*, const bf16*, int, bf16*, int, const int*, int, const int*,
                              const int*, const int*, const int*, int, int, int, int, int, float, int, const bf16*,
                              int, cudaStream_t) {
     return SLB_ERR_BAD_ARG;
 }
-int slb_attention_kv_tc_capped_bf16(const bf16*, int, const bf16*, const bf16*, int, bf16*, int, const int*, int,
+int slb_attention_kv_tc_capped_bf16(const bf16*, int, int, const bf16*, const bf16*, int, bf16*, int, const int*, int,
                                     const int*, const int*, const int*, const int*, int, int, int, int, int, float,
                                     int, const bf16*, int, float, const float*, int, const float*, const float*, float,
                                     cudaStream_t) {
     return SLB_ERR_BAD_ARG;
 }
-int slb_attention_kv_tc_maps_bf16(const bf16*, int, const bf16*, const bf16*, float*, int, const int*, int, const int*,
+int slb_attention_kv_tc_maps_bf16(const bf16*, int, int, const bf16*, const bf16*, float*, int, const int*, int, const int*,
                                   const int*, const int*, const int*, int, int, int, int, int, int, float, int,
                                   cudaStream_t) {
     return SLB_ERR_BAD_ARG;

@@ -6,7 +6,7 @@
 // them), so the g query heads of a group share every key/value tile.  Per 64-key
 // tile, with both accumulators in tensor memory (TMEM):
 //
-//   loader warps    TMA tensor copies (128-byte swizzle) of the tile's pages of K (warp 0)
+//   loader warps    TMA tensor copies (128-byte swizzle) of the queries, then of the tile's pages of K (warp 0)
 //                   and of V (warp 6) into two-stage shared-memory rings of their own
 //                                                          -> k_full[stage], v_full[stage]
 //   MMA warp        S = Q.K^T   (tcgen05.mma M=128 N=64,  K=16 x D/16)  -> s_full (scores ready,
@@ -31,6 +31,14 @@
 // TMEM is rescaled rarely.  Two blocks fit on an SM: one does its softmax while the
 // other's MMAs run.
 //
+// What bounds it: a tile's 64 exponentials a row (512 cycles a block and tile, 700 reached with two blocks an
+// SM) and about 4 us of look-ups, first copies and result a block.  The queries come by one copy a panel, and only
+// rows that no copy brings are zeroed, by the loaders.  A few long tiles (a portion of a prompt late in its request)
+// leave SMs empty: then the blocks of a cluster share a tile's keys and add their parts up through shared memory
+// (`splits`).  us before these and the packed arithmetic -> now: 2,048 tokens of 28 / 4 heads of 128 43.5 -> 39.3, 14 / 2
+// heads of 64 30.2 -> 26.4; 449 tokens after 512 beside 31 single ones, 14 / 2 heads 17.3 -> 14.8; 16 tokens after
+// 1,500 22.4 -> 10.6.
+//
 // Every mbarrier wait is bounded; a role that gives up records a code in the status
 // word and leaves its loop; the block then frees its TMEM and returns without a result.
 //
@@ -38,7 +46,7 @@
 // tp_model.py:136-157); masking and softmax follow it (r <= a, optional window).
 #include <cuda.h>
 
-#include "common.cuh"
+#include "softmax_util.cuh"
 #include "tma_util.cuh"
 
 #if (SLB_HEAD_DIM == 64 || SLB_HEAD_DIM == 128)
@@ -59,7 +67,10 @@ constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
 constexpr int OFF_V = OFF_K + 2 * KV_TILE_BYTES;
 constexpr int OFF_BAR = OFF_V + 2 * KV_TILE_BYTES;
-constexpr size_t TC_ATTN_SMEM = OFF_BAR + 128;
+constexpr int OFF_ML = OFF_BAR + 128;          // a row's reference and sum, for the blocks that share its keys
+constexpr size_t TC_ATTN_SMEM = OFF_ML + BM * 8;
+constexpr int MAX_SPLITS = 8;
+static_assert(OFF_BAR - OFF_K >= BM * D * 4, "the rings hold a block's partial result");
 constexpr uint32_t SPIN_LIMIT = 1u << 18;     // a poll that suspends takes about 4 us: about a second
 constexpr float RESCALE_THRESHOLD = 8.f;       // log2 of the largest probability tolerated
 
@@ -165,6 +176,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
 }
+// the 64 scores of this thread's row
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&s)[64]) {
+    uint32_t v[2][32];
+    tmem_ld32(taddr, v[0]);
+    tmem_ld32(taddr + 32, v[1]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 64; ++i) s[i] = __uint_as_float(v[i >> 5][i & 31]);
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -176,24 +196,26 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
           "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
-// 2^x in one MUFU instruction (exp2f adds a range fix-up around it; the probabilities
-// here are rounded to bfloat16 anyway, and -inf gives 0)
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+using slb_softmax::pack2;
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ unsigned pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<unsigned*>(&v);
+// the float at `mine` in block `rank` of the cluster
+__device__ __forceinline__ float cluster_float(const float* mine, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
 __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
-    const bf16* __restrict__ q, int ldq, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, int ldo,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_q,
     const int* __restrict__ ctx_len, const int* __restrict__ tile_seq, const int* __restrict__ tile_row0,
-    int H, int Hkv, int ps, int box_rows, float scale_log2, int window, int* __restrict__ status) {
+    int H, int Hkv, int ps, int box_rows, float scale_log2, int window, int splits, int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // All barriers come in pairs indexed by tile parity.  s_full[b]: Q.K^T of a tile is done
     // (its scores are ready and its keys may be replaced); pv_done[b]: its P.V is done (its
@@ -203,15 +225,17 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
     uint64_t* s_full = v_full + 2;                                      // [2]
     uint64_t* p_full = s_full + 2;                                      // [2], one per score buffer
     uint64_t* pv_done = p_full + 2;                                     // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+    uint64_t* q_full = pv_done + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 1);
 
     pdl_wait();
     const int warp = slb_warp(), lane = threadIdx.x & 31;
     // Blocks are handed out in the order of their linear index: tile by tile from the last
     // (most keys) to the first, all kv heads of a tile together, so that no head's long
     // tiles start late.
-    const int kvh = blockIdx.x % Hkv;
-    const int tile = (int)(gridDim.x / Hkv) - 1 - (int)(blockIdx.x / Hkv);
+    const int rank = (int)blockIdx.x % splits, unit = (int)blockIdx.x / splits, units = (int)gridDim.x / splits;
+    const int kvh = unit % Hkv;
+    const int tile = units / Hkv - 1 - unit / Hkv;
     const int s = tile_seq[tile];
     const int row0 = tile_row0[tile];
     const int g = H / Hkv;
@@ -224,7 +248,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
     const int pos_base = ctx - qlen;
     const int* table = block_table + (size_t)s * max_pages;
     const bool aligned = (smem_u32(smem) & 1023u) == 0;     // the swizzle needs 1024-byte alignment
-    if (nrows <= 0 || !aligned) {
+    if (nrows <= 0 || !aligned) {                            // (every block of a cluster, or none)
         if (!aligned && threadIdx.x == 0) atomicCAS(status, 0, 0x900);
         return;
     }
@@ -232,8 +256,14 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
     const int p_last = pos_base + tok0 + (nrows - 1) / g;
     int kbeg = 0;
     if (window > 0) kbeg = max(0, p_first - window + 1) / BN * BN;
-    const int kend = p_last + 1;
-    const int ntiles = (kend - kbeg + BN - 1) / BN;
+    int kend = p_last + 1;
+    int ntiles = (kend - kbeg + BN - 1) / BN;
+    if (splits > 1) {                                       // this block's share of the keys (maybe none)
+        const int per = (ntiles + splits - 1) / splits, first = min(ntiles, rank * per);
+        ntiles = min(ntiles, first + per) - first;
+        kbeg += first * BN;
+        kend = min(kend, kbeg + ntiles * BN);
+    }
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
@@ -241,6 +271,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             mbar_init(&v_full[i], 1);
             mbar_init(&pv_done[i], 1);
         }
+        mbar_init(q_full, 1);
         mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
         mbar_init(&p_full[0], 128); mbar_init(&p_full[1], 128);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -250,29 +281,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
                      ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // K/V stages start as zeros so that rows no copy fills (absent pages) hold finite values
-    for (int i = threadIdx.x; i < 4 * KV_TILE_BYTES / 16; i += THREADS)
-        reinterpret_cast<uint4*>(smem + OFF_K)[i] = make_uint4(0, 0, 0, 0);
-    // Q tile: the softmax threads copy their rows into the swizzled operand layout
-    if (warp >= 2 && warp < 6) {
-        const int r = (warp & 3) * 32 + lane;
-        unsigned char* qs = smem + OFF_Q;
-        if (r < nrows) {
-            const int tl = r / g, hg = r - tl * g;
-            const bf16* src = q + (size_t)(q0 + tok0 + tl) * ldq + (size_t)(kvh * g + hg) * D;
-#pragma unroll
-            for (int c = 0; c < D / 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src + c * 8);
-                *reinterpret_cast<uint4*>(qs + (c >> 3) * (BM * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < D / 8; ++c)
-                *reinterpret_cast<uint4*>(qs + (c >> 3) * (BM * 128) + r * 128 + ((c & 7) << 4)) =
-                    make_uint4(0, 0, 0, 0);
-        }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -302,6 +310,12 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             }
             return row;
         };
+        if (keys && ntiles > 0 && slb_elected()) {          // the queries: whole tokens, a panel a copy (rows beyond the
+            mbar_expect_tx(q_full, PANELS * (BM / g) * g * 128);               // tile's are computed and not stored)
+#pragma unroll
+            for (int p = 0; p < PANELS; ++p)
+                slb_tma::tma_load_3d(smem + OFF_Q + p * (BM * 128), &map_q, q_full, p * 64, kvh * g, q0 + tok0);
+        }
         int row = lookup(0);
         for (int j = 0; j < ntiles; ++j) {
             const int st = j & 1;
@@ -311,6 +325,16 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
                 break;
             }
             const unsigned got = __ballot_sync(0xffffffffu, row >= 0);
+            if (got != (1u << boxes) - 1u) {               // rows that no copy brings (absent pages) hold zeros
+                for (int b = 0; b < boxes; ++b) {
+                    if (got >> b & 1u) continue;
+                    for (int i = lane; i < PANELS * box_rows * 8; i += 32)
+                        *reinterpret_cast<uint4*>(ring + st * KV_TILE_BYTES + i / (box_rows * 8) * KV_PANEL_BYTES +
+                                                  b * box_rows * 128 + i % (box_rows * 8) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
             if (slb_elected()) {
                 const uint32_t bytes = (uint32_t)__popc(got) * (uint32_t)box_rows * 128u * PANELS;
                 if (bytes) mbar_expect_tx(&full[st], bytes); else mbar_arrive(&full[st]);
@@ -356,7 +380,9 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             }
             return true;
         };
-        bool ok = issue_qk(0);
+        bool ok = true;
+        if (ntiles > 0 && !mbar_spin(q_full, 0)) { gave_up(status, 0x204, 1, 0, ntiles); ok = false; }
+        if (ok && ntiles > 0) ok = issue_qk(0);
         if (ok && ntiles > 1) ok = issue_qk(1);
         for (int j = 0; j < ntiles && ok; ++j) {
             const int st = j & 1;
@@ -383,55 +409,34 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
         const int pos = r < nrows ? pos_base + tok0 + r / g : -1;
         float m_ref = -INFINITY, l = 0.f;
         bool ok = true;
+        const bool live = quarter * 32 < nrows;             // (a warp whose rows are all padding only hands tiles on)
         for (int j = 0; j < ntiles && ok; ++j) {
-            if (!mbar_spin(&s_full[j & 1], (j >> 1) & 1)) { if (lane == 0) gave_up(status, 0x301, 2, j, ntiles); ok = false; break; }
+            if (!(live ? mbar_spin(&s_full[j & 1], (j >> 1) & 1) : mbar_wait(&s_full[j & 1], (j >> 1) & 1))) {
+                if (lane == 0) gave_up(status, 0x301, 2, j, ntiles);
+                ok = false;
+                break;
+            }
+            if (!live) {
+                mbar_arrive(&p_full[j & 1]);
+                continue;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t raw[2][32];
-            tmem_ld32(tmem + lane_base + S_COL + 64 * (j & 1), raw[0]);
-            tmem_ld32(tmem + lane_base + S_COL + 64 * (j & 1) + 32, raw[1]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float s[64];
+            tmem_ld64(tmem + lane_base + S_COL + 64 * (j & 1), s);
             const int k0 = kbeg + j * BN;
             // raw scores stay unscaled; masked ones become -inf.  A tile that every row of
             // the block sees completely needs no mask (rows of padding compute garbage that
             // is never stored).
-            const bool open = k0 + BN - 1 <= p_first && (window <= 0 || p_last - k0 < window);
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, not one
-            if (open) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(raw[h][i]));
-            } else {
-                const int hi = min(BN, min(kend, pos + 1) - k0);      // visible keys: [lo, hi)
-                const int lo = window > 0 ? max(0, pos - window + 1 - k0) : 0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int c = h * 32 + i;
-                        if (!(c >= lo && c < hi)) raw[h][i] = __float_as_uint(-INFINITY);
-                        mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(raw[h][i]));
-                    }
-            }
-            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // scale > 0
+            const bool open = k0 + BN - 1 <= p_first && k0 + BN <= kend && (window <= 0 || p_last - k0 < window);
+            if (!open) slb_softmax::mask_keys(s, window > 0 ? pos - window + 1 - k0 : 0, min(kend, pos + 1) - k0);
+            const float mt = slb_softmax::max_of(s) * scale_log2;     // scale > 0
             float alpha = 1.f;
             if (mt > m_ref + RESCALE_THRESHOLD || (m_ref == -INFINITY && mt != -INFINITY)) {
                 alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mt);
                 m_ref = mt;
             }
-            const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-            float sm[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t packed[32];
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float p0 = fast_exp2(fmaf(__uint_as_float(raw[h][i]), scale_log2, -m_use));
-                    const float p1 = fast_exp2(fmaf(__uint_as_float(raw[h][i + 1]), scale_log2, -m_use));
-                    sm[(i >> 1) & 3] += p0 + p1;
-                    packed[h * 16 + i / 2] = pack2(p0, p1);
-                }
-            l = l * alpha + ((sm[0] + sm[1]) + (sm[2] + sm[3]));
+            l = l * alpha + slb_softmax::exponentials(s, scale_log2, m_ref == -INFINITY ? 0.f : m_ref, packed);
             if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
                 // the accumulator is rescaled (rarely): P.V of the previous tile must be done
                 if (!mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1)) { if (lane == 0) gave_up(status, 0x302, 2, j, ntiles); ok = false; break; }
@@ -452,31 +457,91 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(&p_full[j & 1]);
         }
-        if (ok) {
+        if (ok && ntiles > 0) {
             if (!mbar_wait(&pv_done[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1)) { if (lane == 0) gave_up(status, 0x303, 2, ntiles, ntiles); ok = false; }
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         pdl_launch_dependents();
-        const float inv = l > 0.f ? 1.f / l : 0.f;
-        const int tl = r / g, hg = r - tl * g;
-        bf16* dst = out + (size_t)(q0 + tok0 + tl) * ldo + (size_t)(kvh * g + hg) * D;
+        if (splits == 1) {
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            const int tl = r / g, hg = r - tl * g;
+            bf16* dst = out + (size_t)(q0 + tok0 + tl) * ldo + (size_t)(kvh * g + hg) * D;
 #pragma unroll
-        for (int c0 = 0; c0 < D; c0 += 32) {
-            uint32_t ov[32];
-            tmem_ld32(tmem + lane_base + O_COL + c0, ov);            // warp-wide: every lane takes part
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (ok && r < nrows) {
+            for (int c0 = 0; c0 < D; c0 += 32) {
+                uint32_t ov[32];
+                tmem_ld32(tmem + lane_base + O_COL + c0, ov);        // warp-wide: every lane takes part
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (ok && r < nrows) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint4 v;
-                    v.x = pack2(__uint_as_float(ov[i]) * inv, __uint_as_float(ov[i + 1]) * inv);
-                    v.y = pack2(__uint_as_float(ov[i + 2]) * inv, __uint_as_float(ov[i + 3]) * inv);
-                    v.z = pack2(__uint_as_float(ov[i + 4]) * inv, __uint_as_float(ov[i + 5]) * inv);
-                    v.w = pack2(__uint_as_float(ov[i + 6]) * inv, __uint_as_float(ov[i + 7]) * inv);
-                    *reinterpret_cast<uint4*>(dst + c0 + i) = v;
+                    for (int i = 0; i < 32; i += 8) {
+                        uint4 v;
+                        v.x = pack2(__uint_as_float(ov[i]) * inv, __uint_as_float(ov[i + 1]) * inv);
+                        v.y = pack2(__uint_as_float(ov[i + 2]) * inv, __uint_as_float(ov[i + 3]) * inv);
+                        v.z = pack2(__uint_as_float(ov[i + 4]) * inv, __uint_as_float(ov[i + 5]) * inv);
+                        v.w = pack2(__uint_as_float(ov[i + 6]) * inv, __uint_as_float(ov[i + 7]) * inv);
+                        *reinterpret_cast<uint4*>(dst + c0 + i) = v;
+                    }
+                }
+            }
+        } else {
+            // This block's part of the result, for the other blocks of the row: columns of a thread's row side by side in the
+            // idle rings, and (reference, sum); a block without keys, or one that gave up, counts for nothing.
+            float* part = reinterpret_cast<float*>(smem + OFF_K);
+            float* ml = reinterpret_cast<float*>(smem + OFF_ML);
+            const bool counts = ok && ntiles > 0;
+            ml[r * 2] = counts ? m_ref : -INFINITY;
+            ml[r * 2 + 1] = counts ? l : 0.f;
+            if (ntiles > 0) {
+#pragma unroll
+                for (int c0 = 0; c0 < D; c0 += 32) {
+                    uint32_t ov[32];
+                    tmem_ld32(tmem + lane_base + O_COL + c0, ov);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) part[(c0 + i) * BM + r] = counts ? __uint_as_float(ov[i]) : 0.f;
                 }
             }
         }
+    }
+    if (splits > 1) {
+        __syncwarp();
+        cluster_sync();
+        if (warp >= 2 && warp < 6) {
+            // Thread r finishes its row's share of the columns, the blocks' parts added in their order.
+            const int r = (warp & 3) * 32 + lane, tl = r / g, hg = r - tl * g;
+            const float* part = reinterpret_cast<const float*>(smem + OFF_K);
+            const float* ml = reinterpret_cast<const float*>(smem + OFF_ML);
+            float m = -INFINITY, l = 0.f, w[MAX_SPLITS];
+            for (int k = 0; k < splits; ++k) m = fmaxf(m, cluster_float(ml + r * 2, k));
+#pragma unroll
+            for (int k = 0; k < MAX_SPLITS; ++k) {
+                w[k] = 0.f;
+                if (k >= splits) continue;
+                const float mk = cluster_float(ml + r * 2, k);
+                if (mk != -INFINITY) w[k] = exp2f(mk - m);
+                l += w[k] * cluster_float(ml + r * 2 + 1, k);
+            }
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            const int share = D / splits;                    // (a multiple of 8)
+            bf16* dst = out + (size_t)(q0 + tok0 + tl) * ldo + (size_t)(kvh * g + hg) * D;
+            if (r < nrows) {
+                for (int c = rank * share; c < (rank + 1) * share; c += 8) {
+                    float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int k = 0; k < MAX_SPLITS; ++k) {
+                        if (k >= splits || w[k] == 0.f) continue;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[i] += w[k] * cluster_float(part + (c + i) * BM + r, k);
+                    }
+                    uint4 v;
+                    v.x = pack2(o[0] * inv, o[1] * inv); v.y = pack2(o[2] * inv, o[3] * inv);
+                    v.z = pack2(o[4] * inv, o[5] * inv); v.w = pack2(o[6] * inv, o[7] * inv);
+                    *reinterpret_cast<uint4*>(dst + c) = v;
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();                                      // (the parts stay until every block has read them)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -504,25 +569,30 @@ int slb_prefill_attention_tc_supported(int ps, int group) {
 int slb_prefill_attention_tc_tile_rows(int group) { return group >= 1 && group <= BM ? (BM / group) * group : 0; }
 
 // num_pages: pages in k_cache / v_cache ([num_pages][Hkv][ps][D]).
-int slb_prefill_attention_tc_bf16(const bf16* q, int ldq, const bf16* kc, const bf16* vc, bf16* out, int ldo,
+// tokens: rows of q.  splits: blocks (a cluster) that share the keys of a tile of rows, 1, 2, 4 or 8.
+int slb_prefill_attention_tc_bf16(const bf16* q, int ldq, int tokens, const bf16* kc, const bf16* vc, bf16* out, int ldo,
                                   const int* block_table, int max_pages, const int* cu_q,
                                   const int* ctx_len, const int* tile_seq, const int* tile_row0,
                                   int num_tiles, int H, int Hkv, int ps, int num_pages, float scale,
-                                  int window, cudaStream_t st) {
+                                  int window, int splits, cudaStream_t st) {
     if (num_tiles <= 0) return 0;
+    if (tokens <= 0 || (splits != 1 && splits != 2 && splits != 4 && splits != 8)) return SLB_ERR_BAD_ARG;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || max_pages <= 0 || num_pages <= 0 || !(scale > 0.f))
         return SLB_ERR_BAD_ARG;
     if (!slb_prefill_attention_tc_supported(ps, H / Hkv)) return SLB_ERR_BAD_ARG;
     if (ldq % 8 || ldo % 8 || ((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) % 16)
         return SLB_ERR_BAD_ARG;
-    if ((long long)num_tiles * Hkv > 0x7fffffffll) return SLB_ERR_TOO_LARGE;
+    if ((long long)num_tiles * Hkv * splits > 0x7fffffffll) return SLB_ERR_TOO_LARGE;
     const int box_rows = ps < BN ? ps : BN;
-    CUtensorMap map_k, map_v;
+    CUtensorMap map_q, map_k, map_v;
+    const int g = H / Hkv;
     const long long rows = (long long)num_pages * Hkv * ps;
     if (rows > 0x7fffffffll) return SLB_ERR_TOO_LARGE;    // box coordinates are 32-bit
     // (a block-table entry outside [0, num_pages) names rows outside the tensor map: the copy
     // reads zeros there, never memory outside the cache)
-    int rc = make_cache_map(&map_k, kc, rows, box_rows);
+    int rc = slb_tma::make_query_map(&map_q, q, D, H, tokens, ldq, g, BM / g);
+    if (rc != 0) return rc;
+    rc = make_cache_map(&map_k, kc, rows, box_rows);
     if (rc != 0) return rc;
     rc = make_cache_map(&map_v, vc, rows, box_rows);
     if (rc != 0) return rc;
@@ -532,9 +602,23 @@ int slb_prefill_attention_tc_bf16(const bf16* q, int ldq, const bf16* kc, const 
     int* status = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&status, tc_attn_status);
     if (e != cudaSuccess) return (int)e;
-    return slb_launch(prefill_attention_tc_kernel, dim3((unsigned)num_tiles * Hkv), dim3(THREADS), TC_ATTN_SMEM, st, q, ldq,
-                      map_k, map_v, out, ldo, block_table, max_pages, cu_q, ctx_len, tile_seq, tile_row0, H, Hkv,
-                      ps, box_rows, scale * 1.4426950408889634f, window, status);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)num_tiles * Hkv * splits);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = TC_ATTN_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = slb_pdl_enabled ? attr : attr + 1;
+    cfg.numAttrs = (slb_pdl_enabled ? 1 : 0) + (splits > 1 ? 1 : 0);
+    return (int)cudaLaunchKernelEx(&cfg, prefill_attention_tc_kernel, map_q, map_k, map_v, out, ldo, block_table, max_pages,
+                                   cu_q, ctx_len, tile_seq, tile_row0, H, Hkv, ps, box_rows, scale * 1.4426950408889634f,
+                                   window, splits, status);
 }
 
 // copies the twelve ints that say where waits gave up last (see tc_attn_where)

@@ -37,7 +37,7 @@ CORE_SOURCES = ["elementwise.cu", "rope_cache.cu", "attention_generic.cu", "gemm
                 "decay_gated_chunk.cu", "token_mix.cu", "delta_rule.cu", "delta_rule_chunk.cu",
                 "gated_recurrence.cu", "bottleneck.cu", "state_space.cu",
                 "state_space_chunk.cu"]
-HEADERS = ["common.cuh", "no_alloc.h", "mma_util.cuh", "tma_util.cuh", "decay_attention.cuh",
+HEADERS = ["common.cuh", "no_alloc.h", "mma_util.cuh", "tma_util.cuh", "softmax_util.cuh", "decay_attention.cuh",
            "delta_rule.cuh", "gated_act.cuh", "state_space.cuh"]
 
 _lock = threading.Lock()

@@ -44,6 +44,22 @@ static inline int make_rows_map(CUtensorMap* map, const void* ptr, int row_elems
     return r == CUDA_SUCCESS ? 0 : SLB_ERR_BAD_ARG;
 }
 
+// Queries [tokens][heads][row_elems] (a token's rows `ld` elements apart): boxes of `box_tokens` tokens x `box_heads`
+// heads x 64 elements, which land as rows of 128 bytes in that order
+static inline int make_query_map(CUtensorMap* map, const void* ptr, int row_elems, int heads, long long tokens, int ld,
+                                 int box_heads, int box_tokens) {
+    EncodeTiledFn fn = encode_tiled();
+    if (fn == nullptr) return SLB_ERR_BAD_ARG;
+    const cuuint64_t dims[3] = {(cuuint64_t)row_elems, (cuuint64_t)heads, (cuuint64_t)tokens};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_elems * 2, (cuuint64_t)ld * 2};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)box_heads, (cuuint32_t)box_tokens};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : SLB_ERR_BAD_ARG;
+}
+
 // The same matrix seen as [panels of 64 elements][rows][64]: a box of
 // {64, box_rows, row_elems / 64} brings box_rows whole rows with ONE copy and lands
 // as [panel][row][64 elements], each 128-byte line swizzled as in the 2-D form.

@@ -470,6 +470,27 @@ def has_fast_attention(head_dim: int) -> bool:
 use_tc_prefill = True       # tcgen05 prefill attention where it applies (head size 64/128)
 
 
+prefill_force_splits = 0    # measurements and tests: blocks that share a tile's keys (1, 2, 4, 8), 0: by the rule below
+
+
+def prefill_splits(units: int, longest_context: int, window: int, head_dim: int) -> int:
+    """Blocks (a cluster) that share the keys of a tile of query rows.  A key tile takes a block 0.6 us, adding the blocks'
+    parts up 2.5 us (head size 64) to 3.5 us (128), so the keys must be many, more so where the blocks then share SMs.
+    us with 1 / 2 / 4 / 8 blocks, units (tiles of rows x kv heads), key tiles: 14 heads of 64, 34, 5 8.2 / 9.6 / 9.4 / 17.3;
+    40, 11 11.4 / 11.1 / 11.2 / 19.1; 78, 11 12.0 / 12.3 / 18.3 / 29.9; 112, 15 14.8 / 15.4 / 21.6 / 40.1; 42, 33 25.8 / 18.4
+    / 16.6 / 21.1; 8, 17 15.4 / 13.3 / 11.4 / 10.6; 28 heads of 128, 80, 11 12.1 / 15.5 / 23.9 / 37.2; 84, 33 28.1 / 26.8 /
+    27.0 / 38.7; 16, 17 17.6 / 16.7 / 13.9 / 14.4; 12, 32 24.8 / 19.3 / 14.8 / 13.1."""
+    if prefill_force_splits:
+        return prefill_force_splits
+    seen = min(longest_context, window + 63) if window > 0 else longest_context
+    tiles, sms, best = -(-seen // 64), _num_sms(), 1
+    for splits, alone, shared in ((2, 12, 24), (4, 16, 32), (8, 18, 32)):
+        need = alone + (4 if head_dim > 64 else 0) if splits * units <= sms else shared
+        if splits * units <= 2 * sms and tiles >= need:
+            best = splits
+    return best
+
+
 def prefill_attention(ctx, q, k_cache, v_cache, out, block_table, num_heads, num_kv_heads,
                       head_dim, page_size, scale, window) -> None:
     lib = L.attention(head_dim)
@@ -478,10 +499,11 @@ def prefill_attention(ctx, q, k_cache, v_cache, out, block_table, num_heads, num
             and lib.slb_prefill_attention_tc_supported(page_size, group)):
         tile_seq, tile_row0, n = ctx.attention_tiles(group, lib.slb_prefill_attention_tc_tile_rows(group))
         L.check(lib.slb_prefill_attention_tc_bf16(
-            q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
+            q.data_ptr(), q.stride(0), q.shape[0], k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
             out.stride(0), block_table.data_ptr(), block_table.shape[1], ctx.cu_q.data_ptr(),
             ctx.ctx_len.data_ptr(), tile_seq.data_ptr(), tile_row0.data_ptr(), n, num_heads,
-            num_kv_heads, page_size, k_cache.shape[0], float(scale), int(window), _stream()),
+            num_kv_heads, page_size, k_cache.shape[0], float(scale), int(window),
+            prefill_splits(n * num_kv_heads, ctx.split_hint_len, window, head_dim), _stream()),
             "prefill_attention_tc")
         return
     tile_seq, tile_row0, n = ctx.attention_tiles(num_heads // num_kv_heads,
@@ -1186,7 +1208,7 @@ def attention_kv_tc(ctx, q, k_cache, v_cache, tied: bool, out, block_table, num_
     lib = L.attention_kv(k_dim, v_dim)
     group = num_heads // num_kv_heads
     tile_seq, tile_row0, n = ctx.attention_tiles(group, lib.slb_attention_kv_tc_tile_rows(group))
-    args = (q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), 1 if tied else 0, out.data_ptr(),
+    args = (q.data_ptr(), q.stride(0), q.shape[0], k_cache.data_ptr(), v_cache.data_ptr(), 1 if tied else 0, out.data_ptr(),
             out.stride(0), block_table.data_ptr(), block_table.shape[1], ctx.cu_q.data_ptr(),
             ctx.ctx_len.data_ptr(), tile_seq.data_ptr(), tile_row0.data_ptr(), n, num_heads, num_kv_heads,
             page_size, k_cache.shape[0], float(scale), int(window), _p(head_gate),
@@ -1207,7 +1229,7 @@ def attention_kv_tc_maps(ctx, q, k_cache, v_cache, out, block_table, num_heads: 
     group = num_heads // num_kv_heads
     tile_seq, tile_row0, n = ctx.attention_tiles(group, lib.slb_attention_kv_tc_tile_rows(group))
     L.check(lib.slb_attention_kv_tc_maps_bf16(
-        q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0),
+        q.data_ptr(), q.stride(0), q.shape[0], k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0),
         block_table.data_ptr(), block_table.shape[1], ctx.cu_q.data_ptr(), ctx.ctx_len.data_ptr(),
         tile_seq.data_ptr(), tile_row0.data_ptr(), n, num_heads, num_kv_heads, maps, page_size,
         k_cache.shape[0], float(scale), int(window), _stream()), "attention_kv_tc")

@@ -289,8 +289,8 @@ def attention(head_dim: int) -> ctypes.CDLL:
                 f"the attention kernels for head size {head_dim} are not available: {e}") from e
         _declare(lib, _ATTN_SIGNATURES, True)
         if hasattr(lib, "slb_prefill_attention_tc_bf16"):
-            lib.slb_prefill_attention_tc_bf16.argtypes = [P, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I,
-                                                          F, I, P]
+            lib.slb_prefill_attention_tc_bf16.argtypes = [P, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I,
+                                                          F, I, I, P]
             lib.slb_prefill_attention_tc_bf16.restype = I
         lib.slb_decode_attention_scratch_bytes.argtypes = [I, I, I]
         lib.slb_decode_attention_scratch_bytes.restype = ctypes.c_longlong
@@ -322,10 +322,10 @@ _ATTN_KV_SIGNATURES = {
     "slb_attention_kv_tc_tile_rows": [I],
     "slb_attention_kv_tc_status": [I],
     "slb_attention_kv_tc_where": [P],
-    "slb_attention_kv_tc_bf16": [P, I, P, P, I, P, I, P, I, P, P, P, P, I, I, I, I, I, F, I, P, I, P],
-    "slb_attention_kv_tc_capped_bf16": [P, I, P, P, I, P, I, P, I, P, P, P, P, I, I, I, I, I, F, I, P, I, F, P, I, P,
+    "slb_attention_kv_tc_bf16": [P, I, I, P, P, I, P, I, P, I, P, P, P, P, I, I, I, I, I, F, I, P, I, P],
+    "slb_attention_kv_tc_capped_bf16": [P, I, I, P, P, I, P, I, P, I, P, P, P, P, I, I, I, I, I, F, I, P, I, F, P, I, P,
                                         P, F, P],
-    "slb_attention_kv_tc_maps_bf16": [P, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, I, F, I, P],
+    "slb_attention_kv_tc_maps_bf16": [P, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, I, F, I, P],
 }
 
 

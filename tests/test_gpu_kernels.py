@@ -497,6 +497,28 @@ def test_prefill_attention_tensor_cores(H, Hkv, D, ps, window):
             kernels_module.use_tc_prefill = True
 
 
+@pytest.mark.parametrize("splits", [2, 4, 8])
+@pytest.mark.parametrize("H,Hkv,D,ps", [(7, 1, 64, 8), (28, 4, 128, 16), (3, 3, 64, 64), (8, 1, 128, 32)])
+@pytest.mark.parametrize("window", [0, 40])
+def test_prefill_attention_with_keys_shared_by_a_cluster(H, Hkv, D, ps, window, splits):
+    """Blocks that share a tile's keys, among them blocks without any (one key, a window of 40), a tile with one row and
+    requests of one token beside portions: the bound of the unsplit kernel."""
+    case = PagedCase([37, 150, 1, 963, 34, 300], [37, 19, 1, 1, 2, 300], H, Hkv, D, ps,
+                     torch.bfloat16, seed=D + window + splits)
+    case.scatter()
+    ctx, q, table = _ctx_for(case)
+    from servelab_b200.ops import kernels as kernels_module
+    want = case.reference(window=window or None)
+    kernels_module.prefill_force_splits = splits
+    try:
+        out = torch.full_like(q, 3.0)
+        K().prefill_attention(ctx, q, case.kc, case.vc, out, table, H, Hkv, D, ps, 1 / math.sqrt(D), window)
+    finally:
+        kernels_module.prefill_force_splits = 0
+    assert K().prefill_attention_tc_status(D, reset=True) == 0, "a bounded wait gave up"
+    assert (out.float().cpu() - want).abs().max() <= TOL["bfloat16"]
+
+
 def test_prefill_attention_tcgen05_many_launches_of_a_long_prompt():
     """A 2,048-token prompt at the 7B head layout, 300 launches back to back with matrix
     products between them: 137,000 blocks whose roles (loader, MMA issuer, softmax
