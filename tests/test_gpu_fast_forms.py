@@ -606,3 +606,57 @@ def test_routed_experts_on_sorted_rows(T, E, top, h, I, half):
         y = x[t].double() @ wg[e].double().T
         want = want.index_add(0, t, w[t, k].double()[:, None] * (_act64(y[:, :I], y[:, I:], "silu") @ wd[e].double().T))
     assert (got - want).norm() <= 6e-3 * want.norm()
+
+
+@pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (5, 1, 1, 5), (32, 4, 2, 4), (60, 3, 2, 6), (100, 1, 1, 32), (128, 32, 9, 8),
+                                               (128, 2, 1, 3)])
+@pytest.mark.parametrize("score_fn", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("corrected", [False, True])
+def test_choice_of_up_to_128_experts(E, groups, keep, top, score_fn, corrected):
+    """Rows with equal scores, zeros of both signs, infinities and no numbers, chosen one by one on the host: the same ids,
+    weights to the rounding of the exponentials and of a sum of 128 (2e-6)."""
+    T, g = 41, gen(E + top)
+    z = (torch.randn(T, E, device=DEV, generator=g) * 2).round(decimals=1)
+    z[1] = 0.0
+    z[2, ::2] = -0.0
+    z[3, E // 2:] = float("-inf")
+    if score_fn == "sigmoid":                                  # (a row's softmax has no number once one logit has none)
+        z[4, ::3] = float("nan")
+        z[5, ::2] = float("inf")
+    corr = (torch.randn(E, device=DEV, generator=g) * 0.1).round(decimals=1) if corrected else None
+    ids, w = K().moe_route_scored(z, groups, keep, top, 1.5, True, score_fn, corr, 1, 1e-9)
+    zc, per = z.cpu(), E // groups
+    for t in range(T):
+        s = torch.softmax(zc[t], 0) if score_fn == "softmax" else torch.sigmoid(zc[t])
+        c = zc[t] if score_fn == "sigmoid" and corr is None and groups == 1 else s + (corr.cpu() if corr is not None else 0.0)
+        if score_fn == "sigmoid" and groups == 1 and corr is None or t < 3 and corr is None:
+            c = zc[t]                                          # (the same order; float32 sums differ from the kernel's)
+        cs, open_groups = c.tolist(), list(range(groups))
+        if groups > 1:
+            score = []
+            for k in range(groups):
+                part = [v for v in cs[k * per:(k + 1) * per] if v == v]
+                score.append(max(part) if part else 0.0)
+            open_groups = sorted(open_groups, key=lambda k: (-score[k], k))[:keep]
+        left = [e for e in range(E) if e // per in open_groups and cs[e] > float("-inf")]
+        order = sorted(left, key=lambda e: (-cs[e], e))[:top]
+        order += [None] * (top - len(order))
+        if score_fn == "sigmoid" and corr is None and groups == 1 or t < 3 and corr is None:
+            assert ids[t].tolist() == [0 if e is None else e for e in order], (t, order)
+        if score_fn == "softmax" or t != 4:
+            got = ids[t].tolist()
+            weight = [0.0 if e is None else float(s[i]) for e, i in zip(order, got)]
+            want = torch.tensor(weight) / (sum(weight) + 1e-9) * 1.5
+            assert torch.allclose(w[t].cpu(), want, rtol=2e-6, atol=1e-7), t
+
+
+@pytest.mark.parametrize("E,top", [(7, 3), (32, 4), (64, 8), (128, 32)])
+@pytest.mark.parametrize("score_fn", ["softmax", "sigmoid"])
+def test_choice_of_few_experts_equals_the_general_kernel(E, top, score_fn):
+    """The same logits padded with minus infinities to more experts than the other kernel takes: the same bits."""
+    z = torch.randn(300, E, device=DEV, generator=gen(E))
+    z[7] = z[7, 0]
+    wide = torch.full((300, 200), float("-inf"), device=DEV)
+    wide[:, :E] = z
+    a, b = (K().moe_route_scored(v, 1, 1, top, 2.0, False, score_fn) for v in (z, wide))
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
