@@ -10,6 +10,10 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// 1 / (1 + e^-z) for results of type T: rounded to bfloat16, from the hardware exponential and reciprocal
+template <typename T> __device__ __forceinline__ float sigmoid_for(float z) {
+    return sizeof(T) == 2 ? rcp_approx(1.0f + __expf(-z)) : 1.0f / (1.0f + expf(-z));
+}
 // For results that are rounded to bfloat16: the hardware exponential and reciprocal (errors of
 // a few 1e-7 relative, a thousand times below the rounding).  The correctly rounded reciprocal is a call a value:
 // half of the time of a product's epilogue with it (13,200 cycles a tile of 256 tokens, tanh-GELU 6,500).

@@ -26,7 +26,7 @@
 // over the latent, rotation of the rest; queries rotated from `rot_off` on, not normed).
 // One block a token (and group of vectors), one warp a vector at a time; the token's sines and
 // cosines are formed once a block; float32 arithmetic, angles in float32.
-#include "common.cuh"
+#include "gated_act.cuh"
 
 #define HP_WARPS 4
 #define HP_MAX_D 1152
@@ -533,12 +533,13 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const T* __restrict__
     const size_t t = blockIdx.x;
     for (int c = threadIdx.x; c < N; c += blockDim.x) {
         const float z = to_float(gate[t * ldg + c / group]);
-        out[t * ldo + c] = from_float<T>(to_float(x[t * ldx + c]) / (1.0f + expf(-z)));
+        out[t * ldo + c] = from_float<T>(sizeof(T) == 2 ? to_float(x[t * ldx + c]) * sigmoid_for<T>(z) : to_float(x[t * ldx + c]) / (1.0f + expf(-z)));
     }
 }
 
 // The same on bfloat16 rows in 16-byte pieces (8 elements under one gate value or 8 of them): a piece a
-// thread over all rows, so that every load is in flight at once (2,082 rows of 2,048: 14.6 -> 7.0 us).
+// thread over all rows, so that every load is in flight at once (2,082 rows of 2,048: 14.6 -> 7.0 us; 2,048
+// rows 5.7 -> 4.4 with the approximate reciprocal).
 __global__ void __launch_bounds__(256) sigmoid_gate_vec_kernel(const bf16* __restrict__ x, int ldx,
                                                                const bf16* __restrict__ gate, int ldg,
                                                                bf16* __restrict__ out, int ldo, int row_pieces,
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_vec_kernel(const bf16* __res
     }
     unpack8(raw, v);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = v[e] / (1.0f + expf(-z[e]));
+    for (int e = 0; e < 8; ++e) v[e] *= sigmoid_for<bf16>(z[e]);
     *reinterpret_cast<uint4*>(out + t * ldo + c) = pack8(v);
 }
 

@@ -15,7 +15,7 @@
 //                        ([group][2][size]); w and gate optional; act: sigmoid or SiLU.
 //
 // All arithmetic float32; sums over a row run in an order that depends only on the row's size.
-#include "common.cuh"
+#include "gated_act.cuh"
 
 #define HY_MAX_STREAMS 8
 
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(128) group_norm_gate_kernel(
         if (w != nullptr) x *= w[col];
         if (gate != nullptr) {
             const float z = to_float(gate[(size_t)t * ldg + col]);
-            const float sg = 1.0f / (1.0f + expf(-z));
+            const float sg = sigmoid_for<T>(z);
             x *= gate_act == 2 ? z * sg : sg;
         }
         out[(size_t)t * ldo + col] = from_float<T>(x);
@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(128) group_norm_gate_kernel(
 // a thread keeps GGN_NV vectors of V elements in registers, longer parts are formed again.
 #define GGN_THREADS 256
 #define GGN_NV 4
-__device__ __forceinline__ float gated_by(float x, float z, int gate_act) {
-    const float sg = 1.0f / (1.0f + expf(-z));
+template <typename T> __device__ __forceinline__ float gated_by(float x, float z, int gate_act) {
+    const float sg = sigmoid_for<T>(z);
     return x * (gate_act == 2 ? z * sg : sg);
 }
 __device__ __forceinline__ void ggn_load(const float* p, float (&v)[4]) {
@@ -200,13 +200,13 @@ __global__ void __launch_bounds__(GGN_THREADS) gate_group_norm_kernel(
         if (c < size) {
 #pragma unroll
             for (int e = 0; e < V; ++e) {
-                v[j][e] = gated_by(v[j][e], z[j][e], gate_act);
+                v[j][e] = gated_by<T>(v[j][e], z[j][e], gate_act);
                 ss += v[j][e] * v[j][e];
             }
         }
     }
     for (int c = threadIdx.x + GGN_NV * V * blockDim.x; c < size; c += blockDim.x) {
-        const float u = gated_by(xr[c], to_float(gr[c]), gate_act);
+        const float u = gated_by<T>(xr[c], to_float(gr[c]), gate_act);
         ss += u * u;
     }
     const float rstd = factor / sqrtf(block_sum(ss, scratch) / (float)size + eps);
@@ -222,13 +222,14 @@ __global__ void __launch_bounds__(GGN_THREADS) gate_group_norm_kernel(
         }
     }
     for (int c = threadIdx.x + GGN_NV * V * blockDim.x; c < size; c += blockDim.x)
-        o[c] = from_float<T>(gated_by(xr[c], to_float(gr[c]), gate_act) * rstd * (w != nullptr ? w[c0 + c] : 1.f));
+        o[c] = from_float<T>(gated_by<T>(xr[c], to_float(gr[c]), gate_act) * rstd * (w != nullptr ? w[c0 + c] : 1.f));
 }
 
 // Both orders of norm and gate for parts of whole 16-byte pieces up to 1,024 elements: a warp a (token, part) with
 // the part in registers, all loads issued together, no block-wide sum to wait for.  What bounds it is memory
 // (float32 row in, gate in, row out) and the gate's exponentials.  Norm then gate, a warp that reads element by
-// element and twice against this: 2,048 tokens of 8 x 256 11.4 -> 8.7 us, of 16 x 128 14.1 -> 10.8.
+// element and twice against this: 2,048 tokens of 8 x 256 11.4 -> 8.7 us, of 16 x 128 14.1 -> 10.8.  (The approximate
+// reciprocal for bfloat16 results: 2,912 tokens of 4 x 512 10.1 -> 8.0, 2,048 of 16 x 128 10.3 -> 9.7.)
 template <typename T, int NV, int MAPS, bool GATE_FIRST>
 __global__ void __launch_bounds__(128) group_norm_warp_kernel(
     const float* __restrict__ in, int ldi, const float* __restrict__ lam, const float* __restrict__ w, float eps,
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(128) group_norm_warp_kernel(
     for (int j = 0; j < NV; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            if (GATE_FIRST) v[j][e] = gated_by(v[j][e], z[j][e], gate_act);
+            if (GATE_FIRST) v[j][e] = gated_by<T>(v[j][e], z[j][e], gate_act);
             ss += v[j][e] * v[j][e];
         }
     const float rstd = factor / sqrtf(warp_sum(ss) / (float)size + eps);
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(128) group_norm_warp_kernel(
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             v[j][e] = v[j][e] * rstd * wv[e];
-            if (!GATE_FIRST && gate != nullptr) v[j][e] = gated_by(v[j][e], z[j][e], gate_act);
+            if (!GATE_FIRST && gate != nullptr) v[j][e] = gated_by<T>(v[j][e], z[j][e], gate_act);
         }
         ggn_store(out + t * ldo + (size_t)g * size + c, v[j]);
     }
