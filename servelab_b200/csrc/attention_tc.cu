@@ -328,9 +328,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             if (got != (1u << boxes) - 1u) {               // rows that no copy brings (absent pages) hold zeros
                 for (int b = 0; b < boxes; ++b) {
                     if (got >> b & 1u) continue;
-                    for (int i = lane; i < PANELS * box_rows * 8; i += 32)
-                        *reinterpret_cast<uint4*>(ring + st * KV_TILE_BYTES + i / (box_rows * 8) * KV_PANEL_BYTES +
-                                                  b * box_rows * 128 + i % (box_rows * 8) * 16) = make_uint4(0, 0, 0, 0);
+                    slb_tma::zero_box(ring + st * KV_TILE_BYTES + b * box_rows * 128, PANELS, KV_PANEL_BYTES, box_rows * 128,
+                                      lane);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();

@@ -106,4 +106,12 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
+// Zeros in the rows of a box that no copy brings: `bytes` of each of its panels, panel_bytes apart (a warp; `bytes` a
+// multiple of 1024)
+__device__ __forceinline__ void zero_box(unsigned char* box, int panels, int panel_bytes, int bytes, int lane) {
+    for (int p = 0; p < panels; ++p)
+        for (int i = lane * 16; i < bytes; i += 512)
+            *reinterpret_cast<uint4*>(box + p * panel_bytes + i) = make_uint4(0, 0, 0, 0);
+}
+
 }  // namespace slb_tma
