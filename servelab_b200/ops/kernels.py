@@ -1601,13 +1601,15 @@ def state_space(ctx, u: torch.Tensor, dt: torch.Tensor, state: torch.Tensor, out
             and ctx.num_tokens >= state_space_chunk_min_tokens * ctx.num_seqs):
         c = _StateSpaceChunkArgs()
         tile_seq, tile_row0, n = ctx.attention_tiles(1, L.core().slb_state_space_chunk_tokens())
-        work = torch.empty((max(n, 1), num_heads, state_dim, value_dim), dtype=_F32, device=u.device)
+        work = torch.empty((max(n, 1), num_heads, state_dim, -(-value_dim // 16) * 16), dtype=_F32, device=u.device)
         total = torch.empty((max(n, 1), num_heads), dtype=_F32, device=u.device)
         c.a, c.tile_seq, c.tile_row0, c.num_tiles = a, tile_seq.data_ptr(), tile_row0.data_ptr(), n
         c.work, c.total = work.data_ptr(), total.data_ptr()
-        L.check(L.core().slb_state_space_chunk_bf16(_ct.byref(c), ctx.num_seqs, _stream()), "state_space (chunks)")
+        # (a padded step may be replayed with other lengths)
+        longest = 0 if getattr(ctx, "_padded_tiles", None) is not None else max(ctx.q_lens)
+        L.check(L.core().slb_state_space_chunk_bf16(_ct.byref(c), ctx.num_seqs, longest, _stream()), "state_space (chunks)")
         global launch_count
-        launch_count += 2
+        launch_count += 1
         return
     fn = getattr(L.core(), "slb_state_space_" + _suffix(u.dtype))
     L.check(fn(_ct.byref(a), ctx.num_seqs, _stream()), "state_space")

@@ -378,6 +378,18 @@ def test_experts_products_at_few_and_many_rows(T, E, top, h, I):
 def test_chunks_in_pieces_are_those_of_the_general_kernels(H, P, N, G, lens):
     """Rows at an odd address go to the general kernels, whose weighted x is rounded in another order before its split
     (2^-17 of every term)."""
+    _chunks_in_pieces(H, P, N, G, lens)
+
+
+@pytest.mark.parametrize("lens", [[700, 65, 1300], [2000], [64] * 40 + [1]])
+@pytest.mark.parametrize("H,P,N,G", [(48, 64, 128, 2), (20, 136, 64, 1), (33, 64, 64, 1), (128, 8, 128, 1)])
+def test_blocks_of_several_heads_are_those_of_the_general_kernels(H, P, N, G, lens):
+    """Sizes whose blocks take two heads and more, a remainder of heads at the end of a group, heads of several blocks of
+    columns."""
+    _chunks_in_pieces(H, P, N, G, lens)
+
+
+def _chunks_in_pieces(H, P, N, G, lens):
     g, T = gen(H + len(lens)), sum(lens)
     ctx, _ = step(lens)
     rows = torch.randn(T, H * P + 2 * G * N, device=DEV, generator=g).bfloat16()
