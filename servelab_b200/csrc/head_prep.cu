@@ -26,6 +26,8 @@
 // over the latent, rotation of the rest; queries rotated from `rot_off` on, not normed).
 // One block a token (and group of vectors), one warp a vector at a time; the token's sines and
 // cosines are formed once a block; float32 arithmetic, angles in float32.
+#include <type_traits>
+
 #include "gated_act.cuh"
 
 #define HP_WARPS 4
@@ -236,10 +238,11 @@ __device__ __forceinline__ float square8(const float* v) {
 }
 
 // PIECES: 16-byte pieces of a vector a lane may hold (2: vectors of more than 256 elements).  ROW: all
-// heads of a token are normed together (one round and one block then hold the whole token).
-template <int PIECES, bool ROW>
-__global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constant__ HeadPrepArgs a,
-                                                            const __grid_constant__ HeadPrepPlan p) {
+// heads of a token are normed together (one round and one block then hold the whole token).  DENSE: a third more
+// warps an SM, with some registers spilled (the launch decides).
+template <int PIECES, bool ROW, bool DENSE>
+__global__ void __launch_bounds__(256, (PIECES == 1 ? 3 : 2) + (DENSE ? 1 : 0)) head_prep_vec_kernel(
+    const __grid_constant__ HeadPrepArgs a, const __grid_constant__ HeadPrepPlan p) {
     extern __shared__ __align__(16) float hp_smem[];
     __shared__ float2 row_part[8];
     float* cs_tab = hp_smem;                              // of the token's angles, once a block
@@ -252,8 +255,6 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
     const int step = warps * gridDim.y;
     const int pos = a.positions[t];
     int page = -1;                                        // where this token's key and value go
-    if (a.k_cache != nullptr || a.v_cache != nullptr)
-        page = a.block_table[(size_t)a.seq_of_token[t] * a.max_pages + pos / a.page_size];
     for (int first = blockIdx.y * warps + warp, round = 0; round * HPV_ITEMS * step < p.items;
          ++round, first += HPV_ITEMS * step) {
         uint4 raw[HPV_ITEMS][PIECES];
@@ -275,7 +276,9 @@ __global__ void __launch_bounds__(256) head_prep_vec_kernel(const __grid_constan
                     raw[j][c] = *reinterpret_cast<const uint4*>(row + kd.off + unit[j] * kd.stride + piece * 8);
             }
         }
-        if (round == 0) {
+        if (round == 0) {                                 // (its lookup waits for two loads: behind the row's)
+            if (a.k_cache != nullptr || a.v_cache != nullptr)
+                page = a.block_table[(size_t)a.seq_of_token[t] * a.max_pages + pos / a.page_size];
             for (int i = threadIdx.x; i < a.rot_dims / 2; i += blockDim.x) {
                 float sn, cs;
                 sincosf((float)pos * a.freq[i], &sn, &cs);
@@ -585,8 +588,18 @@ static int launch_head_prep(const HeadPrepArgs& a, int num_tokens, cudaStream_t 
         // (a step of few tokens: a block a few vectors, so that it still fills the device)
         const int split = num_tokens < 512 && !a.row_norm ? (plan.items + warps - 1) / warps : 1;
         const bool wide = plan.kind[0].pieces > 32 || plan.kind[1].pieces > 32 || plan.kind[2].pieces > 32;
-        auto kernel = a.row_norm ? (wide ? head_prep_vec_kernel<2, true> : head_prep_vec_kernel<1, true>)
-                                 : (wide ? head_prep_vec_kernel<2, false> : head_prep_vec_kernel<1, false>);
+        auto pick = [&](auto dense) {
+            return a.row_norm ? (wide ? head_prep_vec_kernel<2, true, dense.value> : head_prep_vec_kernel<1, true, dense.value>)
+                              : (wide ? head_prep_vec_kernel<2, false, dense.value> : head_prep_vec_kernel<1, false, dense.value>);
+        };
+        // (a block is a chain of latencies, 2.8 us, and a round of blocks costs that whatever it holds: with more warps an
+        // SM, spilled registers and an eighth (long vectors: a third) more a round, when that saves rounds.  16 + 4 heads
+        // of 128 turned: 1,024 tokens 9.8 -> 8.0 us, 2,048 14.4 -> 12.7; 40 + 8 heads 1,024 22.7 -> 16.9; all steps with
+        // it: 700 tokens 1.2-1.3 times as long, 256 the same)
+        const long long blocks = (long long)num_tokens * split, sms = slb_num_sms();
+        const long long usual = sms * ((wide ? 16 : 24) / warps), dense = sms * ((wide ? 24 : 32) / warps);
+        const bool fewer = 24 * ((blocks + usual - 1) / usual) > (wide ? 32 : 27) * ((blocks + dense - 1) / dense);
+        auto kernel = fewer ? pick(std::true_type{}) : pick(std::false_type{});
         HeadPrepArgs read = a;                           // (a bias has the elements too that are not read)
         if (a.q_bias != nullptr && !a.row_norm)
             read.q_bias += head_prep_drop(a.q_norm_dims, a.q_unit_dims, a.rot_dims ? a.q_rot_off : 0, a.q_skip);

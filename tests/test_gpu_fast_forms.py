@@ -76,7 +76,7 @@ HEADS = {   # q heads, kv heads, key size, value size, rotated, halves, norm, un
 
 
 @pytest.mark.parametrize("name", HEADS)
-@pytest.mark.parametrize("lens", [[1], [3, 1, 40], [700]])
+@pytest.mark.parametrize("lens", [[1], [3, 1, 40], [700], [1100]])
 def test_heads_in_pieces_are_those_of_the_general_kernel(name, lens):
     """The general kernel runs on rows at odd addresses; both work in float32 and differ in the order of a head's sum
     of squares: one rounding to bfloat16 (2^-8 of a value) and 2^-16 of the largest where a rotation cancels."""
