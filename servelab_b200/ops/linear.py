@@ -4,9 +4,10 @@ float32: always this package's CUDA-core kernel (true 32-bit, fixed summation
 order per output).  bfloat16: the vendor library's tensor-core GEMM through
 torch (the reference's engine also calls a library for its products,
 servelab/parallel/tp_model.py:48-53), except for shapes whose rows are not
-16-byte aligned, which go to the CUDA-core kernel, and for small token counts
+16-byte aligned, which go to the CUDA-core kernel, for small token counts
 (decode steps), which go to this package's tcgen05 weight-streaming kernels
-(TMA-fed, accumulating in tensor memory).
+(TMA-fed, accumulating in tensor memory), and for gate|up products of many
+tokens, whose activation is in the epilogue of this package's pair kernel.
 """
 
 from __future__ import annotations
