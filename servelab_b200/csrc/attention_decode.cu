@@ -126,7 +126,7 @@ __device__ __forceinline__ BoxGeometry box_geometry(int rows) {
 // One tile's copies, issued by the calling warp.  Lane b looks box b up (box_rows keys of
 // one page, every panel, in ONE tiled copy each for K and V); `page` is that box's entry
 // of the block table.  Boxes that are not fetched are zero-filled by the whole warp with
-// ordinary stores; lane 0 arrives on `bar` (count 1) with the bytes of all copies.
+// ordinary stores; an elected lane arrives on `bar` (count 1) with the bytes of all copies.
 __device__ __forceinline__ void produce_tile(unsigned char* Kd, unsigned char* Vd, uint64_t* bar,
                                              const CUtensorMap* map_k, const CUtensorMap* map_v,
                                              int page, int k0, int ctx, int kvh, int Hkv, int ps,
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(NTHREADS) decode_attention_ws_kernel(
                 nxt = lookup(group + 1);
             }
             const int page = __shfl_sync(0xffffffffu, cur, (box0 + lane) & 31);
-            if (!mbar_wait(&empty_bar[st], ((t / stages) - 1) & 1)) {
+            if (!slb_warp_agrees(mbar_wait(&empty_bar[st], ((t / stages) - 1) & 1))) {
                 if (lane == 0) { atomicCAS(&dec_status_word, 0, 0x10); failed = 1; }
                 break;
             }
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(NTHREADS) decode_attention_ws_kernel(
         constexpr int VPRE = D <= 128 ? MT : 0;            // V fragments fetched before the softmax
         for (int t = 0; t < ntiles; ++t) {
             const int st = t % stages;
-            if (!mbar_wait(&full_bar[st], (t / stages) & 1)) {
+            if (!slb_warp_agrees(mbar_wait(&full_bar[st], (t / stages) & 1))) {
                 if (lane == 0) { atomicCAS(&dec_status_word, 0, 0x20); failed = 1; }
                 break;
             }

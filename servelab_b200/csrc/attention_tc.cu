@@ -100,18 +100,17 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
+// Bounded wait for the phase of the given parity, entered by a whole warp: false in every lane if it ran out in one.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
-        uint32_t done;
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < SPIN_LIMIT && !done; ++i)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
+    return slb_warp_agrees(done != 0);
 }
 // The same wait for hand-overs on the critical path of a tile (scores ready, P ready):
 // test_wait does not suspend the thread, so the waiter sees the phase within tens of
@@ -119,16 +118,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 // shorter).
 __device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < SPIN_LIMIT * 64u; ++i) {
-        uint32_t done;
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < SPIN_LIMIT * 64u && !done; ++i)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
+    return slb_warp_agrees(done != 0);
 }
 // Shared-memory matrix descriptor, 128-byte swizzle, rows of 128 bytes in groups of 8
 // (1024 bytes).  lbo16: leading byte offset >> 4 (distance of 64-element panels for an

@@ -87,6 +87,10 @@ __device__ __forceinline__ bool slb_elected() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
     return yes != 0;
 }
+// What a warp made of its lanes' polls of a barrier, for waits that the whole warp enters: true if all of them saw the
+// phase.  Each lane polls up to its bound for itself; without this vote a bound that ran out in some lanes only would
+// send them out of the loop while the others wait for them at the next election, shuffle or collective load.
+__device__ __forceinline__ bool slb_warp_agrees(bool seen) { return __all_sync(0xffffffffu, seen); }
 // the index of this thread's warp, in a uniform register
 __device__ __forceinline__ int slb_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 

@@ -65,19 +65,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-// Bounded wait for the phase with the given parity; false after the poll limit.
+// Bounded wait for the phase with the given parity, entered by a whole warp: false in every lane if the polls of one
+// ran out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < SLB_TC_SPIN_LIMIT; ++i) {
-        uint32_t done;
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < SLB_TC_SPIN_LIMIT && !done; ++i)
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
+    return slb_warp_agrees(done != 0);
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
                                             int c0, int c1) {

@@ -1,0 +1,58 @@
+"""Bounded waits of the kernels, read from their sources: no GPU is made to run out of one."""
+
+import os
+import re
+
+import pytest
+
+from servelab_b200.csrc import build
+
+CSRC = os.path.dirname(build.__file__)
+# kernels whose roles go on with instructions that a whole warp executes (elections, shuffles, tensor memory)
+WARP_KERNELS = ["attention_tc.cu", "attention_kv_tc.cu", "attention_decode.cu", "gemm_rows.cu", "gemm_tcgen05.cu"]
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def body(text, at):
+    """The braces' contents from the first brace behind ``at`` on."""
+    start = text.index("{", at)
+    depth = 0
+    for i in range(start, len(text)):
+        depth += (text[i] == "{") - (text[i] == "}")
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError("no closing brace")
+
+
+def test_the_list_is_complete():
+    elected = [n for n in sorted(os.listdir(CSRC)) if n.endswith(".cu") and "slb_elected()" in source(n)]
+    assert set(elected) <= set(WARP_KERNELS)
+
+
+@pytest.mark.parametrize("name", WARP_KERNELS)
+def test_a_warp_gives_a_wait_up_as_one(name):
+    """A bound that runs out in some lanes only must not part them from the others, who would wait for them at the next
+    election or shuffle: the outcome of every wait is voted on, in the wait or around its call."""
+    text = source(name)
+    voted, plain = set(), {"mbar_wait"}                    # (mbar_wait of mma_util.cuh is a single thread's)
+    for m in re.finditer(r"__device__ __forceinline__ bool (\w+)\(uint64_t\* bar, uint32_t parity\)", text):
+        if re.search(r"return slb_warp_agrees\(done != 0\);\s*}$", body(text, m.end())):
+            assert body(text, m.end()).count("return") == 1
+            voted.add(m.group(1))
+        else:
+            plain.add(m.group(1))
+    plain -= voted
+    for m in re.finditer(r"\b(%s)\(&?\w" % "|".join(plain), text) if plain else ():
+        before = text[max(0, m.start() - 200):m.end()]
+        assert ("slb_warp_agrees(" + m.group(1) in before
+                or re.search(r"if \(tid == 0\)\s+for [^\n]*\s+\w+\(&\w$", before)), m.group(0)
+    assert voted or "slb_warp_agrees(mbar_wait" in text
+
+
+def test_the_vote_is_of_all_lanes():
+    text = source("common.cuh")
+    assert "__all_sync(0xffffffffu, seen)" in body(text, text.index("bool slb_warp_agrees("))
