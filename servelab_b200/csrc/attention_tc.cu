@@ -40,7 +40,8 @@
 // 1,500 22.4 -> 10.6.
 //
 // Every mbarrier wait is bounded; a role that gives up records a code in the status
-// word and leaves its loop; the block then frees its TMEM and returns without a result.
+// word and leaves its loop; the block then frees its TMEM and returns without a result, and so do the blocks that
+// share keys with it.
 //
 // Reference analogue: the torch loop over sequences (servelab/parallel/
 // tp_model.py:136-157); masking and softmax follow it (r <= a, optional window).
@@ -68,7 +69,8 @@ constexpr int OFF_K = OFF_Q + Q_BYTES;
 constexpr int OFF_V = OFF_K + 2 * KV_TILE_BYTES;
 constexpr int OFF_BAR = OFF_V + 2 * KV_TILE_BYTES;
 constexpr int OFF_ML = OFF_BAR + 128;          // a row's reference and sum, for the blocks that share its keys
-constexpr size_t TC_ATTN_SMEM = OFF_ML + BM * 8;
+constexpr int OFF_GAVE = OFF_ML + BM * 8;      // ... and whether this block gave up
+constexpr size_t TC_ATTN_SMEM = OFF_GAVE + 16;
 constexpr int MAX_SPLITS = 8;
 static_assert(OFF_BAR - OFF_K >= BM * D * 4, "the rings hold a block's partial result");
 constexpr uint32_t SPIN_LIMIT = 1u << 18;     // a poll that suspends takes about 4 us: about a second
@@ -269,6 +271,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             mbar_init(&pv_done[i], 1);
         }
         mbar_init(q_full, 1);
+        *reinterpret_cast<volatile int*>(smem + OFF_GAVE) = 0;
         mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
         mbar_init(&p_full[0], 128); mbar_init(&p_full[1], 128);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -481,10 +484,12 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             }
         } else {
             // This block's part of the result, for the other blocks of the row: columns of a thread's row side by side in the
-            // idle rings, and (reference, sum); a block without keys, or one that gave up, counts for nothing.
+            // idle rings, and (reference, sum); a block without keys counts for nothing, after one that gave up no block
+            // of the cluster has a result.
             float* part = reinterpret_cast<float*>(smem + OFF_K);
             float* ml = reinterpret_cast<float*>(smem + OFF_ML);
             const bool counts = ok && ntiles > 0;
+            if (!ok) *reinterpret_cast<volatile int*>(smem + OFF_GAVE) = 1;
             ml[r * 2] = counts ? m_ref : -INFINITY;
             ml[r * 2 + 1] = counts ? l : 0.f;
             if (ntiles > 0) {
@@ -508,7 +513,11 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             const float* part = reinterpret_cast<const float*>(smem + OFF_K);
             const float* ml = reinterpret_cast<const float*>(smem + OFF_ML);
             float m = -INFINITY, l = 0.f, w[MAX_SPLITS];
-            for (int k = 0; k < splits; ++k) m = fmaxf(m, cluster_float(ml + r * 2, k));
+            bool whole = true;                               // (no block's part is missing)
+            for (int k = 0; k < splits; ++k) {
+                m = fmaxf(m, cluster_float(ml + r * 2, k));
+                whole = whole && __float_as_int(cluster_float(reinterpret_cast<const float*>(smem + OFF_GAVE), k)) == 0;
+            }
 #pragma unroll
             for (int k = 0; k < MAX_SPLITS; ++k) {
                 w[k] = 0.f;
@@ -520,7 +529,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             const float inv = l > 0.f ? 1.f / l : 0.f;
             const int share = D / splits;                    // (a multiple of 8)
             bf16* dst = out + (size_t)(q0 + tok0 + tl) * ldo + (size_t)(kvh * g + hg) * D;
-            if (r < nrows) {
+            if (whole && r < nrows) {
                 for (int c = rank * share; c < (rank + 1) * share; c += 8) {
                     float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll

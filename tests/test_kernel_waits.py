@@ -53,6 +53,20 @@ def test_a_warp_gives_a_wait_up_as_one(name):
     assert voted or "slb_warp_agrees(mbar_wait" in text
 
 
+def test_a_cluster_whose_block_gave_up_stores_nothing():
+    """Blocks that share a tile's keys add their parts up: with one part missing the sum is no result.  The block that gave
+    up says so in a word of its own (not by the numbers of its part, which a block without keys leaves as well), every block
+    of the cluster reads all words behind the barrier, and stores only where none is set."""
+    text = source("attention_tc.cu")
+    assert re.search(r"mbar_init\(q_full, 1\);\s*\*reinterpret_cast<volatile int\*>\(smem \+ OFF_GAVE\) = 0;", text)
+    assert "if (!ok) *reinterpret_cast<volatile int*>(smem + OFF_GAVE) = 1;" in text
+    combine = text[text.index("if (splits > 1) {\n        __syncwarp();"):]
+    combine = combine[:combine.index("tcgen05.dealloc")]
+    assert re.search(r"for \(int k = 0; k < splits; \+\+k\) \{[^}]*whole = whole && [^;]*OFF_GAVE\), k\)\) == 0;", combine)
+    stores = [m.start() for m in re.finditer(r"reinterpret_cast<uint4\*>\(dst", combine)]
+    assert len(stores) == 1 and combine.index("if (whole && r < nrows) {") < stores[0]
+
+
 def test_the_vote_is_of_all_lanes():
     text = source("common.cuh")
     assert "__all_sync(0xffffffffu, seen)" in body(text, text.index("bool slb_warp_agrees("))
