@@ -332,9 +332,9 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
             for (int p = 0; p < PANELS_K; ++p)
                 slb_tma::tma_load_3d(smem + OFF_Q + p * (BM * 128), &map_q, q_full, amap * DK + p * 64, kvh * g, q0 + tok0);
         }
-        int row = lookup(0), st = 0;
+        int row = lookup(0), st = 0, asked = 0;
         uint32_t phase = 1;
-        for (int j = 0; j < ntiles; ++j) {
+        for (int j = 0; j < ntiles; ++j, ++asked) {
             const int next_row = lookup(j + 1);
             if (!mbar_wait(&freed[st], phase)) {
                 if (lane == 0) gave_up(status, keys ? 0x101 : 0x102, 0, j, ntiles);
@@ -370,6 +370,10 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
                 phase ^= 1;
             }
         }
+        // (after a wait that gave up copies may be in flight, which must not land in a later block's memory: the last of each
+        // stage is waited for; otherwise the MMAs have waited for them)
+        for (int t = max(0, asked - stages); t < asked; ++t) mbar_wait(&full[t % stages], (t / stages) & 1);
+        if (warp == 0) mbar_wait(q_full, 0);
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |

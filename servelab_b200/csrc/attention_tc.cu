@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             for (int p = 0; p < PANELS; ++p)
                 slb_tma::tma_load_3d(smem + OFF_Q + p * (BM * 128), &map_q, q_full, p * 64, kvh * g, q0 + tok0);
         }
-        int row = lookup(0);
-        for (int j = 0; j < ntiles; ++j) {
+        int row = lookup(0), asked = 0;
+        for (int j = 0; j < ntiles; ++j, ++asked) {
             const int st = j & 1;
             const int next_row = lookup(j + 1);
             if (!mbar_wait(&freed[st], ((j >> 1) & 1) ^ 1)) {
@@ -349,6 +349,10 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_tc_kernel(
             }
             row = next_row;
         }
+        // (after a wait that gave up copies may be in flight, which must not land in a later block's memory: the last of each
+        // stage is waited for; otherwise the MMAs have waited for them)
+        for (int t = max(0, asked - 2); t < asked; ++t) mbar_wait(&full[t & 1], (t >> 1) & 1);
+        if (keys && ntiles > 0) mbar_wait(q_full, 0);
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |

@@ -348,7 +348,8 @@ __global__ void __launch_bounds__(GR_THREADS, 1) gemm_rows_kernel(const __grid_c
                 }
             }
         }
-        if (!ok && rank == 0)                              // (gave up: the copies in flight first)
+        // (after a wait that gave up, the MMA issuer's as well, copies may be in flight; otherwise they have been waited for)
+        if (rank == 0)
             for (uint32_t j = it > (uint32_t)stages ? it - stages : 0; j < it; ++j)
                 mbar_wait(&full[j % stages], (j / stages) & 1);
     } else if (warp == 1) {

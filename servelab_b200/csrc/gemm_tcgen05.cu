@@ -274,9 +274,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_decode_kernel(
         for (int i = 0; i < ahead; ++i)
             if (slb_elected())
                 tma_load_2d(b_stage + i * B_STAGE_BYTES, &map_x, &full[i], (kb_begin + i) * TC_BK, tok_base);
-        int s = 0;
+        int s = 0, asked = ahead;
         uint32_t phase = 0;
-        for (int i = ahead; i < iters; ++i) {
+        for (int i = ahead; i < iters; ++i, ++asked) {
             if (!mbar_wait(&empty[s], phase)) {
                 atomicCAS(status, 0, (1 << 8) | 1);
                 break;
@@ -292,6 +292,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_decode_kernel(
                 phase ^= 1;
             }
         }
+        // (after a wait that gave up copies may be in flight; otherwise the MMA issuer has waited for them)
+        for (int i = max(0, asked - TC_STAGES); i < asked; ++i) mbar_wait(&full[i % TC_STAGES], (i / TC_STAGES) & 1);
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         // instruction descriptor: D float32, A and B bfloat16, both K-major
@@ -679,9 +681,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
         for (int i = 0; i < ahead; ++i)
             if (slb_elected())
                 tma_load_2d(b_stage + i * B_STAGE_BYTES, &map_x, &full[i], (kb_begin + i) * TC_BK, tok_base);
-        int s = 0;
+        int s = 0, asked = ahead;
         uint32_t phase = 0;
-        for (int i = ahead; i < iters; ++i) {
+        for (int i = ahead; i < iters; ++i, ++asked) {
             if (!mbar_wait(&empty[s], phase)) {
                 atomicCAS(status, 0, (1 << 8) | 2);
                 break;
@@ -697,6 +699,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_cluster_kernel(
                 phase ^= 1;
             }
         }
+        // (after a wait that gave up copies may be in flight; otherwise the MMA issuer has waited for them)
+        for (int i = max(0, asked - TC_STAGES); i < asked; ++i) mbar_wait(&full[i % TC_STAGES], (i / TC_STAGES) & 1);
         __syncwarp();
     } else if (warp == 1) {
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |

@@ -53,6 +53,19 @@ def test_a_warp_gives_a_wait_up_as_one(name):
     assert voted or "slb_warp_agrees(mbar_wait" in text
 
 
+@pytest.mark.parametrize("name", ["attention_tc.cu", "attention_kv_tc.cu", "gemm_rows.cu", "gemm_tcgen05.cu"])
+def test_a_loader_waits_for_the_copies_it_has_asked_for(name):
+    """Whichever role gives up, the block must not leave while copies into its shared memory are in flight: every loader ends
+    with a bounded wait for the last copy of each stage, on no condition but being the one that counts them."""
+    text = source(name)
+    loops = [m for m in re.finditer(r"if \(!mbar_wait\(&(?:empty|freed)\[\w+\]", text)]
+    ends = list(re.finditer(r"(if \(rank == 0\)\s*)?for \((?:int|uint32_t) \w+ = (?:max\(0, asked - \w+\)|it > [^;]*); \w+ < (?:asked|it); \+\+\w+\)"
+                            r"\s*mbar_wait\(&full\[", text))
+    assert len(loops) == len(ends) == (2 if name == "gemm_tcgen05.cu" else 1)
+    for a, b in zip(loops, ends):
+        assert a.start() < b.start() and "!ok" not in text[b.start() - 80:b.start()]
+
+
 def test_a_cluster_whose_block_gave_up_stores_nothing():
     """Blocks that share a tile's keys add their parts up: with one part missing the sum is no result.  The block that gave
     up says so in a word of its own (not by the numbers of its part, which a block without keys leaves as well), every block
