@@ -1323,7 +1323,7 @@ moe_tensor_cores = True        # bfloat16: the experts' products on mma.sync (of
 
 def _gather_rows(x: torch.Tensor, plan: torch.Tensor, E: int, P: int, top: int) -> torch.Tensor:
     """The rows of ``x`` in the order of the plan's list of pairs [P, h]."""
-    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+    if x.stride(0) % 8 or x.data_ptr() % 16:
         x = x.clone(memory_format=torch.contiguous_format)
     xs = torch.empty((P, x.shape[1]), dtype=x.dtype, device=x.device)
     L.check(L.core().slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, x.shape[1],
@@ -1361,6 +1361,8 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     n_out = w_down.shape[1]
     P = T * top
     lib = L.core()
+    if x.stride(1) != 1:                                   # (the products read a row's elements as neighbours)
+        x = x.clone(memory_format=torch.contiguous_format)
     vendor = (x.dtype == _BF16 and moe_vendor_grouped and P >= moe_vendor_min_pairs
               and h * inter >= moe_vendor_min_expert_elements and h % 8 == 0
               and inter % 8 == 0 and n_out % 8 == 0 and hasattr(torch, "_grouped_mm"))

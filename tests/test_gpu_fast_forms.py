@@ -247,6 +247,20 @@ def test_router_logits_of_many_tokens(M, E, Kd):
     assert (K().router_logits(x, w).double() - want).norm() <= 1e-6 * want.norm()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,h,I", [(3, 64, 40), (70, 200, 64), (5, 1024, 512)])
+def test_small_steps_of_the_experts_take_rows_of_any_stride(T, h, I, dtype):
+    """Every second column, and a transposed matrix: the same bits as their copies, in each form of the products."""
+    g, E, top = gen(T), 4, 2
+    x = torch.randn(T, 2 * h, device=DEV, generator=g).to(dtype)
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).to(dtype) for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    w = torch.rand(T, top, device=DEV, generator=g)
+    for view in (x[:, ::2], x[:, :h].T.contiguous().T):
+        assert view.stride(1) != 1
+        assert torch.equal(K().moe_experts(view, ids, w, wg, wd, None), K().moe_experts(view.contiguous(), ids, w, wg, wd, None))
+
+
 def test_large_steps_of_the_experts_take_rows_of_any_stride():
     """Every second column of a wider matrix: the library's products took such rows, and so must the steps that read
     them themselves."""
