@@ -905,11 +905,11 @@ def gemm_tc_resid_dyt(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, pos
 
 # ------------------------------------ tcgen05 products of a feed-forward over many tokens
 def gemm_rows_gated_takes(x: torch.Tensor, w: torch.Tensor, block: int) -> bool:
-    """The product with the gated activation in its epilogue: bfloat16 rows of whole 16-byte pieces, gates then ups
-    (``block`` 0, a multiple of 16 of each) or alternating in runs of 64."""
+    """The product with the gated activation in its epilogue: bfloat16 rows of whole 16-byte pieces that do not overlap
+    (a broadcast row goes to the library), gates then ups (``block`` 0, a multiple of 16 of each) or alternating in runs of 64."""
     inter = w.shape[0] // 2
     return (x.dtype == _BF16 and w.dtype == _BF16 and x.shape[0] > 0 and w.stride(1) == 1 and x.stride(1) == 1
-            and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
             and w.data_ptr() % 16 == 0 and block in (0, SWIGLU_BLOCK) and inter % (block or 16) == 0)
 
 

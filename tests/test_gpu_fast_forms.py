@@ -577,6 +577,20 @@ def test_gated_product_of_many_tokens(T, I, Kd, block, nt, act):
     assert (got - want).norm() <= 2.5e-3 * want.norm() and K().gemm_rows_status() == 0
 
 
+@pytest.mark.parametrize("T", [129, 300])
+@pytest.mark.parametrize("block", [0, 64])
+def test_gated_linear_takes_rows_that_overlap(T, block):
+    """A broadcast row and rows 8 elements apart: what their copies give, to the rounding of a second kernel (gate and up
+    rounded to bfloat16 first, 2^-8 of the norm)."""
+    from servelab_b200.ops import linear
+    g = gen(T)
+    buf, w = torch.randn(8 * T + 512, device=DEV, generator=g).bfloat16(), (torch.randn(2048, 512, device=DEV, generator=g) * 0.04).bfloat16()
+    assert K().gemm_rows_gated_pays(T, 1024, 512)
+    for x in (buf[:512].expand(T, 512), buf.as_strided((T, 512), (8, 1))):
+        got, want = linear.gated_linear(x, w, block), linear.gated_linear(x.contiguous(), w, block)
+        assert (got.double() - want.double()).norm() <= 2.0 ** -8 * want.double().norm()
+
+
 @pytest.mark.parametrize("counts", [[0, 1, 300, 33], [256, 257, 0, 17, 513, 1, 2, 31], [700, 2400, 5], [0, 0, 1]])
 @pytest.mark.parametrize("weighted", [False, True])
 def test_experts_products_over_sorted_rows(counts, weighted):
