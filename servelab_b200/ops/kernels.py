@@ -1377,8 +1377,8 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     L.check(getattr(lib, "slb_moe_plan" + form)(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
     if own:
         # Rows sorted by expert, each expert's in tiles of up to 256; a token's results are summed where the second
-        # product left them: in float32, in the steps of many rows of large experts in bfloat16 (their way through
-        # memory is what they cost: 67 MB for 8,192 rows of 2,048).
+        # product left them: in bfloat16 where the vendor's grouped product would leave them so (their way through
+        # memory is what they cost: 67 MB for 8,192 rows of 2,048), else in float32 as the other products do.
         at = plan.numel() - 2 * P
         order = plan[at:at + P]
         xs = _gather_rows(x, plan, E, P, top)
@@ -1388,13 +1388,12 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
             xs.data_ptr(), h, w_gate_up.data_ptr(), h, act.data_ptr(), inter, offsets, E, P, inter, h, 1, 0, *act_args,
             _p(weights if weight_inputs else None), order.data_ptr() if weight_inputs else None, _stream()),
             "gemm_rows_experts")
-        half = P >= moe_vendor_min_pairs and h * inter >= moe_vendor_min_expert_elements
-        ys = torch.empty((P, n_out), dtype=_BF16 if half else _F32, device=x.device)
+        ys = torch.empty((P, n_out), dtype=_BF16 if vendor else _F32, device=x.device)
         L.check(lib.slb_gemm_rows_experts_bf16(
             act.data_ptr(), inter, w_down.data_ptr(), inter, ys.data_ptr(), n_out, offsets, E, P, n_out, inter, 0,
-            0 if half else 1, 0, 0.0, 0.0, None, None, _stream()), "gemm_rows_experts")
+            0 if vendor else 1, 0, 0.0, 0.0, None, None, _stream()), "gemm_rows_experts")
         out = torch.empty((T, n_out), dtype=x.dtype, device=x.device)
-        combine = lib.slb_moe_combine_bf16_sorted if half else lib.slb_moe_combine_bf16_sorted_f32
+        combine = lib.slb_moe_combine_bf16_sorted if vendor else lib.slb_moe_combine_bf16_sorted_f32
         L.check(combine(ys.data_ptr(), n_out, _p(out_weights), _p(shared), shared.stride(0) if shared is not None else 0,
                         out.data_ptr(), out.stride(0), plan.data_ptr(), E, T, top, n_out, _stream()), "moe_combine")
         return out

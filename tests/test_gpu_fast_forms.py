@@ -648,6 +648,27 @@ def test_routed_experts_on_sorted_rows(T, E, top, h, I, half):
     assert (got - want).norm() <= 6e-3 * want.norm()
 
 
+def test_rows_of_an_expert_are_rounded_only_where_the_library_rounds_them(monkeypatch):
+    """Large steps of large experts with the library's grouped product switched off, and a result of 2,044 columns, which it
+    does not take: the experts' rows are float32 until a token's sum, as they are in the other products."""
+    g = gen(9)
+    T, E, top, h, I = 512, 4, 2, 1024, 2048
+    x = torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    wg = (torch.randn(E, 2 * I, h, device=DEV, generator=g) * h ** -0.5).bfloat16()
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    w, asked = torch.rand(T, top, device=DEV, generator=g), []
+    from servelab_b200.ops import library as L
+    lib = L.core()
+    real = lib.slb_gemm_rows_experts_bf16
+    monkeypatch.setattr(lib, "slb_gemm_rows_experts_bf16", lambda *a: asked.append(a[11:13]) or real(*a))
+    for grouped, n_out, f32 in ((True, 1024, 0), (False, 1024, 1), (True, 1020, 1)):
+        wd = (torch.randn(E, n_out, I, device=DEV, generator=g) * I ** -0.5).bfloat16()
+        monkeypatch.setattr(K(), "moe_vendor_grouped", grouped)
+        asked.clear()
+        K().moe_experts(x, ids, w, wg, wd, None)
+        assert asked == [(1, 0), (0, f32)]
+
+
 @pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (5, 1, 1, 5), (32, 4, 2, 4), (60, 3, 2, 6), (100, 1, 1, 32), (128, 32, 9, 8),
                                                (128, 2, 1, 3)])
 @pytest.mark.parametrize("score_fn", ["softmax", "sigmoid"])
