@@ -41,6 +41,18 @@ def _align4(n: int) -> int:
     return (n + 3) & ~3
 
 
+# Context lengths at which launch shapes of a step with prompt portions change, coarse, so that few graphs are captured
+# for one padded size.  The prompt attention shares the keys of a tile from 12 to 22 key tiles of 64 on where blocks are few and
+# from 24 to 32 where the SMs are then shared (``ops.kernels.prefill_splits``): nothing below 1,024 tokens, where the gain is
+# 5 % at most, everything from 2,048 on.
+CONTEXT_CLASSES = (0, 1024, 2048)
+
+
+def context_class(longest: int) -> int:
+    """The largest class that a step's longest context reaches."""
+    return max(c for c in CONTEXT_CLASSES if c <= longest)
+
+
 class StepContext:
     """Device-side view of a step plus a few host-side facts about it."""
 
@@ -264,7 +276,8 @@ class StepContext:
         ctx._host = host
         ctx.q_lens, ctx.state_slot_ids = inner.q_lens, inner.state_slot_ids
         ctx.ctx_lens, ctx.max_ctx_len = inner.ctx_lens, inner.max_ctx_len
-        ctx.split_hint_len = inner.max_ctx_len
+        # (launch shapes are kept with the graph: they follow from the class, as the graph's key does)
+        ctx.split_hint_len = context_class(inner.max_ctx_len)
         ctx.decode_only = False
         ctx.real_sizes = (T, S, R)
         for key in ctx._padded_tiles:                       # the work lists of the kernels that asked

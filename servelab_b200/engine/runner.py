@@ -26,7 +26,7 @@ from ..models.causal_lm import CausalLM
 from ..ops import kernels as K
 from ..parts import BuildEnv
 from ..weights.source import FolderSource, WeightSource
-from .batch import BatchEntry, StepContext
+from .batch import BatchEntry, StepContext, context_class
 
 _DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 
@@ -102,8 +102,8 @@ class ModelRunner:
         self.max_portion_graph_tokens = 2048
         self.max_portion_graphs = 24
         self.portion_graph_after = 2      # times a shape is asked for before it is captured
-        self._portion_graphs = {}         # padded sizes -> (graph, context, logits)
-        self._portion_seen = {}           # padded sizes -> times asked for
+        self._portion_graphs = {}         # padded sizes, context class -> (graph, context, logits)
+        self._portion_seen = {}           # the same -> times asked for
         self.portion_graph_replays = 0
         self._table_rows = {}             # (request, group) -> (stamp, block table as int32 array)
         # through a weak reference: the cache manager must not keep the runner alive in a
@@ -169,8 +169,9 @@ class ModelRunner:
                 and (not self.storage.state_layers or self._padded_state_safe)):
             pad = self._portion_pad(entries)
             if pad is not None:
-                hit = self._portion_graphs.get(pad)
-                seen = self._portion_seen[pad] = self._portion_seen.get(pad, 0) + 1
+                key = self._portion_key(entries, pad)
+                hit = self._portion_graphs.get(key)
+                seen = self._portion_seen[key] = self._portion_seen.get(key, 0) + 1
                 if hit is not None or seen >= self.portion_graph_after:
                     return self._step_portion_graph(entries, pad)
         ctx = StepContext.pack(entries, self.num_groups, self.device)
@@ -196,12 +197,19 @@ class ModelRunner:
         Rp = 1 << (R - 1).bit_length() if R else 0
         return Tp, Sp, Rp
 
+    @staticmethod
+    def _portion_key(entries: List[BatchEntry], pad):
+        """What a step's graph is kept under: its padded sizes and the class of its longest context, so that launch
+        shapes and the order of sums are the step's own and not those of the step that was captured first."""
+        return pad + (context_class(max(e.start + len(e.tokens) for e in entries)),)
+
     def _step_portion_graph(self, entries: List[BatchEntry], pad) -> torch.Tensor:
-        """A step of any composition through the graph captured for its padded sizes.  The
+        """A step of any composition through the graph captured for its padded sizes and context class.  The
         returned logits live in the graph's memory until its next replay."""
         width = -(-self.max_model_len // self.page_size)
         R = sum(len(e.want) for e in entries)
-        hit = self._portion_graphs.pop(pad, None)
+        key = self._portion_key(entries, pad)
+        hit = self._portion_graphs.pop(key, None)
         if hit is None:
             ctx = StepContext.pack(entries, self.num_groups, self.device, min_table_width=width, pad=pad)
             # (the warm-up runs the step and the first replay runs it again: keys land in the same
@@ -226,7 +234,7 @@ class ModelRunner:
             while len(self._portion_graphs) >= self.max_portion_graphs:
                 self._portion_graphs.pop(next(iter(self._portion_graphs)))
         graph, ctx, logits = hit
-        self._portion_graphs[pad] = hit                     # (most recently used last)
+        self._portion_graphs[key] = hit                     # (most recently used last)
         StepContext.pack(entries, self.num_groups, self.device, min_table_width=width, into=ctx, pad=pad)
         graph.replay()
         self.portion_graph_replays += 1

@@ -479,7 +479,9 @@ def prefill_splits(units: int, longest_context: int, window: int, head_dim: int)
     us with 1 / 2 / 4 / 8 blocks, units (tiles of rows x kv heads), key tiles: 14 heads of 64, 34, 5 8.2 / 9.6 / 9.4 / 17.3;
     40, 11 11.4 / 11.1 / 11.2 / 19.1; 78, 11 12.0 / 12.3 / 18.3 / 29.9; 112, 15 14.8 / 15.4 / 21.6 / 40.1; 42, 33 25.8 / 18.4
     / 16.6 / 21.1; 8, 17 15.4 / 13.3 / 11.4 / 10.6; 28 heads of 128, 80, 11 12.1 / 15.5 / 23.9 / 37.2; 84, 33 28.1 / 26.8 /
-    27.0 / 38.7; 16, 17 17.6 / 16.7 / 13.9 / 14.4; 12, 32 24.8 / 19.3 / 14.8 / 13.1."""
+    27.0 / 38.7; 16, 17 17.6 / 16.7 / 13.9 / 14.4; 12, 32 24.8 / 19.3 / 14.8 / 13.1.  Steps that are replayed as graphs
+    name the class of their longest context (and the bound of their tiles, empty ones among them): the choice is kept
+    with the graph."""
     if prefill_force_splits:
         return prefill_force_splits
     seen = min(longest_context, window + 63) if window > 0 else longest_context

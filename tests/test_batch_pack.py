@@ -8,7 +8,8 @@ import random
 import pytest
 import torch
 
-from servelab_b200.engine.batch import BatchEntry, StepContext
+from servelab_b200.engine.batch import BatchEntry, StepContext, context_class
+from servelab_b200.engine.runner import ModelRunner
 
 
 def expected(entries, num_groups, min_width):
@@ -111,8 +112,26 @@ def test_padded_contexts_fresh_and_overwritten(seed):
                     for r0 in range(0, len(e.tokens) * group_size, rows_per_tile)]
             got = list(zip(tile_seq.tolist(), tile_row0.tolist()))
             assert got[:len(want)] == want and all(t == (7, 0) for t in got[len(want):])
+        assert ctx.split_hint_len == context_class(max(e.start + len(e.tokens) for e in entries))
     with pytest.raises(ValueError):
         StepContext.pack(entries, groups, "cpu", min_table_width=width, pad=(512, len(entries), 32))
+
+
+@pytest.mark.parametrize("first,then", [(100, 2100), (2100, 100), (1500, 700), (1023, 1024)])
+def test_launch_shapes_of_a_padded_step_do_not_hang_on_the_step_before(first, then):
+    """A graph is captured with the hint of its context and replayed for other steps: steps of the same padded sizes
+    whose contexts are of two classes have graphs of their own, and the hint is the class, not the captured length."""
+    def step(past):
+        return [BatchEntry(tokens=[1] * 40, start=past, want=(39,), block_tables=[list(range(200))])]
+    pad, keys, hints = (64, 2, 1), [], []
+    for past in (first, then):
+        keys.append(ModelRunner._portion_key(step(past), pad))
+        hints.append(StepContext.pack(step(past), 1, "cpu", min_table_width=200, pad=pad).split_hint_len)
+        assert keys[-1][:3] == pad and hints[-1] == keys[-1][3] == context_class(past + 40) <= past + 40
+        ctx = StepContext.pack(step(first), 1, "cpu", min_table_width=200, pad=pad)
+        StepContext.pack(step(past), 1, "cpu", min_table_width=200, pad=pad, into=ctx)
+        assert ctx.split_hint_len == hints[-1]
+    assert (keys[0] == keys[1]) == (context_class(first + 40) == context_class(then + 40)) == (hints[0] == hints[1])
 
 
 def test_entries_without_stamps_and_empty_want():

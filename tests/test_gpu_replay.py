@@ -123,6 +123,33 @@ def test_steps_with_portions_replayed_as_padded_graphs(model, dtype):
                 assert np.array_equal(got[rid][pos], eager[rid][pos]), (rid, pos)
 
 
+def test_a_portion_replays_the_same_whichever_was_captured_first(tmp_path, monkeypatch):
+    """Steps of one padded size at a short and a long context, in both orders of capture: the same bits, and blocks share
+    a tile's keys at the long context only (one kv head and few tiles: 8 blocks)."""
+    from servelab_b200.config import CacheConfig
+    from servelab_b200.engine.runner import ModelRunner
+    from servelab_b200.ops import kernels as K
+    cfg = dict(H.TINY_E, max_position_embeddings=2560)
+    folder = H.make_model(str(tmp_path), cfg, 3, std_of=H.PEAKED)
+    chosen, rule, got = [], K.prefill_splits, {}
+    monkeypatch.setattr(K, "prefill_splits", lambda *a: chosen.append(rule(*a)) or chosen[-1])
+    for order in ((100, 2300), (2300, 100)):
+        runner = ModelRunner.from_folder(folder, dtype="bfloat16", cache_config=CacheConfig(block_size=16, num_blocks=170),
+                                         max_num_seqs=2, cuda_graphs=True)
+        runner.portion_graph_after = 1
+        assert all(runner.cache.open(str(p)) and runner.cache.ensure(str(p), p + 40) for p in (100, 2300))
+        for cache in runner.storage.layer_caches.values():
+            for t in (cache.k, cache.v):
+                t.copy_(torch.randn(t.shape, device=t.device, generator=torch.Generator(t.device).manual_seed(5)))
+        for past in order + order:
+            chosen.clear()
+            out = runner.step([runner.entry(str(past), [7] * 40, past, (39,))]).clone()
+            assert not chosen or set(chosen) == {8 if past > 2000 else 1}
+            assert torch.equal(out, got.setdefault(past, out)) and out.isfinite().all()
+        assert len(runner._portion_graphs) == 2 and runner.portion_graph_replays == 4
+    assert K.prefill_attention_tc_status(128) == 0
+
+
 def test_float32_cut_invariance(model):
     """In float32 the logits of a position are bit-identical however the tokens are cut."""
     a = _check(model, "float32", H.trace_whole(model["requests"]))
