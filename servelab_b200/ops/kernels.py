@@ -1323,29 +1323,27 @@ moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this ma
 moe_tensor_cores = True        # bfloat16: the experts' products on mma.sync (off: CUDA cores, the twin)
 
 
-def _gather_rows(x: torch.Tensor, plan: torch.Tensor, E: int, P: int, top: int) -> torch.Tensor:
-    """The rows of ``x`` in the order of the plan's list of pairs [P, h]."""
-    if x.stride(0) % 8 or x.data_ptr() % 16:
-        x = x.clone(memory_format=torch.contiguous_format)
-    xs = torch.empty((P, x.shape[1]), dtype=x.dtype, device=x.device)
-    L.check(L.core().slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, x.shape[1],
-                                         xs.data_ptr(), xs.stride(0), _stream()), "moe_gather")
-    return xs
+def _rows_in_pieces(x: torch.Tensor) -> torch.Tensor:
+    """``x``, or a copy of it where its rows are no whole 16-byte pieces."""
+    return x.clone(memory_format=torch.contiguous_format) if x.stride(0) % 8 or x.data_ptr() % 16 else x
 
 
 moe_tcgen05 = True             # bfloat16: the experts' products on tcgen05 (off: the vendor's or mma.sync)
 moe_tcgen05_max_experts = 1024
 
 
-def moe_tcgen05_pays(pairs: int, experts: int, elements: int) -> bool:
-    """Whether they are ahead of the others (``elements``: of one matrix of an expert).  Always for large experts; for
-    others from some rows an expert on, since a list of rows and one launch more come with them.  us, others / tcgen05:
-    32 of 2,048 x 1,408, 4 a token, 1 / 16 / 64 / 250 / 2,048 tokens 39 / 97 / 111 / 173 / 210, 29 / 99 / 103 / 109 / 179; 128
-    of 2,048 x 768, 8 a token, 2 / 4 / 8 / 64 / 512 tokens 47 / 65 / 107 / 236 / 348, 49 / 68 / 91 / 201 / 226; 64 of 1,024 x
-    512, 8 a token, 16 / 64 / 128 / 2,048 tokens 45 / 50 / 72 / 302, 52 / 54 / 55 / 119.  Experts smaller than that stay with
-    one kernel for steps of any size (8 of 512 x 256, 2 a token, 64 / 512 tokens 20 / 32, 19 / 25): its sums are the same
-    whatever the step, and in so small a model a router's choice hangs on them."""
-    return elements >= 1 << 21 or elements >= 1 << 19 and (pairs >= 16 * experts or elements >= 1 << 20 and pairs >= 64)
+def moe_tcgen05_pays(elements: int) -> bool:
+    """Whether experts of this many elements a matrix take them, in steps of any size: a row's sums are the same bits in
+    every tile, so that a token's result (and the next router's choice, where it is a near tie) does not hang on how many
+    others the step has, as it would with a line by the rows an expert.  us, others / tcgen05: 32 of 2,048 x 1,408, 4 a token,
+    1 / 16 / 64 / 250 / 2,048 tokens 39 / 97 / 111 / 173 / 210, 29 / 99 / 103 / 109 / 179; 1 / 4 / 8 / 32 / 256 / 1,024 tokens of
+    128 of 2,048 x 768, 8 a token, 37 / 70 / 110 / 195 / 255 / 484, 31 / 71 / 102 / 172 / 214 / 248; 32 of 1,024 x 1,024, 4 a
+    token, 25 / 33 / 39 / 53 / 78 / 176, 23 / 34 / 45 / 51 / 55 / 67; 16 of 1,024 x 768, 4 a token, 24 / 26 / 37 / 39 / 61 / 135, 23
+    / 25 / 31 / 32 / 36 / 53; 64 of 1,024 x 512, 8 a token, 24 / 30 / 39 / 50 / 81 / 176, 23 / 35 / 44 / 54 / 59 / 79 (what a
+    list of rows and one launch more cost shows at 4 to 64 tokens); 16 of 1,024 x 512, 2 a token, 21 / 23 / 24 / 33 / 36 / 67,
+    21 / 22 / 22 / 25 / 26 / 33.  Smaller ones stay with the other kernel (8 of 512 x 256, 2 a token, 64 / 512 tokens 20 / 32,
+    19 / 25)."""
+    return elements >= 1 << 19
 
 
 def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor,
@@ -1372,33 +1370,38 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     mma = (x.dtype == _BF16 and moe_tensor_cores and h % 8 == 0 and inter % 8 == 0 and n_out % 2 == 0
            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
     own = (x.dtype == _BF16 and moe_tcgen05 and moe_tensor_cores and 0 < P and E <= moe_tcgen05_max_experts and h % 8 == 0
-           and inter % 16 == 0 and n_out % 4 == 0 and moe_tcgen05_pays(P, E, h * inter)
+           and inter % 16 == 0 and n_out % 4 == 0 and moe_tcgen05_pays(h * inter)
            and all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (w_gate_up, w_down)))
-    form = "" if own or vendor or mma else "_simt"         # (the tiles' rows differ)
-    plan = torch.empty(getattr(lib, f"slb_moe_plan{form}_ints")(P, E), dtype=torch.int32, device=x.device)
-    L.check(getattr(lib, "slb_moe_plan" + form)(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
     if own:
         # Rows sorted by expert, each expert's in tiles of up to 256; a token's results are summed where the second
         # product left them: in bfloat16 where the vendor's grouped product would leave them so (their way through
         # memory is what they cost: 67 MB for 8,192 rows of 2,048), else in float32 as the other products do.
-        at = plan.numel() - 2 * P
-        order = plan[at:at + P]
-        xs = _gather_rows(x, plan, E, P, top)
-        act = torch.empty((P, inter), dtype=x.dtype, device=x.device)
-        offsets = plan.data_ptr() + 4 * E
-        L.check(lib.slb_gemm_rows_experts_bf16(
-            xs.data_ptr(), h, w_gate_up.data_ptr(), h, act.data_ptr(), inter, offsets, E, P, inter, h, 1, 0, *act_args,
-            _p(weights if weight_inputs else None), order.data_ptr() if weight_inputs else None, _stream()),
-            "gemm_rows_experts")
-        ys = torch.empty((P, n_out), dtype=_BF16 if vendor else _F32, device=x.device)
-        L.check(lib.slb_gemm_rows_experts_bf16(
-            act.data_ptr(), inter, w_down.data_ptr(), inter, ys.data_ptr(), n_out, offsets, E, P, n_out, inter, 0,
-            0 if vendor else 1, 0, 0.0, 0.0, None, None, _stream()), "gemm_rows_experts")
+        # (one allocation for the plan and the rows between the launches: an eager step of a small model is bound by the
+        # host, and an allocation is 2 us of it)
+        x, ints, stream = _rows_in_pieces(x), lib.slb_moe_plan_ints(P, E), _stream()
+        ends, total = [], 0
+        for n in (4 * ints, 2 * P * h, 2 * P * inter, (2 if vendor else 4) * P * n_out):
+            total += -(-n // 256) * 256
+            ends.append(total)
+        work = torch.empty(total, dtype=torch.uint8, device=x.device)
         out = torch.empty((T, n_out), dtype=x.dtype, device=x.device)
+        plan = work.data_ptr()
+        offsets, order, xs, act, ys = plan + 4 * E, plan + 4 * (ints - 2 * P), *(plan + e for e in ends[:3])
+        L.check(lib.slb_moe_plan(ids.data_ptr(), P, E, plan, stream), "moe_plan")
+        L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan, E, P, top, h, xs, h, stream), "moe_gather")
+        L.check(lib.slb_gemm_rows_experts_bf16(
+            xs, h, w_gate_up.data_ptr(), h, act, inter, offsets, E, P, inter, h, 1, 0, *act_args,
+            weights.data_ptr() if weight_inputs else None, order if weight_inputs else None, stream), "gemm_rows_experts")
+        L.check(lib.slb_gemm_rows_experts_bf16(
+            act, inter, w_down.data_ptr(), inter, ys, n_out, offsets, E, P, n_out, inter, 0, 0 if vendor else 1, 0, 0.0, 0.0,
+            None, None, stream), "gemm_rows_experts")
         combine = lib.slb_moe_combine_bf16_sorted if vendor else lib.slb_moe_combine_bf16_sorted_f32
-        L.check(combine(ys.data_ptr(), n_out, _p(out_weights), _p(shared), shared.stride(0) if shared is not None else 0,
-                        out.data_ptr(), out.stride(0), plan.data_ptr(), E, T, top, n_out, _stream()), "moe_combine")
+        L.check(combine(ys, n_out, _p(out_weights), _p(shared), shared.stride(0) if shared is not None else 0,
+                        out.data_ptr(), out.stride(0), plan, E, T, top, n_out, stream), "moe_combine")
         return out
+    form = "" if vendor or mma else "_simt"                # (the tiles' rows differ)
+    plan = torch.empty(getattr(lib, f"slb_moe_plan{form}_ints")(P, E), dtype=torch.int32, device=x.device)
+    L.check(getattr(lib, "slb_moe_plan" + form)(ids.data_ptr(), P, E, plan.data_ptr(), _stream()), "moe_plan")
     if vendor:
         # Large steps: the vendor's grouped product over the rows sorted by expert (the plan's list
         # and offsets stay on the device), as the dense products of large steps go to the vendor's
@@ -1407,7 +1410,10 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         at = plan.numel() - 2 * P
         ends = plan[E + 1:2 * E + 1]                                   # cumulative row counts
         order = plan[at:at + P]                                        # pairs sorted by expert
-        xs = _gather_rows(x, plan, E, P, top)
+        x = _rows_in_pieces(x)
+        xs = torch.empty((P, h), dtype=x.dtype, device=x.device)
+        L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan.data_ptr(), E, P, top, h, xs.data_ptr(),
+                                        xs.stride(0), _stream()), "moe_gather")
         gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
         mark("library grouped gemm")
         act = torch.empty((P, inter), dtype=x.dtype, device=x.device)

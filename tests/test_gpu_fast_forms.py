@@ -638,7 +638,7 @@ def test_routed_experts_on_sorted_rows(T, E, top, h, I, half):
     wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
     ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
     w, shared = torch.rand(T, top, device=DEV, generator=g), torch.randn(T, h, device=DEV, generator=g).bfloat16()
-    assert K().moe_tcgen05_pays(T * top, E, h * I) and half == (T * top >= K().moe_vendor_min_pairs)
+    assert K().moe_tcgen05_pays(h * I) and half == (T * top >= K().moe_vendor_min_pairs)
     got = K().moe_experts(x, ids, w, wg, wd, shared).double()
     want = shared.double()
     for e in range(E):
@@ -667,6 +667,18 @@ def test_rows_of_an_expert_are_rounded_only_where_the_library_rounds_them(monkey
         asked.clear()
         K().moe_experts(x, ids, w, wg, wd, None)
         assert asked == [(1, 0), (0, f32)]
+
+
+@pytest.mark.parametrize("E,h,I,top", [(16, 1024, 512, 2), (64, 1024, 512, 8), (16, 1024, 768, 4), (8, 1024, 1024, 4), (8, 512, 256, 2)])
+def test_a_token_of_routed_experts_does_not_hang_on_the_step(E, h, I, top):
+    """Experts below the library's sizes: a token's result is the same bits alone, among a few and in a large step."""
+    g, T = gen(E + I), 400
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    x, w = torch.randn(T, h, device=DEV, generator=g).bfloat16(), torch.rand(T, top, device=DEV, generator=g)
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    whole = K().moe_experts(x, ids, w, wg, wd, None)
+    for n in (1, 3, 17, 64, 150):
+        assert torch.equal(K().moe_experts(x[:n], ids[:n], w[:n], wg, wd, None), whole[:n])
 
 
 @pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (5, 1, 1, 5), (32, 4, 2, 4), (60, 3, 2, 6), (100, 1, 1, 32), (128, 32, 9, 8),
