@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) gemm_rows_kernel(const __grid_c
                             gv *= wt;
                             uv *= wt;
                         }
-                        r[m] = act_mul_fast<ACT>(gv, uv, a.limit, a.alpha);
+                        r[m] = act_mul_sums<ACT>(gv, uv, a.limit, a.alpha);
                     }
                     bf16* dst = static_cast<bf16*>(a.out) + (size_t)(t.tok + c + 2 * p + up) * a.ldo + f4;
 #pragma unroll

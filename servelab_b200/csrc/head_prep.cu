@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const T* __restrict__
     const size_t t = blockIdx.x;
     for (int c = threadIdx.x; c < N; c += blockDim.x) {
         const float z = to_float(gate[t * ldg + c / group]);
-        out[t * ldo + c] = from_float<T>(sizeof(T) == 2 ? to_float(x[t * ldx + c]) * sigmoid_for<T>(z) : to_float(x[t * ldx + c]) / (1.0f + expf(-z)));
+        const float v = to_float(x[t * ldx + c]);
+        out[t * ldo + c] = from_float<T>(sizeof(T) == 2 ? v * sigmoid_for<T>(z) : v / (1.0f + expf(-z)));
     }
 }
 

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(128) group_norm_gate_kernel(
 // a thread keeps GGN_NV vectors of V elements in registers, longer parts are formed again.
 #define GGN_THREADS 256
 #define GGN_NV 4
+// (T: of a result that is rounded at once; float where the gated value is squared and summed)
 template <typename T> __device__ __forceinline__ float gated_by(float x, float z, int gate_act) {
     const float sg = sigmoid_for<T>(z);
     return x * (gate_act == 2 ? z * sg : sg);
@@ -200,13 +201,13 @@ __global__ void __launch_bounds__(GGN_THREADS) gate_group_norm_kernel(
         if (c < size) {
 #pragma unroll
             for (int e = 0; e < V; ++e) {
-                v[j][e] = gated_by<T>(v[j][e], z[j][e], gate_act);
+                v[j][e] = gated_by<float>(v[j][e], z[j][e], gate_act);
                 ss += v[j][e] * v[j][e];
             }
         }
     }
     for (int c = threadIdx.x + GGN_NV * V * blockDim.x; c < size; c += blockDim.x) {
-        const float u = gated_by<T>(xr[c], to_float(gr[c]), gate_act);
+        const float u = gated_by<float>(xr[c], to_float(gr[c]), gate_act);
         ss += u * u;
     }
     const float rstd = factor / sqrtf(block_sum(ss, scratch) / (float)size + eps);
@@ -222,14 +223,15 @@ __global__ void __launch_bounds__(GGN_THREADS) gate_group_norm_kernel(
         }
     }
     for (int c = threadIdx.x + GGN_NV * V * blockDim.x; c < size; c += blockDim.x)
-        o[c] = from_float<T>(gated_by<T>(xr[c], to_float(gr[c]), gate_act) * rstd * (w != nullptr ? w[c0 + c] : 1.f));
+        o[c] = from_float<T>(gated_by<float>(xr[c], to_float(gr[c]), gate_act) * rstd * (w != nullptr ? w[c0 + c] : 1.f));
 }
 
 // Both orders of norm and gate for parts of whole 16-byte pieces up to 1,024 elements: a warp a (token, part) with
 // the part in registers, all loads issued together, no block-wide sum to wait for.  What bounds it is memory
 // (float32 row in, gate in, row out) and the gate's exponentials.  Norm then gate, a warp that reads element by
 // element and twice against this: 2,048 tokens of 8 x 256 11.4 -> 8.7 us, of 16 x 128 14.1 -> 10.8.  (The approximate
-// reciprocal for bfloat16 results: 2,912 tokens of 4 x 512 10.1 -> 8.0, 2,048 of 16 x 128 10.3 -> 9.7.)
+// reciprocal for gates behind the norm and bfloat16 results: 2,048 of 16 x 128 10.3 -> 9.5.  Gates before the norm enter
+// its sum and have the full exponential and division: 2,912 tokens of 4 x 512 9.8, with the approximate ones 7.7.)
 template <typename T, int NV, int MAPS, bool GATE_FIRST>
 __global__ void __launch_bounds__(128) group_norm_warp_kernel(
     const float* __restrict__ in, int ldi, const float* __restrict__ lam, const float* __restrict__ w, float eps,
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(128) group_norm_warp_kernel(
     for (int j = 0; j < NV; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            if (GATE_FIRST) v[j][e] = gated_by<T>(v[j][e], z[j][e], gate_act);
+            if (GATE_FIRST) v[j][e] = gated_by<float>(v[j][e], z[j][e], gate_act);
             ss += v[j][e] * v[j][e];
         }
     const float rstd = factor / sqrtf(warp_sum(ss) / (float)size + eps);

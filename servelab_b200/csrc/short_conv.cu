@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) qk_conv_cache_kernel(
     }
     if (act == 1) {
 #pragma unroll
-        for (int v = 0; v < VEC; ++v) y[v] = sizeof(T) == 2 ? silu_mul_fast(y[v], 1.0f) : silu_mul(y[v], 1.0f);
+        for (int v = 0; v < VEC; ++v) y[v] = silu_for<T>(y[v]);
     }
     if (c < q_size) {
         if (temp_coef != 0.f) {
@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(256) qk_conv_cache_kernel(
 // read (SC_RUN + TAPS - 1) / SC_RUN times instead of TAPS times and the taps once; all its rows are in flight
 // before the first is used.  Tokens near a request's start take the rows before them from its record.
 // What bounds it is memory and, with SiLU, the exponentials.  3,072 channels, 4 taps: 2,048 tokens 16.8 -> 8.9 us;
-// with SiLU 19.6 -> 13.0, and 10.5 since bfloat16 results take the approximate reciprocal.  (8 channels a thread: 161 registers, slower.)
+// with SiLU 19.6 -> 13.0, and 10.5 since bfloat16 results take the approximate reciprocal.  (8 channels a thread: 161
+// registers, slower.)
 constexpr int SC_RUN = 8;
 template <typename T> __device__ __forceinline__ void load4(const T* p, float (&v)[4]);
 template <> __device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) { load_vec<float, 4>(p, v); }
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(128) conv_run_kernel(
     auto finish = [&](int t, int s, float (&y)[4]) {
         if (act == 1) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) y[v] = sizeof(T) == 2 ? silu_mul_fast(y[v], 1.0f) : silu_mul(y[v], 1.0f);
+            for (int v = 0; v < 4; ++v) y[v] = silu_for<T>(y[v]);
         }
         if (c < q_size) {
             if (temp_coef != 0.f) {

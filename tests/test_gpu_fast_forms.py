@@ -223,6 +223,23 @@ def test_gate_before_norm_of_many_parts(dtype, size, T):
         assert torch.equal(out[-7:], run(x[-7:], gate[-7:]))
 
 
+@pytest.mark.parametrize("T,groups,size", [(257, 8, 64), (257, 8, 100), (3, 4, 512), (2, 1, 2048), (2, 3, 4500)])
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+def test_gate_before_norm_is_float32_whatever_the_result(T, groups, size, act):
+    """The gated value enters a float32 sum of squares: bfloat16 results are the float32 results rounded, bit for bit (the
+    same kernel, the same order of the sums)."""
+    g = gen(size)
+    n = groups * size
+    x, w = torch.randn(T, n, device=DEV, generator=g), torch.randn(n, device=DEV, generator=g)
+    gate = (torch.randn(T, n, device=DEV, generator=g) * 6).bfloat16()
+    outs = []
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.empty(T, n, device=DEV, dtype=dtype)
+        K().gate_group_norm(x, gate.to(dtype), groups, out, eps=1e-6, weight=w, factor=1.5, gate_activation=act)
+        outs.append(out.bfloat16())
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n", [4, 1024, 1028, 2048, 3584, 4100])
 def test_sum_of_two_norms_against_64_bits(dtype, n):
