@@ -464,10 +464,22 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float s[64];
             tmem_ld64(tmem + lane_base + S_COL + 64 * (j & 1), s);
+            const int k0 = kbeg + j * BN;
+            const bool open = k0 + BN - 1 <= p_first && k0 >= all_first;
             if (cap_in > 0.f) {
+                // the largest score that counts: keys that a row does not see may be anything (slots that no request has
+                // written, another one's), and so may rows of padding, and neither may decide how the others are capped
                 float big = 0.f;
+                if (open) {
 #pragma unroll
-                for (int i = 0; i < 64; ++i) big = fmaxf(big, fabsf(s[i]));
+                    for (int i = 0; i < 64; ++i) big = fmaxf(big, fabsf(s[i]));
+                } else {
+                    const int lo = pos_first - k0, hi = min(kend, pos + 1) - k0;
+#pragma unroll
+                    for (int i = 0; i < 64; ++i)
+                        if (i >= lo && i < hi) big = fmaxf(big, fabsf(s[i]));
+                }
+                if (r >= nrows) big = 0.f;
                 // (the exponential and the reciprocal of the general form are what four cycles of the multiply-adds' units
                 // cost: 2,000 cycles a tile, this form 900)
                 if (__any_sync(0xffffffffu, !(big * to_x <= 0.35f)))
@@ -475,7 +487,6 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
                 else
                     cap_small_scores(s, to_x);
             }
-            const int k0 = kbeg + j * BN;
             if (slopes != nullptr) {
                 const float base = slope * (float)(k0 - pos);
 #pragma unroll
@@ -484,7 +495,6 @@ __global__ void __launch_bounds__(THREADS, TMEM_COLS == 512 ? 1 : 2) attention_k
             // raw scores stay unscaled; masked ones become -inf.  A tile that every row of
             // the block sees completely needs no mask (rows of padding compute garbage that
             // is never stored).
-            const bool open = k0 + BN - 1 <= p_first && k0 >= all_first;
             if (!open) slb_softmax::mask_keys(s, pos_first - k0, min(kend, pos + 1) - k0);
             float alpha = 1.f;
             uint32_t packed[32];

@@ -230,6 +230,33 @@ def test_attention_with_a_soft_cap_and_a_sink(dtype, spike, shape, decode):
             assert K.attention_kv_tc_status(Dk, Dv) == 0 and K.attention_kv_mma_status(Dk, Dv) == 0
 
 
+@pytest.mark.parametrize("shape", [(8, 2, 64, 64, 90), (6, 1, 128, 128, None), (3, 3, 128, 64, 40)])
+def test_a_soft_cap_does_not_hang_on_slots_that_no_request_has_written(shape):
+    """Scores small enough for the cap's series, in portions that end inside a page and inside a tile: the same bits
+    whether unwritten slots hold huge numbers, zeros or another request's keys, and with another request behind the
+    last one (its queries fill up the last tile's rows)."""
+    from servelab_b200.ops import attention as A, kernels as K
+    Hq, G, Dk, Dv, window = shape
+    ctxs, qlens, ps = [301, 65, 70], [37, 64, 3], 16
+    case = _attention_case(7, Hq, G, Dk, Dv, window, ctxs, qlens, ps, torch.bfloat16, None, 6.0, None)
+    assert K.attention_kv_tc_takes(Dk, Dv, ps, Hq // G, False)
+    empty, results = case["kc"] > 1e29, []
+    for fill in (None, 0.0, 3.0):
+        kc = case["kc"] if fill is None else torch.where(empty, torch.full_like(case["kc"], fill), case["kc"])
+        for behind in (0, 40):
+            q, entries = case["q"], list(case["entries"])
+            if behind:
+                q = torch.cat([q, torch.full((behind, q.shape[1]), 40.0, device=DEV, dtype=q.dtype)])
+                entries.append(_entry(behind, 0, [0, 1, 2]))
+            ctx = _ctx(entries)
+            out = torch.zeros(q.shape[0], Hq * Dv, dtype=torch.bfloat16, device=DEV)
+            A.kv_attention(ctx, q, kc, torch.where(case["vc"] > 1e29, torch.zeros_like(case["vc"]), case["vc"]), Dv, out,
+                           ctx.block_tables[0], Hq, G, Dk, Dv, ps, 0.2, window or 0, None, 6.0, None)
+            results.append(out[:sum(qlens)])
+    assert all(torch.equal(r, results[0]) for r in results)
+    assert (results[0].double().cpu() - case["want"]).abs().max() < 6e-2 * max(1.0, float(case["want"].abs().max()))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_single_tokens_with_key_splits_cap_sink_and_gate(dtype):
     """Few requests with long contexts: the keys of a request are split over blocks, and the sink
