@@ -916,23 +916,24 @@ def gemm_rows_gated_takes(x: torch.Tensor, w: torch.Tensor, block: int) -> bool:
 
 
 def gemm_rows_gated_pays(m: int, inter: int, k: int) -> bool:
-    """Whether that product is ahead of the library's and the activation's kernel.  A pair of SMs has 128 features, so
-    matrices with few of them leave SMs idle (1,024 x 512, us at 200 / 512 / 1,000 / 2,048 tokens: library 5.9 / 6.2 / 7.0 /
-    9.0, own 5.9 / 6.7 / 7.2 / 8.2; 512 x 1,536 5.9 / 6.8 / 8.8 / 13.6, own 5.3 / 6.5 / 7.9 / 11.1).  Up to 128 tokens both
-    wait for the weights, and the library's tiles are full at 64 and 128 (2,048 x 2,816 at 33 / 64 / 100 / 128 tokens 9.3 /
-    7.6 / 9.8 / 7.8, own 8.7 / 8.8 / 9.3 / 9.2; 896 x 4,864 8.9 / 9.9 / 8.1 / 7.0, own 7.5 / 8.4 / 7.0 / 7.2), and many
-    features must fill whole rounds of the SMs (148 pairs' tiles of 3,584 x 18,944 at 65 / 128 tokens 52 / 56, own 45 / 45;
-    108 of 5,120 x 13,824 52 / 60, own 56 / 57)."""
+    """Whether that product is ahead of the library's and the activation's kernel.  A pair of SMs has 128 features and walks
+    all of K for them, 0.29 us a hundred, where the library cuts K: K may be the longer the more tiles of features there
+    are.  us, library / own, weights not in L2: 8 tiles of K = 896 / 1,152 / 1,536 / 2,048 / 3,584, 48 tokens 5.5 / 5.5, 5.7
+    / 6.2, 6.3 / 7.0, 6.8 / 8.5, 8.3 / 13.1, 100 tokens 6.7 / 5.6, 7.1 / 6.2, 7.6 / 7.0, 8.3 / 8.5, 10.1 / 13.2, 200 tokens 7.0 /
+    6.1, 7.4 / 6.7, 7.9 / 7.7, 8.7 / 9.2, 10.6 / 13.8; 22 tiles of the same, 48 tokens 6.7 / 6.5, 7.3 / 7.1, 8.4 / 8.0, 9.6 / 9.7,
+    12.2 / 14.7, 64 tokens 8.0 / 6.4, 9.1 / 7.0, 10.9 / 7.9, 9.6 / 9.5, 12.7 / 14.5, 128 tokens 7.9 / 6.6, 8.4 / 7.2, 9.0 / 8.2, 9.8 /
+    9.8, 12.9 / 14.8, 200 tokens 8.6 / 7.0 ... 16.3 / 15.2; 38 tiles of 896 / 3,584, 64 tokens 9.3 / 7.2, 17.2 / 15.8, 128 tokens 9.0
+    / 7.3, 17.6 / 16.6.  With fewer than 8 tiles only long steps gain whatever K (2 tiles of 2,048, 1,000 / 2,048 tokens 7.9 /
+    9.6, own 9.1 / 9.3).  Up to 128 tokens many features must fill whole rounds of the SMs (148 tiles of 3,584 at 65 / 128
+    tokens 52 / 55, own 45 / 46; 75 30 / 34, own 36 / 35)."""
     tiles, pairs = -(-inter // 128), _num_sms() // 2
     if m <= 16:                                                # (the weight-streaming products' steps)
         return False
-    if m > 128:
-        return tiles >= 8 or m >= 1500
-    if tiles > pairs:
+    if m >= 1500:
+        return True
+    if m <= 128 and tiles > pairs:
         return 10 * tiles >= 9 * pairs * -(-tiles // pairs)
-    if 48 < m <= 64 or m > 112:
-        return k <= 1024 and m <= 64 and tiles >= 8
-    return tiles >= 8
+    return tiles >= 8 and k <= (96 if m <= 64 else 144 if m <= 128 else 240) * tiles
 
 
 def gemm_rows_gated(x: torch.Tensor, w: torch.Tensor, block: int, activation: str = "silu",

@@ -116,3 +116,15 @@ def test_k_splits_have_blocks_of_their_own_and_finer_ones_an_sm(n, k, groups, sp
     kblocks = -(-k // 64)
     for s in (splits, K.tc_decode_splits(n, k, groups)):
         assert (s - 1) * -(-kblocks // s) < kblocks
+
+
+@pytest.mark.parametrize("m,inter,k,own", [
+    (16, 4864, 896, False), (17, 4864, 896, True), (20, 1024, 3584, False), (112, 1024, 3584, False), (512, 1024, 3584, False),
+    (1500, 1024, 3584, True), (48, 1024, 2048, False), (64, 2816, 1536, True), (64, 2816, 3584, False), (128, 2816, 2048, True),
+    (128, 2816, 3584, False), (200, 2816, 3584, True), (64, 896, 896, False), (200, 768, 2048, False), (128, 18944, 3584, True),
+    (65, 9600, 3584, False), (480, 4864, 896, True), (2048, 18944, 3584, True)])
+def test_gated_products_with_few_features_and_a_long_k_stay_with_the_library(monkeypatch, m, inter, k, own):
+    """A tile of features walks all of K alone: on either side of the line by tokens, features and K."""
+    from servelab_b200.ops import kernels
+    monkeypatch.setattr(kernels, "_num_sms", lambda: 148)
+    assert kernels.gemm_rows_gated_pays(m, inter, k) is own
