@@ -485,6 +485,8 @@ def prefill_splits(units: int, longest_context: int, window: int, head_dim: int)
     if prefill_force_splits:
         return prefill_force_splits
     seen = min(longest_context, window + 63) if window > 0 else longest_context
+    if seen <= 11 * 64:                                    # (fewer key tiles than any line below: the host's way of short steps)
+        return 1
     tiles, sms, best = -(-seen // 64), _num_sms(), 1
     for splits, alone, shared in ((2, 12, 24), (4, 16, 32), (8, 18, 32)):
         need = alone + (4 if head_dim > 64 else 0) if splits * units <= sms else shared

@@ -128,3 +128,14 @@ def test_gated_products_with_few_features_and_a_long_k_stay_with_the_library(mon
     from servelab_b200.ops import kernels
     monkeypatch.setattr(kernels, "_num_sms", lambda: 148)
     assert kernels.gemm_rows_gated_pays(m, inter, k) is own
+
+
+def test_short_prompts_do_not_pay_for_the_choice_of_a_cluster(monkeypatch):
+    """Below twelve key tiles no block shares its keys, and that is known from the length alone: the device is not asked."""
+    from servelab_b200.ops import kernels
+    asked = []
+    monkeypatch.setattr(kernels, "_num_sms", lambda: asked.append(1) or 148)
+    assert all(kernels.prefill_splits(units, n, w, D) == 1 for units in (1, 16, 400) for n in (1, 64, 704) for w in (0, 40, 5000)
+               for D in (64, 128))
+    assert kernels.prefill_splits(16, 4000, 600, 64) == 1 and not asked
+    assert kernels.prefill_splits(16, 705, 0, 64) == 2 and asked
