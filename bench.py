@@ -425,7 +425,7 @@ def main(argv=None) -> int:
     def kernel_status():
         """Status words of the kernels with bounded waits and page checks (0 = nothing happened)."""
         D = cfg["head_dim"]
-        status = {"gemm_tc": K.gemm_tc_status(), "attention": K.attention_status(D),
+        status = {"gemm_tc": K.gemm_tc_status(), "gemm_rows": K.gemm_rows_status(), "attention": K.attention_status(D),
                   "prefill_attention_tc": K.prefill_attention_tc_status(D),
                   "decode_attention": K.decode_attention_status(D),
                   "cache_write": K.cache_write_status()}

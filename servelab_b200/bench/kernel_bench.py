@@ -402,7 +402,7 @@ def main(argv=None) -> int:
           f"{shape[4]}, vocabulary {shape[5]}; page {PAGE}; peaks ({peaks['source']}) "
           f"{peaks['hbm_gbs']:.0f} GB/s, {peaks['bf16_tflops']:.0f} TFLOP/s")
     print(render(rows, args.markdown))
-    status = {"gemm_tc": K.gemm_tc_status(), "attention": K.attention_status(shape[3]),
+    status = {"gemm_tc": K.gemm_tc_status(), "gemm_rows": K.gemm_rows_status(), "attention": K.attention_status(shape[3]),
               "prefill_attention_tc": K.prefill_attention_tc_status(shape[3]),
               "decode_attention": K.decode_attention_status(shape[3])}
     print("kernel status words (0 = no bounded wait gave up):", json.dumps(status))

@@ -80,6 +80,16 @@ def test_a_cluster_whose_block_gave_up_stores_nothing():
     assert len(stores) == 1 and combine.index("if (whole && r < nrows) {") < stores[0]
 
 
+@pytest.mark.parametrize("path", ["bench.py", os.path.join("servelab_b200", "bench", "kernel_bench.py")])
+def test_benchmarks_read_the_status_of_every_kernel_they_run(path):
+    """A run counts as clean by these words: the products of a prompt's feed-forward are among them."""
+    with open(os.path.join(os.path.dirname(os.path.dirname(CSRC)), path)) as f:
+        words = re.search(r"status = (\{.*?\})", f.read(), re.S).group(1)
+    for call in ("gemm_tc_status()", "gemm_rows_status()", "attention_status(", "prefill_attention_tc_status(",
+                 "decode_attention_status("):
+        assert "K." + call in words
+
+
 def test_the_vote_is_of_all_lanes():
     text = source("common.cuh")
     assert "__all_sync(0xffffffffu, seen)" in body(text, text.index("bool slb_warp_agrees("))
