@@ -973,6 +973,21 @@ static int launch_state_walk(const StateSpaceChunkArgs& c, int num_seqs, int sli
     return slb_launch(state_chunk_walk_kernel<NB>, dim3(num_seqs, c.a.H, slices * (c.a.N / NB)), dim3(SC_THREADS), smem, st, c);
 }
 
+// Whether a step takes the kernels for rows in whole pieces (NN), and whether these have the chunks side by side.  The walk
+// is a chain of about 0.9 us a chunk of the longest request; the chunks side by side take a launch more and the states' way
+// through memory twice more (us walked / side by side: 2,048 tokens of 32 heads of 128 x 64 68 / 55, of 16 of 64 x 64 40 /
+// 27; 256 of them 18.5 / 19.0 and 12.7 / 13.6; 16 x 256 of 32 heads 77 / 105).
+static bool sc_in_pieces(const StateSpaceArgs& a) {
+    return ((a.ld | a.x_off | a.b_off | a.c_off | a.P) & 7) == 0 && ((uintptr_t)a.u & 15) == 0 &&
+           (long long)a.H * ((a.P + SC_EV - 1) / SC_EV) <= 65535 && (a.N == 64 || a.N == 128);
+}
+static bool sc_side_by_side(const StateSpaceChunkArgs& c, int num_seqs, int longest) {
+    const StateSpaceArgs& a = c.a;
+    const int chunks = longest > 0 ? (longest + SC_CHUNK - 1) / SC_CHUNK : (c.num_tiles + num_seqs - 1) / num_seqs;
+    const int slices = (a.P + SC_EV - 1) / SC_EV;
+    return 0.9 * chunks > 3.5 + 0.0176 / 8192 * ((double)c.num_tiles * a.H * slices * SC_EV * a.N);
+}
+
 template <int NN>
 static int launch_state_chunks(const StateSpaceChunkArgs& c, int num_seqs, int longest, cudaStream_t st) {
     static unsigned long long done = 0;
@@ -981,11 +996,7 @@ static int launch_state_chunks(const StateSpaceChunkArgs& c, int num_seqs, int l
     if (rc != 0) return rc;
     const int slices = (a.P + SC_EV - 1) / SC_EV, units = a.H / a.G * slices, per = sc_units(a, c.num_tiles, 2);
     const long long whole = (long long)num_seqs * a.H * slices, room = 2 * slb_num_sms();
-    // The walk is a chain of about 0.9 us a chunk of the longest request; the chunks side by side take a launch more and
-    // the states' way through memory twice more (us walked / side by side: 2,048 tokens of 32 heads of 128 x 64 68 / 55, of
-    // 16 of 64 x 64 40 / 27; 256 of them 18.5 / 19.0 and 12.7 / 13.6; 16 x 256 of 32 heads 77 / 105).
-    const int chunks = longest > 0 ? (longest + SC_CHUNK - 1) / SC_CHUNK : (c.num_tiles + num_seqs - 1) / num_seqs;
-    if (0.9 * chunks > 3.5 + 0.0176 / 8192 * ((double)c.num_tiles * a.H * slices * SC_EV * NN)) {
+    if (sc_side_by_side(c, num_seqs, longest)) {
         static unsigned long long done_sums = 0;
         const size_t smem = (size_t)SC_CHUNK * (SC_LDX + NN + SC_PAD) * sizeof(bf16);
         rc = slb_configure(&done_sums, state_chunk_sums_kernel<NN>, smem);
@@ -1006,6 +1017,11 @@ static int launch_state_chunks(const StateSpaceChunkArgs& c, int num_seqs, int l
 
 extern "C" {
 int slb_state_space_chunk_tokens() { return SC_CHUNK; }
+// kernels that slb_state_space_chunk_bf16 launches for the same arguments
+int slb_state_space_chunk_launches(const StateSpaceChunkArgs* c, int num_seqs, int longest) {
+    if (num_seqs <= 0 || c->num_tiles <= 0) return 0;
+    return sc_in_pieces(c->a) && !sc_side_by_side(*c, num_seqs, longest) ? 2 : 3;
+}
 // u bfloat16; the tile list cuts every request's tokens of the step into chunks of slb_state_space_chunk_tokens()
 // (request, first row), a request's in order.
 // work: num_tiles x H x N x (P rounded up to 16) numbers; longest: tokens of the longest request (0: not known, the mean
@@ -1019,12 +1035,10 @@ int slb_state_space_chunk_bf16(const StateSpaceChunkArgs* c, int num_seqs, int l
         (((uintptr_t)c->work | (uintptr_t)a.out) & 15))
         return SLB_ERR_BAD_ARG;
     if (a.N > SC_MAX_N || a.H > 65535 || a.P > 65535) return SLB_ERR_TOO_LARGE;
-    const bool pieces = ((a.ld | a.x_off | a.b_off | a.c_off | a.P) & 7) == 0 && ((uintptr_t)a.u & 15) == 0;
     const int elems = a.N * a.P;
     const bool quads = elems % 4 == 0 && a.state_stride % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
-    const bool whole = pieces && (long long)a.H * ((a.P + SC_EV - 1) / SC_EV) <= 65535;
-    if (whole && a.N == 128) return launch_state_chunks<128>(*c, num_seqs, longest, st);
-    if (whole && a.N == 64) return launch_state_chunks<64>(*c, num_seqs, longest, st);
+    if (sc_in_pieces(a))
+        return a.N == 128 ? launch_state_chunks<128>(*c, num_seqs, longest, st) : launch_state_chunks<64>(*c, num_seqs, longest, st);
     static unsigned long long done_local = 0, done_out = 0;
     int rc = slb_configure(&done_local, state_chunk_local_kernel, sc_local_smem(SC_MAX_N));
     if (rc == 0) rc = slb_configure(&done_out, state_chunk_out_kernel, sc_out_smem(SC_MAX_N));

@@ -1620,8 +1620,8 @@ def state_space(ctx, u: torch.Tensor, dt: torch.Tensor, state: torch.Tensor, out
         # (a padded step may be replayed with other lengths)
         longest = 0 if getattr(ctx, "_padded_tiles", None) is not None else max(ctx.q_lens)
         L.check(L.core().slb_state_space_chunk_bf16(_ct.byref(c), ctx.num_seqs, longest, _stream()), "state_space (chunks)")
-        global launch_count
-        launch_count += 1
+        global launch_count                                # (the call above counts as one)
+        launch_count += L.core().slb_state_space_chunk_launches(_ct.byref(c), ctx.num_seqs, longest) - 1
         return
     fn = getattr(L.core(), "slb_state_space_" + _suffix(u.dtype))
     L.check(fn(_ct.byref(a), ctx.num_seqs, _stream()), "state_space")

@@ -118,6 +118,7 @@ _CORE_SIGNATURES = {
     "slb_state_space_max_state": [],
     "slb_state_space_chunk_tokens": [],
     "slb_state_space_chunk_bf16": [P, I, I, P],
+    "slb_state_space_chunk_launches": [P, I, I],
     "slb_embed_norm_streams_f32": [P, P, P, F, P, I, I, I, I, P],
     "slb_embed_norm_streams_bf16": [P, P, P, F, P, I, I, I, I, P],
     "slb_hyper_mix_norm_f32": [P, P, I, P, P, P, P, F, P, I, P, I, I, I, P],

@@ -420,6 +420,29 @@ def test_blocks_of_several_heads_are_those_of_the_general_kernels(H, P, N, G, le
     _chunks_in_pieces(H, P, N, G, lens)
 
 
+@pytest.mark.parametrize("H,N,odd,lens,launches", [(32, 64, False, [64] * 20, 2), (32, 128, False, [100], 2), (4, 64, False, [2000], 3),
+                                                   (4, 64, True, [64] * 20, 3), (4, 96, False, [100], 3)])
+def test_launches_of_the_chunks_are_counted(H, N, odd, lens, launches):
+    """Walk and outputs; sums, scan and outputs; the general form on rows at an odd address and for other state sizes."""
+    from torch.profiler import ProfilerActivity, profile
+    P, T, g = 64, sum(lens), gen(N)
+    ctx, _ = step(lens)
+    u = torch.randn(T, H * P + 2 * N, device=DEV, generator=g).bfloat16()
+    u = odd_view(u) if odd else u
+    dt, state, out = torch.zeros(T, H, device=DEV), torch.zeros(len(lens), H * N * P, device=DEV), torch.zeros(T, H * P, device=DEV)
+    one = torch.ones(H, device=DEV)
+
+    def run():
+        K().state_space(ctx, u, dt, state, out, num_heads=H, value_dim=P, state_dim=N, groups=1, dt_bias=one, rate=one, skip=one)
+    run()
+    before = K().launch_count
+    with profile(activities=[ProfilerActivity.CUDA]) as seen:
+        run()
+        torch.cuda.synchronize()
+    kernels = sum(e.count for e in seen.key_averages() if "state_chunk" in e.key)
+    assert K().launch_count - before == launches == kernels
+
+
 def _chunks_in_pieces(H, P, N, G, lens):
     g, T = gen(H + len(lens)), sum(lens)
     ctx, _ = step(lens)
