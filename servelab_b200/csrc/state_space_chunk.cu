@@ -975,8 +975,11 @@ static int launch_state_walk(const StateSpaceChunkArgs& c, int num_seqs, int sli
 
 // Whether a step takes the kernels for rows in whole pieces (NN), and whether these have the chunks side by side.  The walk
 // is a chain of about 0.9 us a chunk of the longest request; the chunks side by side take a launch more and the states' way
-// through memory twice more (us walked / side by side: 2,048 tokens of 32 heads of 128 x 64 68 / 55, of 16 of 64 x 64 40 /
-// 27; 256 of them 18.5 / 19.0 and 12.7 / 13.6; 16 x 256 of 32 heads 77 / 105).
+// through memory twice more (us walked / side by side, state size x values, heads: 64 x 32, 8, 320 / 384 / 512 / 2,048 tokens
+// 12.4 / 12.6, 13.1 / 12.4, 14.5 / 12.6, 33.6 / 18.0; 64 x 64, 32, 512 / 1,024 / 2,048 21.6 / 17.7, 36.0 / 23.2, 64.7 / 37.8, 64
+// heads 25.4 / 22.7, 43.6 / 36.2, 80.3 / 63.9; 128 x 64, 32, 256 / 512 / 768 / 1,024 / 2,048 18.3 / 18.8, 23.6 / 22.0, 33.6 / 29.5,
+// 38.8 / 33.0, 69.1 / 53.5, 64 heads 19.4 / 20.3, 29.1 / 30.2, 39.6 / 39.9, 49.3 / 49.4, 90.9 / 92.9; 4 x 512 of 32 heads 41.9 /
+// 50.8, 16 x 400 121 / 179).
 static bool sc_in_pieces(const StateSpaceArgs& a) {
     return ((a.ld | a.x_off | a.b_off | a.c_off | a.P) & 7) == 0 && ((uintptr_t)a.u & 15) == 0 &&
            (long long)a.H * ((a.P + SC_EV - 1) / SC_EV) <= 65535 && (a.N == 64 || a.N == 128);
@@ -985,7 +988,7 @@ static bool sc_side_by_side(const StateSpaceChunkArgs& c, int num_seqs, int long
     const StateSpaceArgs& a = c.a;
     const int chunks = longest > 0 ? (longest + SC_CHUNK - 1) / SC_CHUNK : (c.num_tiles + num_seqs - 1) / num_seqs;
     const int slices = (a.P + SC_EV - 1) / SC_EV;
-    return 0.9 * chunks > 3.5 + 0.0176 / 8192 * ((double)c.num_tiles * a.H * slices * SC_EV * a.N);
+    return 0.9 * chunks > 4.7 + 0.009 / 8192 * ((double)c.num_tiles * a.H * slices * SC_EV * a.N);
 }
 
 template <int NN>
