@@ -1394,10 +1394,10 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         L.check(lib.slb_moe_gather_bf16(x.data_ptr(), x.stride(0), plan, E, P, top, h, xs, h, stream), "moe_gather")
         L.check(lib.slb_gemm_rows_experts_bf16(
             xs, h, w_gate_up.data_ptr(), h, act, inter, offsets, E, P, inter, h, 1, 0, *act_args,
-            weights.data_ptr() if weight_inputs else None, order if weight_inputs else None, stream), "gemm_rows_experts")
+            weights.data_ptr() if weight_inputs else None, order if weight_inputs else None, stream), "moe_gate_up")
         L.check(lib.slb_gemm_rows_experts_bf16(
             act, inter, w_down.data_ptr(), inter, ys, n_out, offsets, E, P, n_out, inter, 0, 0 if vendor else 1, 0, 0.0, 0.0,
-            None, None, stream), "gemm_rows_experts")
+            None, None, stream), "moe_down")
         combine = lib.slb_moe_combine_bf16_sorted if vendor else lib.slb_moe_combine_bf16_sorted_f32
         L.check(combine(ys, n_out, _p(out_weights), _p(shared), shared.stride(0) if shared is not None else 0,
                         out.data_ptr(), out.stride(0), plan, E, T, top, n_out, stream), "moe_combine")

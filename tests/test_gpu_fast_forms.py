@@ -721,6 +721,18 @@ def test_a_token_of_routed_experts_does_not_hang_on_the_step(E, h, I, top):
         assert torch.equal(K().moe_experts(x[:n], ids[:n], w[:n], wg, wd, None), whole[:n])
 
 
+@pytest.mark.parametrize("h,I", [(256, 128), (1024, 512), (1024, 2048)])
+def test_profiles_name_the_experts_products_alike_in_every_form(h, I):
+    """The comparisons of architectures look the two products up by these names, whichever kernels run."""
+    from servelab_b200.ops.profile import StepProfile
+    g, E, T, top = gen(h), 4, 20, 2
+    wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
+    ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
+    with StepProfile() as seen:
+        K().moe_experts(torch.randn(T, h, device=DEV, generator=g).bfloat16(), ids, torch.rand(T, top, device=DEV, generator=g), wg, wd, None)
+    assert {"moe_plan", "moe_gate_up", "moe_down", "moe_combine"} <= set(seen.totals())
+
+
 @pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (5, 1, 1, 5), (32, 4, 2, 4), (60, 3, 2, 6), (100, 1, 1, 32), (128, 32, 9, 8),
                                                (128, 2, 1, 3)])
 @pytest.mark.parametrize("score_fn", ["softmax", "sigmoid"])
