@@ -278,7 +278,23 @@ def test_small_steps_of_the_experts_take_rows_of_any_stride(T, h, I, dtype):
         assert torch.equal(K().moe_experts(view, ids, w, wg, wd, None), K().moe_experts(view.contiguous(), ids, w, wg, wd, None))
 
 
-def test_large_steps_of_the_experts_take_rows_of_any_stride():
+EXPERTS_FORMS = {"tcgen05": "slb_gemm_rows_experts_bf16", "library": "_grouped_mm", "mma": "slb_moe_gate_up_mma_bf16"}
+
+
+def experts_form(monkeypatch, form):
+    """Leaves routed experts one form of their products; the list it returns names the products that ran."""
+    from servelab_b200.ops import library as L
+    monkeypatch.setattr(K(), "moe_tcgen05", form == "tcgen05")
+    monkeypatch.setattr(K(), "moe_vendor_grouped", form == "library")
+    ran = []
+    for owner, name in ((L.core(), EXPERTS_FORMS["tcgen05"]), (torch, EXPERTS_FORMS["library"]), (L.core(), EXPERTS_FORMS["mma"])):
+        real = getattr(owner, name)
+        monkeypatch.setattr(owner, name, lambda *a, real=real, name=name, **kw: ran.append(name) or real(*a, **kw))
+    return ran
+
+
+@pytest.mark.parametrize("form", EXPERTS_FORMS)
+def test_large_steps_of_the_experts_take_rows_of_any_stride(monkeypatch, form):
     """Every second column of a wider matrix: the library's products took such rows, and so must the steps that read
     them themselves."""
     g = gen(3)
@@ -291,7 +307,10 @@ def test_large_steps_of_the_experts_take_rows_of_any_stride():
     wg, wd = ((torch.randn(*s, device=DEV, generator=g) * s[-1] ** -0.5).bfloat16() for s in ((E, 2 * I, h), (E, h, I)))
     ids = torch.stack([torch.randperm(E, device=DEV, generator=g)[:top] for _ in range(T)]).int().contiguous()
     p = torch.rand(T, top, device=DEV, generator=g)
-    wide, packed = (K().moe_experts(v, ids, p, wg, wd, None) for v in (x[:, ::2], x[:, ::2].contiguous()))
+    ran = experts_form(monkeypatch, form)
+    packed = K().moe_experts(x[:, ::2].contiguous(), ids, p, wg, wd, None)
+    assert set(ran) == {EXPERTS_FORMS[form]}
+    wide = K().moe_experts(x[:, ::2], ids, p, wg, wd, None)
     assert torch.equal(wide, packed)
 
 
@@ -356,7 +375,8 @@ def test_rows_of_a_tile_follow_the_rows_an_expert_gets():
     assert [rows(16 * n, 16) for n in (8, 9, 64, 65)] == [16, 32, 32, 64]
 
 
-def test_pairs_without_an_expert_add_nothing_in_large_steps():
+@pytest.mark.parametrize("form", ["tcgen05", "library"])
+def test_pairs_without_an_expert_add_nothing_in_large_steps(monkeypatch, form):
     """The list of a plan has an entry for every pair, also where ids are no expert's: in range, and the step's sum is
     that of the other pairs (the zero weights beside valid ids: the same products, the same bits)."""
     from servelab_b200.ops import library as L
@@ -373,10 +393,12 @@ def test_pairs_without_an_expert_add_nothing_in_large_steps():
     order, rows = plan[-2 * P:-P].cpu(), int(plan[2 * E])
     assert rows == P - int(bad.sum()) and (order[rows:] == 0).all()
     assert torch.equal(order[:rows].sort().values, (~bad).view(-1).nonzero().view(-1).int().cpu())
+    ran = experts_form(monkeypatch, form)
     for weighted in (False, True):
         got = K().moe_experts(x, holes, w, wg, wd, None, weight_inputs=weighted)
         want = K().moe_experts(x, ids, torch.where(bad, 0.0, w), wg, wd, None, weight_inputs=weighted)
         assert torch.equal(got, want)
+    assert set(ran) == {EXPERTS_FORMS[form]}
 
 
 @pytest.mark.parametrize("T,E,top,h,I", [(1, 8, 2, 64, 40), (3, 4, 4, 128, 72), (33, 8, 2, 200, 64), (64, 8, 2, 64, 136),

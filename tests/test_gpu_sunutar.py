@@ -543,12 +543,12 @@ def test_router_takes_the_largest_sigmoids_and_keeps_them():
 @pytest.mark.parametrize("shape", [(40, 48, 24, 5, 2), (70, 50, 14, 3, 3), (1, 64, 64, 1, 1), (200, 128, 64, 9, 1),
                                    (600, 2048, 1024, 3, 2)])
 def test_experts_weighted_at_their_inputs(dtype, shape):
-    """The clamped activation is not linear, so a weight at the output would differ; the large shape takes the
-    library's grouped product in bfloat16."""
+    """The clamped activation is not linear, so a weight at the output would differ; the large shape has each form of
+    the bfloat16 products in turn."""
     from servelab_b200.ops import kernels as K
     T, h, ff, E, top = shape
     if dtype == torch.float32 and h > 1000:
-        pytest.skip("the large shape is there for the grouped product")
+        pytest.skip("the large shape is there for the bfloat16 products")
     g = torch.Generator().manual_seed(h)
     x = torch.randn(T, h, generator=g).to(dtype)
     W = {}
@@ -567,13 +567,15 @@ def test_experts_weighted_at_their_inputs(dtype, shape):
     tol = 1e-5 if dtype == torch.float32 else 2e-2
     _close(K.moe_experts(*args), want, tol)
     if dtype == torch.bfloat16:
-        K.moe_vendor_grouped = False
+        K.moe_tcgen05 = False
         try:
-            _close(K.moe_experts(*args), want, tol, "own products")
+            _close(K.moe_experts(*args), want, tol, "the library's grouped product")
+            K.moe_vendor_grouped = False
+            _close(K.moe_experts(*args), want, tol, "mma.sync")
             K.moe_tensor_cores = False
             _close(K.moe_experts(*args), want, tol, "CUDA cores")
         finally:
-            K.moe_vendor_grouped = K.moe_tensor_cores = True
+            K.moe_tcgen05 = K.moe_vendor_grouped = K.moe_tensor_cores = True
 
 
 @pytest.mark.parametrize("dtype", BOTH)
