@@ -76,12 +76,10 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
     return scratch[32];
 }
 
-// One lane of a converged warp, for instructions that one thread issues (copies by the tensor unit, MMAs, commits):
-// their operands sit in uniform registers, and behind `lane == 0`, which the compiler does not know to be a single
-// lane, every one of them becomes a loop over the lanes (a k-block of a product, two copies and four MMAs: 780 cycles,
-// whatever its size).  Loops around them run with the whole warp, so that addresses and counters stay uniform.  With
-// it, us a step: 8 layers of the 0.5B shape, one request 205 -> 193, 4 layers of the 7B shape, 8 requests 411 -> 402;
-// a latent attention's prompts 158 -> 150.
+// One lane of a converged warp, for instructions that one thread issues (copies by the tensor unit, MMAs, commits).
+// Loops around them run with the whole warp.  Issued behind `lane == 0` instead, a k-block of a product (two copies and
+// four MMAs) took 780 cycles whatever its size.  us a step, `lane == 0` / this: 8 layers of the 0.5B shape, one request
+// 205 / 193, 4 layers of the 7B shape, 8 requests 411 / 402; a latent attention's prompts 158 / 150.
 __device__ __forceinline__ bool slb_elected() {
     uint32_t yes;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));

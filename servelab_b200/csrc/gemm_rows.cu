@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) gemm_rows_kernel(const __grid_c
             const int f4 = f & ~3;
             if constexpr (EPI == GR_GATED) {
                 // 16 tokens at a time, the next ones on their way from tensor memory.  (A short loop: unrolled over
-                // a tile, every instruction of it was fetched for one use, 6 us a launch.)
+                // a tile a launch took 6 us more.)
                 const int up = lane >> 4;                  // lanes 0..15 hold gates, the others their ups
                 float v[16], next[16];
                 if (half * 16 < tokens) {

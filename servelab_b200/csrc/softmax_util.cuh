@@ -1,7 +1,8 @@
 // What the softmax warps of the tcgen05 attention kernels share.  A tile of 64 scores a thread is bound by its 64
 // exponentials (four a cycle and scheduler: 512 cycles), so everything else is done two values or three operands an
-// instruction: 32 maxima, 32 multiply-adds, 32 additions, 32 conversions.  us a tile of 64 keys with one value each: 1,175
-// cycles for a block alone on its SM, 1,400 for two.
+// instruction: 32 maxima, 32 multiply-adds, 32 additions, 32 conversions.  (One value each, a tile took 1,175 cycles for a
+// block alone on its SM and 1,400 for two; with this 2,048 tokens of 28 / 4 heads of 128 went from 43.6 to 38.9 us, the
+// other changes of the attention kernel among them.)
 #pragma once
 
 #include "common.cuh"

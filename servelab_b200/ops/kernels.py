@@ -1316,13 +1316,15 @@ def moe_route(logits: torch.Tensor, groups: int, keep: int, top: int, route_scal
     return ids, weights
 
 
-moe_vendor_grouped = True      # bfloat16 steps of many rows: the vendor's grouped product (off: this package's)
+# Where the tcgen05 products (below) do not take the operands -- an intermediate size that is no multiple of 16, results of
+# a width that is no multiple of 4, matrices that are not contiguous -- or are switched off:
+moe_vendor_grouped = True      # bfloat16 steps of many rows: the vendor's grouped product (off: mma.sync)
 moe_vendor_min_pairs = 1024    # (token, choice) pairs from which it is taken ...
-moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this many elements a matrix.  Own / vendor,
+moe_vendor_min_expert_elements = 1 << 21   # ... for experts of at least this many elements a matrix.  mma.sync / vendor,
                                            # us, 4 experts a token: 32 of 2,048 x 1,408, 128 tokens 136 / 144, 160 144 /
-                                           # 143, 256 178 / 145, 2,048 695 / 208; 16 of 1,024 x 512, 128 tokens 36 /
-                                           # 37, 256 44 / 38, 512 66 / 40, 2,048 160 / 72: the vendor's is ahead of
-                                           # the smaller ones too, which stay with this package's kernel all the same
+                                           # 143, 256 178 / 145, 2,048 695 / 208 (tcgen05 179); 16 of 1,024 x 512, 128
+                                           # tokens 36 / 37, 256 44 / 38, 512 66 / 40, 2,048 160 / 72: the vendor's is
+                                           # ahead of the smaller ones too, which have one kernel for steps of any size
 moe_tensor_cores = True        # bfloat16: the experts' products on mma.sync (off: CUDA cores, the twin)
 
 
